@@ -206,7 +206,6 @@ class EW {
 
    // Device pointers of set-up arrays (tests / bench)
    const double* profile(int which, int axis) const;  // which: 0 dc, 1 str, 2 co
-   const double* weights(int slot) const { return w_.p[slot]; }
    int launches_per_step(int mode) const;
    // Average device time (ms, CUDA events on the EW stream) of each piece of a
    // fused step, each launched nrep times on the current levels without advancing
@@ -271,8 +270,11 @@ class EW {
    double* la_ = nullptr;
    double* irho_ = nullptr;
    double* dprof_[9] = {};  // dc x,y,z ; str x,y,z ; co x,y,z
-   WeightPtrs w_{};
+   FixedCoef fc_{};  // FP64 form: coefficients of the fixed-point stages ...
+   WeightPtrs w_{};  // ... or, without room for them, of the FP64 stages
    double* wstore_ = nullptr;
+   int alloc_stage_coefficients();
+   void free_fixed_coefficients();
    double* lev_[4] = {};
    int iu_ = 0, ium_ = 1;
    double* lu_ = nullptr;   // phase mode work arrays

@@ -1,0 +1,152 @@
+// Block fixed-point arithmetic for the FP64 stage kernels on the integer pipes.
+//
+// GB300 issues FP64 at 1/64 of its FP32 and integer rate: measured per SM and clock,
+// 1.7 FP64 operations against 59 multiply-accumulates of 32 x 32 -> 64 bits, 64 funnel
+// shifts and about 110 simple integer operations.  A stencil sum in FP64 aligns,
+// rounds and normalises every term; here the values a point's stencil reads are aligned
+// once, to the largest exponent among them, as 57-bit integers (4 bits more than an
+// FP64 significand), the differences are exact integer sums, the products are
+// accumulated in 64-bit integers, and only the finished sum is normalised.
+//
+// The error of a sum is a few units of 2^-57 of its largest term, against 2^-53 for each
+// FP64 operation.  Exponents belong to points, never to tiles: a result depends on the
+// values of the point's own stencil alone, so it does not change with the tiling, the
+// launch shape or a decomposition of the grid.
+#pragma once
+
+#include <cstdint>
+
+namespace sw4g {
+
+typedef long long i64;
+
+constexpr int kExpNone = -0x10000000;  // below any exponent
+constexpr int kSplit = 26;  // low limb of values and weights
+constexpr int kMask = (1 << kSplit) - 1;
+
+// x >> d, arithmetic, for any d >= 0 (PTX clamps the amount)
+__device__ __forceinline__ i64 sar(i64 x, int d)
+{
+   i64 r;
+   asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(d));
+   return r;
+}
+
+// x / 2^d rounded to nearest, halves to even, for d >= 0.  Sums are rounded without a
+// bias, which a time loop would accumulate: a constant in every step's acceleration grows
+// as the square of the step count, and the amounts are small, so halves are common.
+// |x| + 2^61 must fit; an amount above 62 leaves 0 or +-1.
+struct Round {
+   int d, some;
+   i64 half;  // 2^(d-1) - 1, and 0 for d = 0
+   __device__ __forceinline__ explicit Round(int amount)
+   {
+      d = min(amount, 62);
+      some = min(amount, 1);
+      asm("shr.u64 %0, %1, %2;" : "=l"(half) : "l"(-1LL), "r"(65 - d));
+   }
+   __device__ __forceinline__ i64 operator()(i64 x) const
+   {
+      return sar(x + half + (i64)((int)sar(x, d) & some), d);
+   }
+};
+
+__device__ __forceinline__ i64 madw(int a, int b, i64 c)
+{
+   i64 r;
+   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+   return r;
+}
+
+__device__ __forceinline__ int max4(int a, int b, int c, int d) { return max(max(a, b), max(c, d)); }
+
+// Three FP64 values as integers m[c] with value m[c] * 2^(e - 1079), |m[c]| < 2^57, e the
+// largest of their biased exponents (at least 1, the subnormals' exponent); bits below
+// 2^-57 of the largest are dropped toward zero.  True if one
+// is not finite; it counts as (less than) the smallest normal number.
+__device__ __forceinline__ bool to_block(double v0, double v1, double v2, i64 m[3], int& e)
+{
+   const double v[3] = {v0, v1, v2};
+   int hi[3], eb[3], any = 0;
+#pragma unroll
+   for (int c = 0; c < 3; c++) {
+      hi[c] = __double2hiint(v[c]);
+      eb[c] = (hi[c] >> 20) & 0x7ff;
+      any = max(any, eb[c]);
+      eb[c] = eb[c] == 2047 ? 0 : eb[c];
+   }
+   e = max(max(eb[0], eb[1]), max(eb[2], 1));
+#pragma unroll
+   for (int c = 0; c < 3; c++) {
+      const int lead = min(eb[c], 1) << 20;
+      const unsigned mh = (unsigned)(hi[c] & 0xfffff) | (unsigned)lead;
+      i64 t = (i64)(((unsigned long long)mh << 32) | (unsigned)__double2loint(v[c])) << 4;
+      t = sar(t, e - max(eb[c], 1));
+      const i64 s = (i64)(hi[c] >> 31);
+      m[c] = (t ^ s) - s;
+   }
+   return any == 2047;
+}
+
+// 8 (fp1 - fm1) + (fm2 - fp2)
+__device__ __forceinline__ i64 d1i(i64 fm2, i64 fm1, i64 fp1, i64 fp2)
+{
+   return ((fp1 - fm1) << 3) + (fm2 - fp2);
+}
+
+// x * C / 2^57 for |x| < 2^62 and a coefficient |C| < 2^57 held as c.x = C >> 26,
+// c.y = (C & kMask) << 5; the product of the two low limbs (below 2^-60 of the largest
+// result) is dropped, the rest rounded.
+__device__ __forceinline__ i64 mulc(i64 x, int2 c)
+{
+   const int xh = (int)(x >> 31), xl = (int)x & 0x7fffffff;
+   const i64 cross = madw(xl, c.x, madw(xh, c.y, 1LL << 30));
+   return madw(xh, c.x, cross >> 31);
+}
+
+// x * f for |x| < 2^61 and a factor 0 < f <= 1 with its full relative precision, rounded
+// to nearest (the supergrid stretching, which falls to 1e-4 at the sides).
+struct Factor {
+   int hi, lo, down;
+   bool on;
+   __device__ __forceinline__ explicit Factor(double f)
+   {
+      on = __double_as_longlong(f) != 0x3ff0000000000000LL;
+      const int h = __double2hiint(f), e = ((h >> 20) & 0x7ff) - 1022;
+      const i64 c = (i64)(((unsigned long long)((h & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(f)) << 4;
+      hi = (int)(c >> kSplit);
+      lo = (int)(c & kMask) << 5;
+      down = -e;
+   }
+   __device__ __forceinline__ i64 operator()(i64 x) const
+   {
+      if (!on) return x;
+      const int xh = (int)(x >> 31), xl = (int)x & 0x7fffffff;
+      const i64 cross = madw(xl, hi, madw(xh, lo, (madw(xl, lo, 1LL << 30) >> 31) + (1LL << 30)));
+      return Round(down)(madw(xh, hi, cross >> 31));
+   }
+};
+
+// A value |v| < 2^e as such a coefficient, C = v * 2^(57 - e) rounded.
+__device__ __forceinline__ int2 to_coef(double v, int e)
+{
+   const i64 c = min(__double2ll_rn(scalbn(v, 57 - e)), (1LL << 57) - 1);
+   return make_int2((int)(c >> kSplit), (int)(c & kMask) << 5);
+}
+
+// p * 2^e as FP64, rounded once; below the normal range 0, above it infinite.
+__device__ __forceinline__ double from_block(i64 p, int e)
+{
+   const double r = __ll2double_rn(p);
+   int hi = __double2hiint(r), lo = __double2loint(r);
+   const int eb = (hi >> 20) & 0x7ff, n = eb == 0 ? 0 : eb + e;
+   hi += e << 20;
+   if (n <= 0) hi = lo = 0;
+   if (n >= 2047) {
+      hi = p < 0 ? 0xfff00000 : 0x7ff00000;
+      lo = 0;
+   }
+   return __hiloint2double(hi, lo);
+}
+
+}  // namespace sw4g

@@ -19,6 +19,21 @@ struct WeightPtrs {
    double* s[kWeightSums];
 };
 
+// Coefficients of the fixed-point stage kernels (stage_fixed.cu): the weights of every
+// interior point's second differences, stored by blocks of kFixedBlock points along x
+// (24 lines of a block in a row; fixed_weight_len entries), the coefficients of the
+// mixed terms and the exponents of both at every array point.
+constexpr int kFixedBlock = 32;
+struct FixedCoef {
+   int2* w = nullptr;
+   int4* c = nullptr;
+   int* e = nullptr;
+   int* bad = nullptr;  // one flag: the material is not finite everywhere
+};
+long long fixed_weight_len(const Box& b);
+int launch_fixed_coef(const Box& b, const double* mu, const double* la, const double* sx, const double* sy,
+                      const double* sz, double h, const FixedCoef& c, cudaStream_t s);
+
 // One fused stage launch over the centred rows [k1,k2] of a SoA grid.
 struct FusedStage {
    Box b;
@@ -34,6 +49,7 @@ struct FusedStage {
    const double* rho = nullptr;
    const double* irho = nullptr;
    WeightPtrs w{};
+   FixedCoef fc{};
    const double* st[3] = {nullptr, nullptr, nullptr};
    const double* dc[3] = {nullptr, nullptr, nullptr};
    const double* co[3] = {nullptr, nullptr, nullptr};
@@ -390,6 +406,7 @@ int launch_inverse(long long n, const double* x, double* y, cudaStream_t s);
 int launch_uacc_slab(const Box& b, int k0, int k1, const double* up, const double* u,
                      const double* um, double* out, cudaStream_t s);
 int launch_fused_stage(const FusedStage& st, cudaStream_t stream);
+int launch_fixed_stage(const FusedStage& st, cudaStream_t stream);
 int launch_stage_rows(int corrector, bool top, const Box& b, int nk, const double* field,
                       const Box& field_box, const double* mu, const double* la, double h,
                       const double* strx, const double* stry, const double* strz,

@@ -1,4 +1,6 @@
-// Fused stage kernels of the elastic time step on Cartesian grids, sm_103a, FP64.
+// Fused stage kernels of the elastic time step on Cartesian grids, sm_103a, FP64: the
+// stages of grids for which the device has no room for the coefficients of the
+// fixed-point stages (stage_fixed.cu, twice as fast), and the set-up they share.
 //
 // One launch computes, for every centred row k1..k2 of the interior,
 //   predictor stage  out = 2u - um + dt^2/rho * L(u)
@@ -878,6 +880,7 @@ int launch_fused_stage(const FusedStage& st, cudaStream_t stream)
    if (st.k2 < st.k1) return kOk;
    const Box& b = st.b;
    if (b.cs != b.npts) return kNotSupported;  // SoA only
+   if (st.fc.w) return launch_fixed_stage(st, stream);
    FusedArgs a;
    a.ib = b.ib; a.ie = b.ie; a.jb = b.jb; a.je = b.je; a.kb = b.kb; a.ke = b.ke;
    a.ni = b.ni; a.nij = b.nij; a.npts = b.npts;
