@@ -89,6 +89,13 @@ int EW::init()
    sbp_coefficients(acof, ghcof, bope, sbop_);
    prof_ = sub_ ? subdomain_profiles(global_, g_, ioff_, joff_) : supergrid_profiles(g_);
 
+   {
+      const int g = g_.sg_order == 4 ? 2 : 3, n[3] = {g_.nx + 4, g_.ny + 4, g_.nz + 4};
+      const int lo[3] = {g, g, g}, hi[3] = {n[0] - 1 - g, n[1] - 1 - g, n[2] - 1 - g};
+      const double* dc[3] = {prof_.dc[0].data(), prof_.dc[1].data(), prof_.dc[2].data()};
+      damp_ = damp_segments(g_.sg_order, dc, n, lo, hi);
+   }
+
    const size_t n = (size_t)npts_;
    SW4G_TRY(cuda_ok(cudaGetDevice(&dev_)));
    if (sub_) {
@@ -158,8 +165,8 @@ int EW::init()
 // The fixed-point stages' coefficients take 212 bytes a point, the FP64 stages' weights
 // 144.  The fixed-point stages run where their coefficients fit and leave room for the
 // phase order's work arrays (72 bytes a point, allocated when first used), so a grid that
-// fits with the FP64 stages alone runs on those: at 512^3 a step takes 98 ms on the FP64
-// stages, 47 ms on the fixed-point ones; an empty 288 GB device holds 7e8 points with
+// fits with the FP64 stages alone runs on those: at 512^3 a step takes 95 ms on the FP64
+// stages, 40 ms on the fixed-point ones; an empty 288 GB device holds 7e8 points with
 // them and 8e8 without.
 int EW::alloc_stage_coefficients()
 {
@@ -921,6 +928,7 @@ int EW::fused_piece(int piece, int ip, int iq)
       fs.irho = irho_;
       fs.w = w_;
       fs.fc = fc_;
+      fs.damp = damp_;
       for (int q = 0; q < 3; q++) {
          fs.st[q] = st[q];
          fs.dc[q] = dc[q];
@@ -972,9 +980,8 @@ int EW::fused_piece(int piece, int ip, int iq)
                                     zc_[side], stream_, rscr_, rows_ctas_));
       }
       if (beta != 0 && g_.sg_order == 6)
-         SW4G_TRY(launch_addsgd(6, 1, bd.ib, bd.ie, bd.jb, bd.je, bd.kb, bd.ke, out, u, um, rho_,
-                                dc[0], dc[1], dc[2], st[0], st[1], st[2], co[0], co[1], co[2], beta,
-                                stream_));
+         SW4G_TRY(launch_damping_lines(6, b, bd.kb, bd.ke, damp_, u, um, out, rho_, irho_, dc, st, co, beta, nullptr,
+                                       stream_));
       return kOk;
    }
    if (piece == 5 || piece == kForceCorr || piece == kBcCorr) {

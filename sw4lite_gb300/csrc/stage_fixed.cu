@@ -3,12 +3,12 @@
 //
 // One launch computes, for every centred row k1..k2 of the interior,
 //   form 0  out = 2u - um + coef/rho * L(u)                            (predictor)
-//   form 1  out = up + coef/rho * L(up - 2u + um) - beta/rho * SG(u - um)   (corrector)
-//   form 2  out = 2u - um + coef/rho * L(up) - beta/rho * SG(u - um)        (adjoint)
-// with L the divergence of stress of the reference's rhs4sg (src/rhs4sg_rev.C:111-348)
-// and SG its 4th-order supergrid damping (src/ew-cfromfort.C:952-1057), in place of the
-// reference's RHSPredCU_center / evalDpDmInTimeCU / RHSCorrCU_center /
-// addSuperGridDampingCU_center (src/EW_cuda.C:1228-1509).
+//   form 1  out = up + coef/rho * L(up - 2u + um)                      (corrector)
+//   form 2  out = 2u - um + coef/rho * L(up)                           (adjoint)
+// with L the divergence of stress of the reference's rhs4sg (src/rhs4sg_rev.C:111-348),
+// in place of the reference's RHSPredCU_center / evalDpDmInTimeCU / RHSCorrCU_center
+// (src/EW_cuda.C:1228-1509); the supergrid damping of forms 1 and 2 follows on the layers
+// alone (damping_lines.cu).
 //
 //  * CTA = 32 x 6 columns marching up z through a 5-plane ring of the stage field in
 //    shared memory, 2-point halo: per point three 57-bit integers with one exponent.
@@ -26,11 +26,11 @@
 //    and all three of its products: those for the x and y outer differences go to shared
 //    memory, those for the z outer difference into a register queue, so a plane is
 //    finished two planes later, when the last product along z is known.
-//  * FP64 remains in forming up - 2u + um, in the update and in the damping.
+//  * FP64 remains in forming up - 2u + um and in the update.
 // What bounds them: the integer pipes (about 2300 instructions a warp of 32 points, half of
-// them at half rate) and, in the corrector's supergrid layers, the FP64 pipe.  At 512^3 the
-// predictor takes 15.2 ms and the corrector 28.2 ms, against 40.6 and 53.8 ms with the
-// sums in FP64 (stage_fused.cu), whose 160 and 198 FP64 operations a point saturate the
+// them at half rate), the corrector also the FP64 operations of its stage field.  At 512^3
+// the predictor takes 15.2 ms and the corrector 22.5 ms with the damping (28.2 ms with the
+// damping inside the kernel), against 40.6 and 53.8 ms with the sums in FP64 (stage_fused.cu), whose 160 and 198 FP64 operations a point saturate the
 // 1.7 that an SM completes per clock.  Against quad precision the levels after 50 steps are off
 // by 0.5 to 0.65 times what they were.
 #include <algorithm>
@@ -58,7 +58,6 @@ struct FixedArgs {
    const double* __restrict__ um;
    const double* __restrict__ up;
    double* __restrict__ out;
-   const double* __restrict__ rho;
    const double* __restrict__ irho;
    const int2* __restrict__ w;    // second-difference weights, by blocks of 32 points
    const int4* __restrict__ c;    // lambda and mu coefficients of the mixed terms
@@ -68,9 +67,7 @@ struct FixedArgs {
    const double* __restrict__ sx;
    const double* __restrict__ sy;
    const double* __restrict__ sz;
-   const double* __restrict__ dc[3];
-   const double* __restrict__ co[3];
-   double coef, beta;
+   double coef;
    int* emax;
 };
 
@@ -241,15 +238,6 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
    };
-
-   // Damping: an axis' term is computed where its profile dc is nonzero at one of the
-   // point's three neighbours along it; elsewhere it is exactly zero.  Tested on the bit
-   // patterns, along x and y once per column.
-   auto damped = [&](int ax, int n) {
-      return nonzero_bits(__ldg(a.dc[ax] + n - 1)) || nonzero_bits(__ldg(a.dc[ax] + n)) || nonzero_bits(__ldg(a.dc[ax] + n + 1));
-   };
-   const bool damping = FORM != 0 && a.beta != 0 && active;
-   const bool dampx = damping && damped(0, i - a.ib), dampy = damping && damped(1, j - a.jb);
 
    // Stretching of the own column, applied where it is not 1
    const double sxi = inside ? __ldg(a.sx + (i - a.ib)) : 1.0, syj = inside ? __ldg(a.sy + (j - a.jb)) : 1.0;
@@ -518,43 +506,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
          const bool st = stx || sty || !is_one(szp);
          const i64 zn[3] = {z.m0, z.m1, z.la};
          const double cr = a.coef * ir;
-         double sg[3] = {0, 0, 0};
-         if (FORM != 0) {
-            const int n[3] = {i - a.ib, j - a.jb, kp - a.kb};
-            const long long off[3] = {1, a.ni, a.nij};
-            const double str[3] = {sxi, syj, szp};
-            const bool damp[3] = {dampx, dampy, damping && damped(2, n[2])};
-#pragma unroll
-            for (int ax = 0; ax < 3; ax++) {
-               if (!damp[ax]) continue;
-               const double d0 = __ldg(a.dc[ax] + n[ax] - 1), d1 = __ldg(a.dc[ax] + n[ax]), d2 = __ldg(a.dc[ax] + n[ax] + 1);
-               const long long o = off[ax];
-               const double x0 = __ldg(a.rho + pp - o) * d0, x1 = __ldg(a.rho + pp) * d1, x2 = __ldg(a.rho + pp + o) * d2;
-               const int b0 = ax == 0 ? 1 : 0, b1 = ax == 2 ? 1 : 2;
-               const double w = str[ax] * __ldg(a.co[b0] + n[b0]) * __ldg(a.co[b1] + n[b1]);
-#pragma unroll
-               for (int c = 0; c < 3; c++) {
-                  const long long q = pp + c * npts;
-                  double d[5];
-#pragma unroll
-                  for (int m = -2; m <= 2; m++) d[m + 2] = __ldg(a.u + q + m * o) - __ldg(a.um + q + m * o);
-                  const double s = x2 * (d[4] - 2 * d[3] + d[2]) - 2 * x1 * (d[3] - 2 * d[2] + d[1]) +
-                                   x0 * (d[2] - 2 * d[1] + d[0]);
-                  sg[c] += w * s;
-               }
-            }
-         }
-         const double birho = a.beta * ir;
 #pragma unroll
          for (int c = 0; c < 3; c++) {
             i64 cz = d1i(sar(sm.gz[z0][c][tid], h0), sar(sm.gz[z1][c][tid], h1), sar(sm.gz[z3][c][tid], h3), sar(zn[c], h4));
             if (st) cz = Factor(c == 0 ? szp * sxi : c == 1 ? szp * syj : szp)(cz);
             const double lu = from_block(of_p(pq[0][c]) + of_z(cz), eF - 1072);
-            double v = base[c] + cr * lu;
-            if (FORM != 0) {
-               v -= birho * sg[c];
-               em = max(em, (__double2hiint(v) >> 20) & 0x7ff);
-            }
+            const double v = base[c] + cr * lu;
+            if (FORM != 0) em = max(em, (__double2hiint(v) >> 20) & 0x7ff);
             a.out[pp + c * npts] = v;
          }
       }
@@ -699,7 +657,6 @@ int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
    a.um = st.um;
    a.up = st.up;
    a.out = st.out;
-   a.rho = st.rho;
    a.irho = st.irho;
    a.w = st.fc.w;
    a.c = st.fc.c;
@@ -708,12 +665,7 @@ int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
    a.sx = st.st[0];
    a.sy = st.st[1];
    a.sz = st.st[2];
-   for (int q = 0; q < 3; q++) {
-      a.dc[q] = st.dc[q];
-      a.co[q] = st.co[q];
-   }
    a.coef = st.coef > 0 ? st.coef : (st.corrector ? st.dt * st.dt / 12 : st.dt * st.dt);
-   a.beta = st.beta;
    a.emax = st.emax;
    const int ni = b.ie - b.ib - 3, nj = b.je - b.jb - 3, nk = st.k2 - st.k1 + 1;
    const int gx = blocks_for(ni, TX), gy = blocks_for(nj, TY);
@@ -745,7 +697,10 @@ int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
       fixed_stage_kernel<1><<<grid, block, smem, stream>>>(a);
    else
       fixed_stage_kernel<2><<<grid, block, smem, stream>>>(a);
-   return launch_status();
+   SW4G_TRY(launch_status());
+   if (form == 0 || st.beta == 0) return kOk;
+   return launch_damping_lines(4, b, st.k1, st.k2, st.damp, st.u, st.um, st.out, st.rho, st.irho, st.dc, st.st, st.co,
+                               st.beta, st.emax, stream);
 }
 
 }  // namespace sw4g

@@ -117,6 +117,30 @@ def test_non_finite_values_reach_the_stencil_and_no_further(bad):
     assert np.array_equal(np.isfinite(got), np.isfinite(ref))
 
 
+@pytest.mark.parametrize("order", [4, 6])
+@pytest.mark.parametrize("shape,gp,top", [((190, 180, 176), 30, 0), ((61, 44, 40), 6, 2), ((40, 36, 38), 25, 2)])
+def test_damping_of_the_layers(order, shape, gp, top):
+    """The layers' own kernel (fused steps) against the kernel that visits every point
+    (the phase order): long and short marches, layers on both sides of an axis and
+    layers that meet, edges and corners in two and three layers."""
+    nx, ny, nz = shape
+    g = sg.grid_desc(nx, ny, nz, H, bc=(2, 2, 2, 2, top, 2), sg_gp=gp, sg_damping=0.02, sg_order=order)
+    _, mat, dt = _problem(shape, top)
+    u, um = smooth_fields(*shape, seed=8)
+    out = []
+    for mode in (sg.MODE_FUSED, sg.MODE_PHASES):
+        ew = sg.EW(g)
+        ew.set_material(*[dev(a) for a in mat])
+        ew.set_time_step(dt, 0.0)
+        ew.set_fields(dev(u), dev(um))
+        ew.step(1, mode)
+        r = dev(np.zeros_like(u))
+        ew.get_fields(r, None)
+        out.append(host(r))
+        ew.close()
+    assert np.max(np.abs(out[0] - out[1])) <= 2.0 ** -45 * np.max(np.abs(out[1]))
+
+
 def test_without_room_for_the_coefficients_the_fp64_stages_run():
     import torch
     shape = (200, 180, 160)
