@@ -560,7 +560,6 @@ int EW::gradient(int nsteps, int ckpt, const double* obs, bool obs_on_device, do
       fs.irho = irho_;
       fs.w = w_;
       fs.fc = fc_;
-      fs.damp = damp_;
       for (int q = 0; q < 3; q++) {
          fs.st[q] = dprof_[3 + q];
          fs.dc[q] = dprof_[q];

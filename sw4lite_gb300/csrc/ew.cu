@@ -89,13 +89,6 @@ int EW::init()
    sbp_coefficients(acof, ghcof, bope, sbop_);
    prof_ = sub_ ? subdomain_profiles(global_, g_, ioff_, joff_) : supergrid_profiles(g_);
 
-   {
-      const int g = g_.sg_order == 4 ? 2 : 3, n[3] = {g_.nx + 4, g_.ny + 4, g_.nz + 4};
-      const int lo[3] = {g, g, g}, hi[3] = {n[0] - 1 - g, n[1] - 1 - g, n[2] - 1 - g};
-      const double* dc[3] = {prof_.dc[0].data(), prof_.dc[1].data(), prof_.dc[2].data()};
-      damp_ = damp_segments(g_.sg_order, dc, n, lo, hi);
-   }
-
    const size_t n = (size_t)npts_;
    SW4G_TRY(cuda_ok(cudaGetDevice(&dev_)));
    if (sub_) {
@@ -928,7 +921,6 @@ int EW::fused_piece(int piece, int ip, int iq)
       fs.irho = irho_;
       fs.w = w_;
       fs.fc = fc_;
-      fs.damp = damp_;
       for (int q = 0; q < 3; q++) {
          fs.st[q] = st[q];
          fs.dc[q] = dc[q];
@@ -980,8 +972,8 @@ int EW::fused_piece(int piece, int ip, int iq)
                                     zc_[side], stream_, rscr_, rows_ctas_));
       }
       if (beta != 0 && g_.sg_order == 6)
-         SW4G_TRY(launch_damping_lines(6, b, bd.kb, bd.ke, damp_, u, um, out, rho_, irho_, dc, st, co, beta, nullptr,
-                                       stream_));
+         SW4G_TRY(launch_damping_layers(6, b, bd.kb, bd.ke, u, um, out, rho_, irho_, dc, st, co, beta, nullptr,
+                                        stream_));
       return kOk;
    }
    if (piece == 5 || piece == kForceCorr || piece == kBcCorr) {

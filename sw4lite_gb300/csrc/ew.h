@@ -270,7 +270,6 @@ class EW {
    double* la_ = nullptr;
    double* irho_ = nullptr;
    double* dprof_[9] = {};  // dc x,y,z ; str x,y,z ; co x,y,z
-   DampSegs damp_{};  // where the supergrid damping acts
    FixedCoef fc_{};  // FP64 form: coefficients of the fixed-point stages ...
    WeightPtrs w_{};  // ... or, without room for them, of the FP64 stages
    double* wstore_ = nullptr;

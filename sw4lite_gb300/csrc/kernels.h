@@ -34,18 +34,12 @@ long long fixed_weight_len(const Box& b);
 int launch_fixed_coef(const Box& b, const double* mu, const double* la, const double* sx, const double* sy,
                       const double* sz, double h, const FixedCoef& c, cudaStream_t s);
 
-// Where a grid's supergrid damping of an order acts along each axis: up to two segments
-// lo..hi (empty: hi = lo - 1) of array indices from 0, from the host's profiles dc (n
-// values each) over the points lo..hi.
-struct DampSegs {
-   int lo[3][2], hi[3][2];
-};
-DampSegs damp_segments(int order, const double* const dc[3], const int n[3], const int lo[3], const int hi[3]);
-// out -= damping of u - um (damping_lines.cu) on the planes k1..k2
-int launch_damping_lines(int order, const Box& b, int k1, int k2, const DampSegs& seg, const double* u,
-                         const double* um, double* out, const double* rho, const double* irho,
-                         const double* const dc[3], const double* const st[3], const double* const co[3],
-                         double beta, int* emax, cudaStream_t s);
+// out -= supergrid damping of u - um on the planes k1..k2, in the layers alone
+// (damping_layers.cu)
+int launch_damping_layers(int order, const Box& b, int k1, int k2, const double* u, const double* um, double* out,
+                          const double* rho, const double* irho, const double* const dc[3],
+                          const double* const st[3], const double* const co[3], double beta, int* emax,
+                          cudaStream_t s);
 
 // One fused stage launch over the centred rows [k1,k2] of a SoA grid.
 struct FusedStage {
@@ -63,7 +57,6 @@ struct FusedStage {
    const double* irho = nullptr;
    WeightPtrs w{};
    FixedCoef fc{};
-   DampSegs damp{};  // where beta acts (fixed-point stages)
    const double* st[3] = {nullptr, nullptr, nullptr};
    const double* dc[3] = {nullptr, nullptr, nullptr};
    const double* co[3] = {nullptr, nullptr, nullptr};

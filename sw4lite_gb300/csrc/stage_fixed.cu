@@ -8,7 +8,7 @@
 // with L the divergence of stress of the reference's rhs4sg (src/rhs4sg_rev.C:111-348),
 // in place of the reference's RHSPredCU_center / evalDpDmInTimeCU / RHSCorrCU_center
 // (src/EW_cuda.C:1228-1509); the supergrid damping of forms 1 and 2 follows on the layers
-// alone (damping_lines.cu).
+// alone (damping_layers.cu).
 //
 //  * CTA = 32 x 6 columns marching up z through a 5-plane ring of the stage field in
 //    shared memory, 2-point halo: per point three 57-bit integers with one exponent.
@@ -122,7 +122,8 @@ __device__ __forceinline__ void copy16(void* dst, const void* src)
 template <int FORM>
 __device__ __forceinline__ double stage_value(const FixedArgs& a, long long q)
 {
-   if (FORM == 1) return (__ldg(a.up + q) - 2 * __ldg(a.u + q)) + __ldg(a.um + q);
+   // fma: 2 * x compiles to x + x, an FP64 operation more
+   if (FORM == 1) return fma(-2.0, __ldg(a.u + q), __ldg(a.up + q)) + __ldg(a.um + q);
    return __ldg((FORM == 0 ? a.u : a.up) + q);
 }
 
@@ -453,7 +454,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
 #pragma unroll
          for (int c = 0; c < 3; c++) {
             const long long q = pp + c * npts;
-            base[c] = FORM == 1 ? __ldg(a.up + q) : 2 * __ldg(a.u + q) - __ldg(a.um + q);
+            base[c] = FORM == 1 ? __ldg(a.up + q) : fma(2.0, __ldg(a.u + q), -__ldg(a.um + q));
          }
       }
       if (k < kend) fetch(k + 3);
@@ -699,7 +700,7 @@ int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
       fixed_stage_kernel<2><<<grid, block, smem, stream>>>(a);
    SW4G_TRY(launch_status());
    if (form == 0 || st.beta == 0) return kOk;
-   return launch_damping_lines(4, b, st.k1, st.k2, st.damp, st.u, st.um, st.out, st.rho, st.irho, st.dc, st.st, st.co,
+   return launch_damping_layers(4, b, st.k1, st.k2, st.u, st.um, st.out, st.rho, st.irho, st.dc, st.st, st.co,
                                st.beta, st.emax, stream);
 }
 
