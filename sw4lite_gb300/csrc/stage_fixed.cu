@@ -644,6 +644,30 @@ int launch_fixed_coef(const Box& b, const double* mu, const double* la, const do
    return launch_status();
 }
 
+// Planes per CTA.  A CTA's march costs its planes and about four more (two planes of ring
+// and two of z products at each end).  Launches that fill the resident slots more than
+// once cost their waves and a tail of CTAs finishing apart; ones that fit at once cost
+// their longest CTA, 1.3 times as much a plane as the share of a full GPU.  Against
+// stage_kchunk's rule (3.5 waves, at least 12 planes): 64^3 121 -> 70 us a stage, a step
+// at 48 x 40 x 36 363 -> 258 us, 101^3 752 -> 710 us, 512^3 unchanged.
+static int planes_per_cta(long long cols, int nk, int slots)
+{
+   if (stage_chunks_override() > 0) return stage_kchunk(cols, nk, 1, 1);
+   int best = nk;
+   double least = 1e30;
+   for (int c = 1; c <= nk; c++) {
+      const int per = (nk + c - 1) / c;
+      if (per < 2 && c > 1) break;
+      const double waves = (double)(cols * ((nk + per - 1) / per)) / slots;
+      const double cost = (per + 4) * (waves <= 1 ? 1.3 : waves + 0.7);
+      if (cost < least * 0.999) {
+         least = cost;
+         best = per;
+      }
+   }
+   return best;
+}
+
 int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
 {
    if (st.k2 < st.k1) return kOk;
@@ -683,14 +707,16 @@ int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
    int dev = 0;
    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kCudaError;
    static bool attr_set[3][64] = {};
-   static int resident[3][64] = {};
+   static int slots[3][64] = {};  // CTAs resident at once
    if (!attr_set[form][dev]) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      int sms = 0;
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
          return kCudaError;
-      resident[form][dev] = resident_ctas(kern, NTHREADS, smem);
+      slots[form][dev] = std::max(1, sms) * resident_ctas(kern, NTHREADS, smem);
       attr_set[form][dev] = true;
    }
-   a.kchunk = st.kchunk > 0 ? st.kchunk : stage_kchunk((long long)gx * gy, nk, resident[form][dev], 12);
+   a.kchunk = st.kchunk > 0 ? st.kchunk : planes_per_cta((long long)gx * gy, nk, slots[form][dev]);
    const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY, 1);
    if (form == 0)
       fixed_stage_kernel<0><<<grid, block, smem, stream>>>(a);
