@@ -621,7 +621,7 @@ constexpr int kRowThreads = 64;
 template <bool DF>
 __device__ __forceinline__ double rlvl(const GradRows& g, const double* d, const float* f, long long q)
 {
-   if (DF) return (double)__ldg(f + q) + (double)__ldg(f + q + g.lo);
+   if (DF) return df_value(__ldg(f + q), __ldg(f + q + g.lo));
    return __ldg(d + q);
 }
 

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "df.cuh"
+
 namespace sw4g {
 
 struct Box {
@@ -60,13 +62,14 @@ struct DFField {
    long long lo;  // offset of the lo half
    __device__ __forceinline__ double get(long long q) const
    {
-      return (double)h[q] + (double)h[q + lo];
+      return df_value(h[q], h[q + lo]);
    }
    __device__ __forceinline__ void set(long long q, double v) const
    {
-      const float a = __double2float_rn(v);
+      float a, b;
+      df_split(v, a, b);
       h[q] = a;
-      h[q + lo] = __double2float_rn(v - (double)a);
+      h[q + lo] = b;
    }
    __device__ __forceinline__ static void copy(const DFField& d, long long qd, const DFField& s,
                                                long long qs)

@@ -486,7 +486,7 @@ struct RdDF {
    long long lo;
    __device__ __forceinline__ double get(long long q) const
    {
-      return (double)__ldg(h + q) + (double)__ldg(h + q + lo);
+      return df_value(__ldg(h + q), __ldg(h + q + lo));
    }
 };
 

@@ -49,7 +49,7 @@ struct PtT {
    __device__ __forceinline__ double u(int c, int i, int j, int k) const
    {
       const long long q = cidx(a.bu, c, i, j, k);
-      if (DF) return (double)__ldg(a.udf + q) + (double)__ldg(a.udf + q + 3 * a.bu.npts);
+      if (DF) return df_value(__ldg(a.udf + q), __ldg(a.udf + q + 3 * a.bu.npts));
       return __ldg(a.u + q);
    }
    __device__ __forceinline__ double mu(int i, int j, int k) const
@@ -358,7 +358,7 @@ struct RowUpdate {
 template <bool DF>
 __device__ __forceinline__ double lvl(const double* d, const float* f, long long q, long long lo)
 {
-   if (DF) return (double)__ldg(f + q) + (double)__ldg(f + q + lo);
+   if (DF) return df_value(__ldg(f + q), __ldg(f + q + lo));
    return __ldg(d + q);
 }
 
@@ -424,14 +424,15 @@ __global__ void __launch_bounds__(256, 2) stage_rows_kernel(OpArgs a, RowUpdate 
          const double lu = a.cof * r[c];
          double v;
          if (w.corrector != 1)
-            v = 2 * lvl<DF>(w.u, w.udf, q, w.lo) - lvl<DF>(w.um, w.umdf, q, w.lo) + cr * lu;
+            v = fma(2.0, lvl<DF>(w.u, w.udf, q, w.lo), -lvl<DF>(w.um, w.umdf, q, w.lo)) + cr * lu;
          else
             v = lvl<DF>(w.up, w.updf, q, w.lo) + cr * lu;
          if (w.corrector != 0 && w.beta != 0) v -= birho * sg4_point<DF>(a.b, w, c, i, j, k);
          if (DF) {
-            const float hh = __double2float_rn(v);
+            float hh, ll;
+            df_split(v, hh, ll);
             w.outdf[q] = hh;
-            w.outdf[q + w.lo] = __double2float_rn(v - (double)hh);
+            w.outdf[q + w.lo] = ll;
          } else {
             w.out[q] = v;
          }

@@ -733,8 +733,8 @@ __global__ void df_slab_kernel(Box bx, int k0, int k1, const float* __restrict__
         q += (long long)gridDim.x * blockDim.x) {
       const int c = (int)(q / nslab);
       const long long p = q % nslab + bx.nij * (long long)(k0 - bx.kb) + c * bx.npts;
-      double v = (double)a[p] + (double)a[p + lo];
-      if (bsub) v -= (double)bsub[p] + (double)bsub[p + lo];
+      double v = df_value(a[p], a[p + lo]);
+      if (bsub) v -= df_value(bsub[p], bsub[p + lo]);
       out[q] = v;
    }
 }

@@ -114,3 +114,34 @@ def test_mixed_rejects_phase_mode():
     with pytest.raises(sg.Sw4gError):
         ew.step(1, sg.MODE_PHASES)
     ew.close()
+
+
+def test_level_conversions_round_as_the_types_do():
+    """The double-float halves of a level are float32(v) and float32(v - hi), and reading
+    a level back adds them in FP64: values over all exponents, ties, subnormal and
+    overflowing halves, signed zeros, infinities and NaN."""
+    nx, ny, nz = 40, 36, 38
+    g = sg.grid_desc(nx, ny, nz, 0.05, bc=(2,) * 6, sg_gp=6, precision=sg.MIXED)
+    ew = sg.EW(g)
+    n = 3 * ew.npts
+    rng = np.random.default_rng(12)
+    v = rng.choice([-1.0, 1.0], n) * np.ldexp(1.0 + rng.random(n), rng.integers(-1074, 1024, n))
+    half = n // 2
+    v[:half] = rng.choice([-1.0, 1.0], half) * np.ldexp(1.0 + rng.random(half), rng.integers(-130, 128, half))
+    tie = 1.0 + (2 * np.arange(64) + 1) * 2.0 ** -24  # half-way between two float32
+    v[:64] = tie
+    v[64:128] = -tie * (1 + 2.0 ** -52)
+    v[128:192] = tie + np.ldexp(1.0, -48) * np.arange(64)
+    v[192:200] = [0.0, -0.0, np.inf, -np.inf, np.nan, 2.0 ** -126, -2.0 ** -149, np.finfo(np.float32).max * (1 + 2.0 ** -25)]
+    with np.errstate(over="ignore", invalid="ignore"):
+        hi = v.astype(np.float32)
+        lo = (v - hi.astype(np.float64)).astype(np.float32)
+        want = hi.astype(np.float64) + lo.astype(np.float64)
+    ew.set_fields(dev(v), dev(v))
+    out = dev(np.zeros(n))
+    ew.get_fields(out, None)
+    got = host(out)
+    ew.close()
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    ok = ~np.isnan(want)
+    assert np.array_equal(got[ok].view(np.int64), want[ok].view(np.int64))
