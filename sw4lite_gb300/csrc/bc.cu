@@ -1,9 +1,12 @@
 // Ghost-point closures on a Cartesian grid, sm_103a: the replacement for the
 // reference's bcfortsg / bcfortsg_indrev (src/ew-cfromfort.C:205-746).
 //
-// Sides are processed in order 0..5 on the caller's stream, one launch per active
-// side, because windows of later sides overlap earlier ones at edges and the
-// free-surface solve reads ghost values written by the lateral sides.
+// Sides are processed in order 0..5 on the caller's stream, because windows of later sides
+// overlap earlier ones at edges and the free-surface solve reads ghost values written by
+// the lateral sides.  Without boundary data and periodic sides every window is zero, their
+// order does not matter and none meets what a free surface reads or writes in z: one launch
+// for all of them (a step at 48 x 40 x 36 spent 25 us on ten launches of 2.5 us), then the
+// free surfaces.
 //   bccnd 1 (Dirichlet) / 2 (supergrid): copy the boundary data into the 2 ghost
 //     planes of the side's window (zero when no data array is given);
 //   bccnd 3 (periodic): copy from the point one period inside;
@@ -32,6 +35,28 @@ __global__ void fill_window_kernel(Box b, Win w, Field u, const double* __restri
       const int i = w.i0 + (int)(r % idel);
 #pragma unroll
       for (int c = 0; c < 3; c++) u.set(cidx(b, c, i, j, k), bforce ? bforce[3 * q + c] : 0.0);
+   }
+}
+
+// The windows of up to six sides set to zero; win n's points follow those before it.
+struct Zeros {
+   Win w[6];
+   unsigned end[6];
+   int n;
+};
+
+template <class Field>
+__global__ void zero_windows_kernel(Box b, Zeros z, Field u)
+{
+   const unsigned total = z.end[z.n - 1];
+   for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
+      int n = 0;
+      while (q >= z.end[n]) n++;
+      const Win w = z.w[n];
+      const unsigned r = q - (n ? z.end[n - 1] : 0), idel = w.i1 - w.i0 + 1, jdel = w.j1 - w.j0 + 1;
+      const int i = w.i0 + (int)(r % idel), j = w.j0 + (int)(r / idel % jdel), k = w.k0 + (int)(r / idel / jdel);
+#pragma unroll
+      for (int c = 0; c < 3; c++) u.set(cidx(b, c, i, j, k), 0.0);
    }
 }
 
@@ -114,10 +139,30 @@ int bc_sides(int soa, int ib, int ie, int jb, int je, int kb, int ke, const int 
                     cudaStream_t s)
 {
    Box b = make_box(soa, ib, ie, jb, je, kb, ke);
+   bool zeros = true;
+   for (int side = 0; side < 6; side++) zeros = zeros && bccnd[side] != 3 && (!bforce || !bforce[side] || bccnd[side] == 0);
+   Zeros z;
+   z.n = 0;
+   long long points = 0;
+   for (int side = 0; side < 6 && zeros; side++) {
+      const int* w6 = wind + 6 * side;
+      const Win w{w6[0], w6[1], w6[2], w6[3], w6[4], w6[5]};
+      if ((bccnd[side] != 1 && bccnd[side] != 2) || w.i1 < w.i0 || w.j1 < w.j0 || w.k1 < w.k0) continue;
+      if (w.i0 < ib || w.i1 > ie || w.j0 < jb || w.j1 > je || w.k0 < kb || w.k1 > ke) return kBadArgument;
+      points += (long long)(w.i1 - w.i0 + 1) * (w.j1 - w.j0 + 1) * (w.k1 - w.k0 + 1);
+      if (points > 0x7fffffffLL) {  // beyond the kernel's 32-bit count
+         zeros = false;
+         break;
+      }
+      z.w[z.n] = w;
+      z.end[z.n++] = (unsigned)points;
+   }
+   if (zeros && z.n > 0) zero_windows_kernel<<<small_grid(points), 256, 0, s>>>(b, z, u);
    for (int side = 0; side < 6; side++) {
       const int* w6 = wind + 6 * side;
       Win w{w6[0], w6[1], w6[2], w6[3], w6[4], w6[5]};
       const int t = bccnd[side];
+      if (zeros && (t == 1 || t == 2)) continue;
       if (t == 1 || t == 2 || t == 3) {
          if (w.i1 < w.i0 || w.j1 < w.j0 || w.k1 < w.k0) continue;
          if (w.i0 < ib || w.i1 > ie || w.j0 < jb || w.j1 > je || w.k0 < kb || w.k1 > ke)

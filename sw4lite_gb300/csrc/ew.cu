@@ -1232,12 +1232,15 @@ int EW::profile_kernels(int nrep, double ms[4])
 
 int EW::launches_per_step(int mode) const
 {
-   int bc = 0;
+   int bc = 0, zero_sides = 0;  // the zero sides of a grid without periodic ones are one launch
+   bool periodic = false;
    for (int s = 0; s < 6; s++) {
       const int t = g_.bc[s];
-      if ((t == kDirichlet || t == kSuperGrid || t == kPeriodic) && bcpts_[s] > 0) bc++;
+      if ((t == kDirichlet || t == kSuperGrid || t == kPeriodic) && bcpts_[s] > 0) zero_sides++;
       if (t == kStressFree) bc++;
+      periodic = periodic || t == kPeriodic;
    }
+   bc += periodic ? zero_sides : zero_sides > 0 ? 1 : 0;
    const int rows = onesided_[4] + onesided_[5];
    const int src = hsrc_.empty() ? 0 : 1;
    const bool damp = prof_.used && g_.sg_damping != 0;
@@ -1252,7 +1255,7 @@ int EW::launches_per_step(int mode) const
    // form adds an FP64 slab of the predictor's field and of the corrector's u - um
    const int mslabs = mixed_ ? rows * (1 + (damp ? 1 : 0)) : 0;
    // and each rows launch its per-column pass
-   return 2 * (2 + 2 * rows + src + bc) + rows + (damp && g_.sg_order == 6 ? 1 : 0) + rec + mslabs +
+   return 2 * (2 + 2 * rows + src + bc) + rows + (damp && (g_.sg_order == 6 || fc_.w) ? 1 : 0) + rec + mslabs +
           curv_launches(mode);
 }
 

@@ -506,11 +506,14 @@ int EW::curv_time_step(double cfl, double* dt)
 int EW::curv_launches(int mode) const
 {
    if (!cv_) return 0;
-   int bc = 1 /* free surface */ + 1 /* interface copy */;
+   int bc = 1 /* free surface */ + 1 /* interface copy */, zero_sides = 0;
+   bool periodic = false;
    for (int s = 0; s < 4; s++) {
       const int t = cv_->bc[s];
-      if ((t == kDirichlet || t == kSuperGrid || t == kPeriodic) && cv_->bcpts[s] > 0) bc++;
+      if ((t == kDirichlet || t == kSuperGrid || t == kPeriodic) && cv_->bcpts[s] > 0) zero_sides++;
+      periodic = periodic || t == kPeriodic;
    }
+   bc += periodic ? zero_sides : zero_sides > 0 ? 1 : 0;
    bc++;  // flat free surface of bcfortsg on the top side
    const bool damp = prof_.used && g_.sg_damping != 0;
    // predictor (both modes): shell, top-row column pass, top rows, stage kernel;
