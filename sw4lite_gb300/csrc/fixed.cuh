@@ -127,6 +127,30 @@ struct Factor {
    }
 };
 
+// x * f / 2^e for |x| < 2^61 and any finite factor f, with its full relative precision,
+// rounded to nearest; f / 2^e is below 1 in magnitude.
+struct Scale {
+   int hi, lo, e;
+   bool neg;
+   __device__ __forceinline__ explicit Scale(double f)
+   {
+      const int h = __double2hiint(f), eb = (h >> 20) & 0x7ff;
+      const int mh = eb == 0 ? 0 : (h & 0xfffff) | 0x100000;  // below the normal range: 0
+      const i64 c = (i64)(((unsigned long long)mh << 32) | (eb == 0 ? 0u : (unsigned)__double2loint(f))) << 4;
+      hi = (int)(c >> kSplit);
+      lo = (int)(c & kMask) << 5;
+      e = eb == 0 ? -5000 : eb - 1022;
+      neg = h < 0;
+   }
+   __device__ __forceinline__ i64 operator()(i64 x) const
+   {
+      const int xh = (int)(x >> 31), xl = (int)x & 0x7fffffff;
+      const i64 cross = madw(xl, hi, madw(xh, lo, (madw(xl, lo, 1LL << 30) >> 31) + (1LL << 30)));
+      const i64 r = madw(xh, hi, cross >> 31);
+      return neg ? -r : r;
+   }
+};
+
 // A value |v| < 2^e as such a coefficient, C = v * 2^(57 - e) rounded.
 __device__ __forceinline__ int2 to_coef(double v, int e)
 {

@@ -414,6 +414,11 @@ int launch_uacc_slab(const Box& b, int k0, int k1, const double* up, const doubl
                      const double* um, double* out, cudaStream_t s);
 int launch_fused_stage(const FusedStage& st, cudaStream_t stream);
 int launch_fixed_stage(const FusedStage& st, cudaStream_t stream);
+// planes per CTA of a fixed-point march of cols CTA columns over nk planes
+int planes_per_cta(long long cols, int nk, int slots);
+// lu = L(u) on the centred rows k1..k2 (operator_fixed.cu)
+int launch_operator_fixed(const Box& b, int k1, int k2, double* lu, const double* u, const double* mu, const double* la,
+                          double h, const double* sx, const double* sy, const double* sz, cudaStream_t s);
 int launch_stage_rows(int corrector, bool top, const Box& b, int nk, const double* field,
                       const Box& field_box, const double* mu, const double* la, double h,
                       const double* strx, const double* stry, const double* strz,

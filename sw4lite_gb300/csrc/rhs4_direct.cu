@@ -1,10 +1,10 @@
-// One-thread-per-point sm_103a kernels for the Cartesian operator rhs4sg:
-// the centred rows and the one-sided SBP boundary rows, AoS or SoA layout.
+// One-thread-per-point sm_103a kernels for the one-sided SBP boundary rows of the
+// Cartesian operator rhs4sg, AoS or SoA layout.
 //
-// They serve the kernel-level drop-in entry point (sw4g_rhs4sg, the replacement
-// for the reference's rhs4sg / rhs4sg_rev, src/EW.C:141-149) for any bounds and
-// onesided flags, and are the baseline the fused z-marching stage kernels
-// (stage_fused.cu) are checked against.
+// With the centred rows' kernel (operator_fixed.cu) they serve the kernel-level drop-in
+// entry point (sw4g_rhs4sg, the replacement for the reference's rhs4sg / rhs4sg_rev,
+// src/EW.C:141-149) for any bounds and onesided flags; fused with the update they are the
+// time loop's rows.
 #include <algorithm>
 
 #include "common.cuh"
@@ -112,36 +112,6 @@ __device__ __forceinline__ void field_stencil(const P_& P, int ax, int c, int i,
 #pragma unroll
    for (int m = -2; m <= 2; m++)
       f[m + 2] = P.u(c, i + (ax == 0) * m, j + (ax == 1) * m, k + (ax == 2) * m);
-}
-
-__global__ void __launch_bounds__(256) rhs4_center_kernel(OpArgs a, int k1)
-{
-   const int i = a.b.ib + 2 + blockIdx.x * blockDim.x + threadIdx.x;
-   const int j = a.b.jb + 2 + blockIdx.y * blockDim.y + threadIdx.y;
-   const int k = k1 + blockIdx.z;
-   if (i > a.b.ie - 2 || j > a.b.je - 2) return;
-   Pt P(a);
-   const double i6 = 1.0 / 6, i144 = 1.0 / 144;
-   const double sx = P.s(0, i), sy = P.s(1, j), sz = P.s(2, k);
-   double am[3][5], bm[3][5];
-   for (int ax = 0; ax < 3; ax++) coef_stencil(P, ax, i, j, k, am[ax], bm[ax]);
-   double r[3];
-   for (int c = 0; c < 3; c++) {
-      double f[5], acc = 0;
-      for (int ax = 0; ax < 3; ax++) {
-         field_stencil(P, ax, c, i, j, k, f);
-         const double sa = ax == 0 ? sx : ax == 1 ? sy : sz;
-         acc += sa * d2var(ax == c ? bm[ax] : am[ax], f);
-      }
-      r[c] = i6 * acc;
-   }
-   r[0] += i144 * (sx * sy * (mixed(P, true, 0, 1, 1, i, j, k) + mixed(P, false, 1, 0, 1, i, j, k)) +
-                   sx * sz * (mixed(P, true, 0, 2, 2, i, j, k) + mixed(P, false, 2, 0, 2, i, j, k)));
-   r[1] += i144 * (sx * sy * (mixed(P, false, 0, 1, 0, i, j, k) + mixed(P, true, 1, 0, 0, i, j, k)) +
-                   sy * sz * (mixed(P, true, 1, 2, 2, i, j, k) + mixed(P, false, 2, 1, 2, i, j, k)));
-   r[2] += i144 * (sx * sz * (mixed(P, false, 0, 2, 0, i, j, k) + mixed(P, true, 2, 0, 0, i, j, k)) +
-                   sy * sz * (mixed(P, false, 1, 2, 1, i, j, k) + mixed(P, true, 2, 1, 1, i, j, k)));
-   for (int c = 0; c < 3; c++) a.lu[cidx(a.b, c, i, j, k)] = a.cof * r[c];
 }
 
 // One-sided rows.  Row r=0..5 is k=1+r (top) or k=nk-5+r (bottom); the SBP table
@@ -487,8 +457,7 @@ int launch_rhs4sg_direct(int soa, int ifirst, int ilast, int jfirst, int jlast, 
    const int k1 = onesided[4] == 1 ? 7 : kfirst + 2;
    const int k2 = onesided[5] == 1 ? nk - 6 : klast - 2;
    if (k2 >= k1) {
-      const dim3 grid(blocks_for(ni, 32), blocks_for(nj, 8), k2 - k1 + 1);
-      rhs4_center_kernel<<<grid, block, 0, stream>>>(a, k1);
+      SW4G_TRY(launch_operator_fixed(a.b, k1, k2, lu, u, mu, la, h, strx, stry, strz, stream));
    }
    if (onesided[4] == 1) {
       const dim3 grid(blocks_for(ni, 32), blocks_for(nj, 8), 6);

@@ -650,7 +650,7 @@ int launch_fixed_coef(const Box& b, const double* mu, const double* la, const do
 // their longest CTA, 1.3 times as much a plane as the share of a full GPU.  Against
 // stage_kchunk's rule (3.5 waves, at least 12 planes): 64^3 121 -> 70 us a stage, a step
 // at 48 x 40 x 36 363 -> 258 us, 101^3 752 -> 710 us, 512^3 unchanged.
-static int planes_per_cta(long long cols, int nk, int slots)
+int planes_per_cta(long long cols, int nk, int slots)
 {
    if (stage_chunks_override() > 0) return stage_kchunk(cols, nk, 1, 1);
    int best = nk;

@@ -134,3 +134,59 @@ def test_bcfortsg(soa, bccnd):
                                     C.cast(sb, sg._D), dmu.data_ptr(), dla.data_ptr(), ptrs,
                                     dsx.data_ptr(), dsy.data_ptr(), stream()))
     assert rel_err(host(du), ref) <= 1e-14
+
+
+def _operator(g, soa, u, mu, la, st):
+    lu = dev(np.zeros_like(u))
+    d = [dev(a) for a in (u, mu, la, *st)]
+    sg.check(sg.lib().sw4g_rhs4sg(soa, *g.bounds, g.nz, _onesided(0, 0), lu.data_ptr(), d[0].data_ptr(), d[1].data_ptr(),
+                                  d[2].data_ptr(), g.h, *[t.data_ptr() for t in d[3:]], stream()))
+    return host(lu)
+
+
+@pytest.mark.parametrize("soa", [1, 0])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (31, 5, 3), (32, 6, 2), (33, 7, 41), (65, 13, 14)])
+@pytest.mark.parametrize("profile", ["ones", "layers", "any"])
+def test_operator_tiles_and_profiles(soa, shape, profile):
+    """Extents at the edges of the operator's 32 x 6 column tiles and of its marches, and
+    stretching profiles of 1, falling to 1e-4 at the sides, and of any sign and size with
+    zeros.  Both sides form sums of about 80 products, each within a few 2^-53 of the
+    largest, (2 mu + lambda) |s|^2 |u| / h^2 times weights that add to less than 64: they
+    differ by less than 2^-46 of 64 such terms."""
+    g = Grid(*shape, h=0.37)
+    rng = np.random.default_rng(sum(shape) + soa)
+    u = g.field3(rng)
+    _, mu, la = g.material(rng, spread=0.9)
+    st = []
+    for n in (g.ni, g.nj, g.nk):
+        s = np.ones(n)
+        if profile == "layers":
+            s = np.maximum(1e-4, np.minimum(1, (np.abs(np.arange(n) - n / 2) / (n / 2) - 1) ** 2))
+        if profile == "any":
+            s = rng.choice([-1.0, 1.0], n) * np.ldexp(1 + rng.random(n), rng.integers(-30, 30, n))
+            s[:: max(2, n // 3)] = 0
+        st.append(np.ascontiguousarray(s))
+    ref = np.zeros_like(u)
+    O.rhs4sg(soa, g.bounds, g.nz, [0] * 6, ref, u, mu, la, g.h, *st)
+    got = _operator(g, soa, u, mu, la, st)
+    big = max(np.max(np.abs(s)) for s in st)
+    scale = 64 * np.max(2 * mu + la) * big * big * np.max(np.abs(u)) / g.h ** 2
+    assert np.max(np.abs(got - ref)) <= 2.0 ** -46 * scale
+
+
+@pytest.mark.parametrize("where", ["u", "mu", "sz"])
+def test_operator_non_finite_inputs(where):
+    g = Grid(40, 20, 22, h=0.3)
+    rng = np.random.default_rng(3)
+    u = g.field3(rng)
+    _, mu, la = g.material(rng)
+    st = list(g.stretching(rng))
+    if where == "u":
+        u.reshape(3, g.nk, g.nj, g.ni)[1, 12, 9, 20] = np.inf
+    elif where == "mu":
+        mu.reshape(g.nk, g.nj, g.ni)[12, 9, 20] = np.nan
+    else:
+        st[2][11] = np.nan
+    ref = np.zeros_like(u)
+    O.rhs4sg(1, g.bounds, g.nz, [0] * 6, ref, u, mu, la, g.h, *st)
+    assert np.array_equal(np.isfinite(_operator(g, 1, u, mu, la, st)), np.isfinite(ref))
