@@ -12,7 +12,8 @@
 // multiplies which component, and the 1/sx, 1/sy factors, are the reference's;
 // they are tabulated in kCross / kSame below.
 //
-// These are the kernel-level entry points (one thread per point) and the
+// These are the kernel-level entry points (one thread per point; the operator's rows away
+// from the SBP top are in curv_operator.cu) and the
 // set-up kernels of a curvilinear grid: metric, grid over a Gaussian hill, the
 // curvilinear free-surface ghost plane (freesurfcurvisg, src/curvilinear-c.C:621),
 // supergrid damping in x, y (addsgd4cfort, src/ew-cfromfort.C:1160/1323) and the
@@ -172,7 +173,6 @@ __device__ __forceinline__ double d2v(const double c[5], const double f[5])
           (1.0 / 6);
 }
 
-template <bool BND>
 __device__ void curv_point(const CurvView& a, int i, int j, int k, double r[3])
 {
    const double sxc = a.SX(i), syc = a.SY(j);
@@ -198,28 +198,17 @@ __device__ void curv_point(const CurvView& a, int i, int j, int k, double r[3])
    for (int c = 0; c < 3; c++)
 #pragma unroll
       for (int d = 0; d < 3; d++) {
-         double s = 0;
-         if (!BND) {
-            double cf[5], f[5];
+         double s = 0, cm[8];
 #pragma unroll
-            for (int m = -2; m <= 2; m++) {
-               cf[m + 2] = a.rr(c, d, i, j, k + m, sxc, syc);
-               f[m + 2] = a.U(d, i, j, k + m);
-            }
-            s = d2v(cf, f);
-         } else {
-            double cm[8];
+         for (int m = 1; m <= 8; m++) cm[m - 1] = a.rr(c, d, i, j, m, sxc, syc);
 #pragma unroll
-            for (int m = 1; m <= 8; m++) cm[m - 1] = a.rr(c, d, i, j, m, sxc, syc);
+         for (int q = 1; q <= 8; q++) {
+            double cq = 0;
 #pragma unroll
-            for (int q = 1; q <= 8; q++) {
-               double cq = 0;
-#pragma unroll
-               for (int m = 1; m <= 8; m++) cq += c_acof[(k - 1) + 6 * (q - 1) + 48 * (m - 1)] * cm[m - 1];
-               s += cq * a.U(d, i, j, q);
-            }
-            s += c_ghcof[k - 1] * cm[0] * a.U(d, i, j, 0);
+            for (int m = 1; m <= 8; m++) cq += c_acof[(k - 1) + 6 * (q - 1) + 48 * (m - 1)] * cm[m - 1];
+            s += cq * a.U(d, i, j, q);
          }
+         s += c_ghcof[k - 1] * cm[0] * a.U(d, i, j, 0);
          r[c] += rs[c][d] * s;
       }
 #pragma unroll
@@ -229,9 +218,8 @@ __device__ void curv_point(const CurvView& a, int i, int j, int k, double r[3])
          const XTerm& t = kCross[c][pr];
          if (t.n == 0) continue;
          const int ao = kOuter[pr], ai = kInner[pr];
-         const bool bo = BND && ao == 2, bi = BND && ai == 2;
-         constexpr int NQ = BND ? 8 : 5;
-         double G[NQ];
+         const bool bo = ao == 2, bi = ai == 2;
+         double G[8];
 #pragma unroll
          for (int s = 0; s < (bo ? 8 : 5); s++) {
             int ii = i, jj = j, kk = k;
@@ -277,7 +265,7 @@ __device__ void curv_point(const CurvView& a, int i, int j, int k, double r[3])
    r[2] *= ijac;
 }
 
-template <bool BND>
+// The SBP rows k1..k2 at the top
 __global__ void __launch_bounds__(128) rhs4sgcurv_kernel(CurvView a, double* __restrict__ lu,
                                                          int k1, int k2)
 {
@@ -286,7 +274,7 @@ __global__ void __launch_bounds__(128) rhs4sgcurv_kernel(CurvView a, double* __r
    const int k = k1 + blockIdx.z;
    if (i > a.b.ie - 2 || j > a.b.je - 2 || k > k2) return;
    double r[3];
-   curv_point<BND>(a, i, j, k, r);
+   curv_point(a, i, j, k, r);
    const long long q = a.p(i, j, k);
 #pragma unroll
    for (int c = 0; c < 3; c++) lu[c * a.b.cs + a.b.ps * q] = r[c];
@@ -554,16 +542,11 @@ int launch_rhs4sgcurv(const CurvSpec& s, const int onesided[6], double* lu, cuda
    if (top) {
       if (s.kb > 0 || s.ke < 8) return kBadArgument;  // the closure reads planes 0..8
       const dim3 g((ni + 31) / 32, (nj + 3) / 4, 6);
-      rhs4sgcurv_kernel<true><<<g, blk, 0, st>>>(v, lu, 1, 6);
+      rhs4sgcurv_kernel<<<g, blk, 0, st>>>(v, lu, 1, 6);
       SW4G_TRY(launch_status());
       k1 = 7;
    }
-   const int k2 = s.ke - 2;
-   if (k2 >= k1) {
-      const dim3 g((ni + 31) / 32, (nj + 3) / 4, k2 - k1 + 1);
-      rhs4sgcurv_kernel<false><<<g, blk, 0, st>>>(v, lu, k1, k2);
-   }
-   return launch_status();
+   return launch_curv_operator(s, k1, s.ke - 2, lu, st);
 }
 
 int launch_rhs4sgcurv_top(const CurvSpec& s, double* lu, cudaStream_t st)
@@ -574,7 +557,7 @@ int launch_rhs4sgcurv_top(const CurvSpec& s, double* lu, cudaStream_t st)
    const int ni = s.ie - s.ib - 3, nj = s.je - s.jb - 3;
    if (ni <= 0 || nj <= 0) return kOk;
    const dim3 blk(32, 4), g((ni + 31) / 32, (nj + 3) / 4, 6);
-   rhs4sgcurv_kernel<true><<<g, blk, 0, st>>>(v, lu, 1, 6);
+   rhs4sgcurv_kernel<<<g, blk, 0, st>>>(v, lu, 1, 6);
    return launch_status();
 }
 

@@ -158,6 +158,8 @@ struct CurvSpec {
 };
 
 int launch_rhs4sgcurv(const CurvSpec& s, const int onesided[6], double* lu, cudaStream_t st);
+// its rows k1..k2 away from the SBP top (curv_operator.cu)
+int launch_curv_operator(const CurvSpec& s, int k1, int k2, double* lu, cudaStream_t st);
 // only the SBP top rows k = 1..6 of the curvilinear operator
 int launch_rhs4sgcurv_top(const CurvSpec& s, double* lu, cudaStream_t st);
 
