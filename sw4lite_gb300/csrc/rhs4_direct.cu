@@ -368,10 +368,8 @@ __device__ __forceinline__ double sg4_point(const Box& b, const RowUpdate& w, in
 }
 
 // DF: the levels (and, when the stage field is not an FP64 slab, the field) are
-// double-float pairs; FDF: the stage field is double-float.
-// DF: the levels (and, when the stage field is not an FP64 slab, the field) are
 // double-float pairs; FDF: the stage field is double-float.  The gx x gy x 6 blocks
-// of 32 x 8 points are strided over by the grid (one CTA per block, or fewer CTAs,
+// of 32 x 8 or 32 x 4 points are strided over by the grid (one CTA per block, or fewer CTAs,
 // each taking several: a persistent grid beside a stage kernel).
 template <bool TOP, bool DF, bool FDF, bool PRE>
 __global__ void __launch_bounds__(256, 2) stage_rows_kernel(OpArgs a, RowUpdate w, int gx, int gy)
@@ -587,8 +585,13 @@ int launch_stage_rows_df(int corrector, bool top, const Box& b, int nz, const do
    }
    const int ni = b.ie - b.ib - 3, nj = b.je - b.jb - 3;
    if (ni <= 0 || nj <= 0) return kOk;
-   const int gx = blocks_for(ni, 32), gy = blocks_for(nj, 8);
-   const dim3 block(32, 8, 1), grid(ctas > 0 ? std::min(ctas, gx * gy * 6) : gx * gy * 6);
+   // Beside the stage kernel fed by tensor copies (i extents that are multiples of 4), whose
+   // nine warps leave registers for four more on an SM: CTAs of four (CTAs of eight waited for
+   // the stage to end; steps of 320^3 11.4 -> 9.8 ms a call of two).  Beside the other one,
+   // which leaves room for eight, CTAs of eight (steps at ragged sizes 727 -> 715 us a call).
+   const int by = ctas > 0 && b.ni % 4 == 0 ? 4 : 8;
+   const int gx = blocks_for(ni, 32), gy = blocks_for(nj, by);
+   const dim3 block(32, by, 1), grid(ctas > 0 ? std::min(ctas, gx * gy * 6) : gx * gy * 6);
    if (rscr) {  // the per-column terms once, then the rows read them
       a.dzc = rscr;
       a.roc = rscr + 18 * b.nij;

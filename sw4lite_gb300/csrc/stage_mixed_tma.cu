@@ -7,23 +7,33 @@
 // pairs after the staging, so every plane's DRAM latency is exposed (it measured
 // 28-31 % of HBM bandwidth with 5-9 long-scoreboard stalls per issue).  Here every
 // input of a plane arrives by bulk tensor copies (cp.async.bulk.tensor) completed on
-// shared-memory mbarriers, issued by one thread one or more planes ahead:
+// shared-memory mbarriers, issued one or more planes ahead by a warp of their own (a
+// plane's 18 to 22 copies issued by a computing warp held the others at the next barrier):
 //
 //  * F(m), the stage fields of plane m over the CTA's 36 x 12 halo tile: one 4-D box
 //    {36, 12, 1, 6} per level (hi of the 3 components, then lo) lands as the
 //    staged plane itself.  Predictor: a 6-slot ring of u planes (k-2..k+2 in use,
 //    k+3 in flight).  Corrector: one raw slot of up, u, um, transformed into the
-//    rounded stage field up - 2u + um (5-plane ring) and the damping field u - um
-//    (3-plane ring) two planes ahead of the compute.  F(m) also brings mu, lambda
+//    rounded stage field up - 2u + um (6-plane ring) and the damping field u - um
+//    (4-plane ring) two planes ahead of the compute.  F(m) also brings mu, lambda
 //    at the CTA's own points, for the z-flux G_z(m) computed right after it lands.
 //  * M(m), everything plane m's compute reads once: mu, lambda (hi, lo) over the
 //    halo tile, rho (corrector), the own points of the update level (up or um),
 //    1/rho, and the twelve second-difference weight arrays over the extents each
-//    axis needs (x: 34 columns, y: 10 rows, z: planes m..m+2).  Two stages: M(k+1)
-//    is in flight while plane k computes.
+//    axis needs (x: 34 columns, y: 10 rows, z: the one plane, m+1 or m+2, that the
+//    registers do not hold from the planes before).  Two stages: M(k+1) is in flight
+//    while plane k computes.
 //
-// One CTA of 32 x 8 threads per SM (~205 KB of shared memory): the copies in
-// flight, not resident warps, hide the DRAM latency.  Tensor copies need 16-byte
+// One CTA of 32 x 8 columns per SM (168 or 192 KB of shared memory): the copies in
+// flight, not resident warps, hide the DRAM latency.  Eight computing warps meet at two
+// barriers a plane; the rings have a slot more than the stencil reads, so that none is
+// needed between a plane's sums and the next plane's arrival.  What bounds it is the
+// latency of those eight warps: 50 % of the issue slots, 47 % of the DRAM rate.  320^3:
+// predictor 1.87 -> 1.59 ms, corrector 2.38 -> 1.90 ms with the producer warp, the z
+// weights in registers, the barrier less and the outer products dealt to the warps
+// together.  Sixteen computing warps (two threads a column) measured 1.81 and 2.15 ms and
+// left no registers for the one-sided rows' CTAs, which run beside: 128 registers a thread
+// leave room for four warps of them (step of 320^3 by two steps a call 10.65 -> 9.11 ms).  Tensor copies need 16-byte
 // aligned row strides, so the launcher takes this path when the array's i extent
 // is a multiple of 4 and falls back to the synchronous kernel otherwise.  Every
 // mbarrier wait gives up after one second: the kernel then records kTimeout in the
@@ -47,7 +57,8 @@ constexpr int TX = 32, TY = 8, HALO = 2;
 constexpr int PX = TX + 2 * HALO;  // 36
 constexpr int PY = TY + 2 * HALO;  // 12
 constexpr int PLANE = PX * PY;     // 432
-constexpr int NTHREADS = TX * TY;
+constexpr int NCOMP = TX * TY;        // threads that compute, one per column
+constexpr int NTHREADS = NCOMP + 32;  // and the warp that issues the copies
 constexpr int OWNP = PX * TY;      // 288: own rows of a tile with the x halo (columns 0..35)
 
 constexpr unsigned long long kWaitLimitNs = 1000000000ull;  // 1 s per mbarrier wait
@@ -62,8 +73,7 @@ struct TmaMaps {
    CUtensorMap ir_own;            // {72,8,1}
    CUtensorMap wx[4];             // {72,8,1}
    CUtensorMap wy[4];             // {72,10,1}
-   CUtensorMap wz1[2];            // {72,8,3}: W1 of the z axis, types 0, 1
-   CUtensorMap wz2[2];            // {72,8,2}: W2 of the z axis
+   CUtensorMap wz[4];             // {72,8,1}: W1, W2 of the z axis, types 0, 1
 };
 
 struct TmaArgs {
@@ -71,6 +81,7 @@ struct TmaArgs {
    long long ni, nij, npts;
    int k1, k2, kchunk;
    float* __restrict__ out;
+   const float2* __restrict__ wz[4];  // z-axis weights (the first planes' plain loads)
    const float* __restrict__ rho;  // z-damping neighbours (plain loads)
    const float* __restrict__ sx;
    const float* __restrict__ sy;
@@ -90,8 +101,6 @@ constexpr int kPairHaloB = 72 * 12 * 4;      // 3456
 constexpr int kPairOwnB = 72 * 8 * 4;        // 2304
 constexpr int kRhoHaloB = align128(36 * 12 * 4);  // 1792
 constexpr int kWyB = align128(72 * 10 * 4);  // 2944
-constexpr int kWz1B = 72 * 8 * 3 * 4;        // 6912
-constexpr int kWz2B = 72 * 8 * 2 * 4;        // 4608
 
 // M stage
 template <int CORR>
@@ -103,12 +112,10 @@ struct MLayout {
    static constexpr int ir = own + kLevOwnB;
    static constexpr int wx = ir + kPairOwnB;
    static constexpr int wy = wx + 4 * kPairOwnB;
-   static constexpr int wz1 = wy + 4 * kWyB;
-   static constexpr int wz2 = wz1 + 2 * kWz1B;
-   static constexpr int bytes = wz2 + 2 * kWz2B;
+   static constexpr int wz = wy + 4 * kWyB;
+   static constexpr int bytes = wz + 4 * kPairOwnB;
    static constexpr unsigned tx_bytes = 2 * 72 * 12 * 4 + (CORR ? 36 * 12 * 4 : 0) + kLevOwnB +
-                                        kPairOwnB + 4 * kPairOwnB + 4 * 72 * 10 * 4 +
-                                        2 * kWz1B + 2 * kWz2B;
+                                        kPairOwnB + 4 * kPairOwnB + 4 * 72 * 10 * 4 + 4 * kPairOwnB;
 };
 
 // whole CTA
@@ -122,11 +129,11 @@ struct Layout {
    static constexpr int m0 = fown + 2 * kPairOwnB;
    static constexpr int m1 = m0 + M::bytes;
    static constexpr int vh = m1 + M::bytes;                 // corrector: stage field ring
-   static constexpr int dd = vh + (CORR ? 15 * PLANE * 4 : 0);
-   static constexpr int gx = dd + (CORR ? 9 * PLANE * 4 : 0);
+   static constexpr int dd = vh + (CORR ? 18 * PLANE * 4 : 0);
+   static constexpr int gx = dd + (CORR ? 12 * PLANE * 4 : 0);
    static constexpr int gy = gx + 3 * TY * PX * 4;
    static constexpr int bar = align128(gy + 3 * PY * TX * 4);
-   static constexpr int bytes = bar + 3 * 8 + 8;            // F barrier, M barriers, abort flag
+   static constexpr int bytes = bar + 3 * 8;                // F barrier, M barriers
    static constexpr unsigned f_tx = (CORR ? 3 : 1) * kLevHaloB + 2 * kPairOwnB;
 };
 static_assert(Layout<1>::bytes <= 227 * 1024, "corrector layout exceeds shared memory");
@@ -205,12 +212,16 @@ __device__ __forceinline__ void fence_async_shared()
    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-__device__ __forceinline__ int mod5(int k) { return ((k % 5) + 5) % 5; }
-__device__ __forceinline__ int mod3(int k) { return ((k % 3) + 3) % 3; }
+// Barrier of the computing warps
+__device__ __forceinline__ void sync_compute()
+{
+   asm volatile("bar.sync 1, %0;" ::"n"(NCOMP) : "memory");
+}
+
 __device__ __forceinline__ int mod6(int k) { return ((k % 6) + 6) % 6; }
 
 template <int CORR>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __maxnreg__(128)
     mixed_stage_tma_kernel(const __grid_constant__ TmaMaps tm, const TmaArgs a)
 {
    using L = Layout<CORR>;
@@ -220,7 +231,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
    float* GY = reinterpret_cast<float*>(smb + L::gy);  // [3][PY][TX]
    const uint32_t barF = smem_u32(smb + L::bar);
    const uint32_t barM0 = barF + 8;
-   volatile int* abort_flag = reinterpret_cast<volatile int*>(smb + L::bar + 24);
 
    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + TX * ty;
    const int i0 = a.ib + 2 + blockIdx.x * TX;
@@ -270,25 +280,43 @@ __global__ void __launch_bounds__(NTHREADS, 1)
          tma3(s + M::wx + q * kPairOwnB, &tm.wx[q], 2 * xt, yo, z, bar);
          tma3(s + M::wy + q * kWyB, &tm.wy[q], 2 * xt, yo, z, bar);
       }
-      for (int t = 0; t < 2; t++) {
-         tma3(s + M::wz1 + t * kWz1B, &tm.wz1[t], 2 * xt, yo, z, bar);
-         tma3(s + M::wz2 + t * kWz2B, &tm.wz2[t], 2 * xt, yo, z, bar);
-      }
+      for (int q = 0; q < 4; q++)
+         tma3(s + M::wz + q * kPairOwnB, &tm.wz[q], 2 * xt, yo, z + (q & 1 ? 1 : 2), bar);
    };
 
    if (tid == 0) {
       mbar_init(barF, 1);
       mbar_init(barM0, 1);
       mbar_init(barM0 + 8, 1);
-      *abort_flag = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       fence_async_shared();
    }
    __syncthreads();
 
+   const int kfin = kend + 2;  // last plane the stencil reads
+   if (threadIdx.y == TY) {
+      // The producer: at each barrier (A) the computing warps have read what the copies
+      // issued next overwrite.  A wait that gave up ends every thread at the next (A).
+      if (tx == 0) {
+         issue_M(kbeg);
+         issue_F(kbeg - 2);
+      }
+      for (int k = kbeg - 4; k <= kend; k++) {
+         if (__syncthreads_or(0)) return;  // (A)
+         if (tx == 0) {
+            fence_async_shared();
+            if (k + 3 <= kfin) issue_F(k + 3);
+            if (k >= kbeg && k + 1 <= kend) issue_M(k + 1);
+         }
+         __syncwarp();
+      }
+      return;
+   }
+
    uint32_t fphase = 0, mphase = 0;  // mphase bit s: parity of M stage s
+   int gave_up = 0;
    auto fail = [&]() {
-      *abort_flag = 1;
+      gave_up = 1;
       if (a.status) atomicOr(a.status, 1 << kTimeout);
    };
    auto wait_F = [&]() {
@@ -303,22 +331,22 @@ __global__ void __launch_bounds__(NTHREADS, 1)
    // stage-field planes: hi/lo rings (predictor: the F ring itself) or the
    // transformed FP32 ring (corrector)
    auto vh_plane = [&](int kk) -> const float* {
-      if (CORR) return reinterpret_cast<const float*>(smb + L::vh) + mod5(kk) * 3 * PLANE;
+      if (CORR) return reinterpret_cast<const float*>(smb + L::vh) + mod6(kk) * 3 * PLANE;
       return reinterpret_cast<const float*>(smb + L::f + mod6(kk) * kLevHaloB);
    };
    auto vl_plane = [&](int kk) -> const float* {  // predictor only
       return reinterpret_cast<const float*>(smb + L::f + mod6(kk) * kLevHaloB) + 3 * PLANE;
    };
    auto dd_plane = [&](int kk) -> float* {  // corrector only
-      return reinterpret_cast<float*>(smb + L::dd) + mod3(kk) * 3 * PLANE;
+      return reinterpret_cast<float*>(smb + L::dd) + (kk & 3) * 3 * PLANE;
    };
 
    // corrector: raw (up, u, um) slot -> rounded up - 2u + um and u - um
    auto transform = [&](int kk) {
       const float* raw = reinterpret_cast<const float*>(smb + L::f);
-      float* vs = reinterpret_cast<float*>(smb + L::vh) + mod5(kk) * 3 * PLANE;
+      float* vs = reinterpret_cast<float*>(smb + L::vh) + mod6(kk) * 3 * PLANE;
       float* ds = dd_plane(kk);
-      for (int idx = tid; idx < PLANE; idx += NTHREADS) {
+      for (int idx = tid; idx < PLANE; idx += NCOMP) {
 #pragma unroll
          for (int c = 0; c < 3; c++) {
             const int q = c * PLANE + idx;
@@ -377,25 +405,22 @@ __global__ void __launch_bounds__(NTHREADS, 1)
    };
 
    float gz[5][3], dq[5][3];
-   const int kfin = kend + 2;  // last plane the stencil reads
-
+   float2 wz1[2][2], wz2[2];  // z-axis W1(k), W1(k+1) and W2(k) of both coefficient types
+   if (active)
+      for (int t = 0; t < 2; t++) {
+         const long long p = gidx(i, j, kbeg);
+         wz1[t][0] = __ldg(a.wz[2 * t] + p);
+         wz1[t][1] = __ldg(a.wz[2 * t] + p + a.nij);
+         wz2[t] = __ldg(a.wz[2 * t + 1] + p);
+      }
    // ---- prologue: planes kbeg-2 .. kbeg+1 into the rings, M(kbeg) in flight ----
-   if (tid == 0) {
-      issue_M(kbeg);
-      issue_F(kbeg - 2);
-   }
 #pragma unroll
    for (int q = 1; q <= 4; q++) {  // slots 1..4 hold planes kbeg-2..kbeg+1
       const int kk = kbeg - 3 + q;
       wait_F();
       if (CORR) transform(kk);
       read_own_material();
-      __syncthreads();
-      if (*abort_flag) return;
-      if (tid == 0) {
-         fence_async_shared();
-         issue_F(kk + 1);
-      }
+      if (__syncthreads_or(gave_up)) return;  // (A)
       if (active) compute_gz(kk, gz[q]);
       if (CORR) {
          const float* dd = dd_plane(kk);
@@ -409,13 +434,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       wait_F();
       if (CORR) transform(k + 2);
       read_own_material();
-      __syncthreads();  // (A)
-      if (*abort_flag) return;
-      if (tid == 0) {
-         fence_async_shared();
-         if (k + 3 <= kfin) issue_F(k + 3);
-         if (k + 1 <= kend) issue_M(k + 1);
-      }
+      if (__syncthreads_or(gave_up)) return;  // (A)
 #pragma unroll
       for (int q = 0; q < 4; q++) {
 #pragma unroll
@@ -451,8 +470,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
          return d1(hm2 + o, lm2 + o, s, hm1 + o, lm1 + o, s, hp1 + o, lp1 + o, s, hp2 + o, lp2 + o, s);
       };
 
-      // x-outer products over 36 x 8, y-outer products over 32 x 12
-      for (int idx = tid; idx < TY * PX; idx += NTHREADS) {
+      // x-outer products over 36 x 8, y-outer products over 32 x 12: 9 + 12 warps' work, dealt
+      // to the 8 warps together (three rounds; two after two took four)
+      auto x_outer = [&](int idx) {
          const int li = idx % PX, ljr = idx / PX;
          const int s = (ljr + HALO) * PX + li;
          const int gi = i0 - HALO + li, gj = j0 + ljr;
@@ -472,8 +492,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
          GX[idx] = g0;
          GX[TY * PX + idx] = g1;
          GX[2 * TY * PX + idx] = g2;
-      }
-      for (int idx = tid; idx < PY * TX; idx += NTHREADS) {
+      };
+      auto y_outer = [&](int idx) {
          const int lic = idx % TX, lj = idx / TX;
          const int s = lj * PX + lic + HALO;
          const int gi = i0 + lic, gj = j0 - HALO + lj;
@@ -493,17 +513,20 @@ __global__ void __launch_bounds__(NTHREADS, 1)
          GY[idx] = g0;
          GY[PY * TX + idx] = g1;
          GY[2 * PY * TX + idx] = g2;
+      };
+#pragma unroll 1
+      for (int w = ty; w < (TY * PX + PY * TX) / 32; w += TY) {
+         if (w < TY * PX / 32) x_outer(32 * w + tx);
+         else y_outer(32 * w + tx - TY * PX);
       }
-      __syncthreads();  // (B)
-      if (*abort_flag) return;
+      sync_compute();  // (B)
 
       if (active) {
          const long long p = gidx(i, j, k);
          // W1(q), W2(q), W2(q+1), W1(q+2) per axis and coefficient type, as (hi, lo)
          const float2* wxs = reinterpret_cast<const float2*>(ms + M::wx);
          const float2* wys = reinterpret_cast<const float2*>(ms + M::wy);
-         const float2* wz1 = reinterpret_cast<const float2*>(ms + M::wz1);
-         const float2* wz2 = reinterpret_cast<const float2*>(ms + M::wz2);
+         const float2* wzs = reinterpret_cast<const float2*>(ms + M::wz);
          float wth[3][2][4], wtl[3][2][4];
 #pragma unroll
          for (int t = 0; t < 2; t++) {
@@ -513,9 +536,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const float2* y1 = wys + (2 * t) * (kWyB / 8);
             const float2* y2 = wys + (2 * t + 1) * (kWyB / 8);
             const float2 r0 = y1[ownr], r1 = y2[ownr], r2 = y2[ownr + PX], r3 = y1[ownr + 2 * PX];
-            const float2* z1 = wz1 + t * (kWz1B / 8);
-            const float2* z2 = wz2 + t * (kWz2B / 8);
-            const float2 s0 = z1[ownr], s1 = z2[ownr], s2 = z2[ownr + OWNP], s3 = z1[ownr + 2 * OWNP];
+            const float2 s0 = wz1[t][0], s1 = wz2[t], s2 = wzs[(2 * t + 1) * OWNP + ownr],
+                         s3 = wzs[2 * t * OWNP + ownr];
+            wz1[t][0] = wz1[t][1];
+            wz1[t][1] = s3;
+            wz2[t] = s2;
             wth[0][t][0] = q0.x; wth[0][t][1] = q1.x; wth[0][t][2] = q2.x; wth[0][t][3] = q3.x;
             wtl[0][t][0] = q0.y; wtl[0][t][1] = q1.y; wtl[0][t][2] = q2.y; wtl[0][t][3] = q3.y;
             wth[1][t][0] = r0.x; wth[1][t][1] = r1.x; wth[1][t][2] = r2.x; wth[1][t][3] = r3.x;
@@ -639,7 +664,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             }
          }
       }
-      __syncthreads();  // (C): GX/GY, M stage k and the oldest ring slot are free
    }
 }
 
@@ -787,10 +811,7 @@ int launch_mixed_stage_tma(const MixedStage& st, cudaStream_t stream)
    for (int q = 0; q < 4; q++) {
       SW4G_TRY(encode(scalar_key(b, st.w2[q], 1, 72, 8, 1), &tm.wx[q]));
       SW4G_TRY(encode(scalar_key(b, st.w2[4 + q], 1, 72, 10, 1), &tm.wy[q]));
-   }
-   for (int t = 0; t < 2; t++) {
-      SW4G_TRY(encode(scalar_key(b, st.w2[8 + 2 * t], 1, 72, 8, 3), &tm.wz1[t]));
-      SW4G_TRY(encode(scalar_key(b, st.w2[9 + 2 * t], 1, 72, 8, 2), &tm.wz2[t]));
+      SW4G_TRY(encode(scalar_key(b, st.w2[8 + q], 1, 72, 8, 1), &tm.wz[q]));
    }
 
    TmaArgs a;
@@ -799,6 +820,7 @@ int launch_mixed_stage_tma(const MixedStage& st, cudaStream_t stream)
    a.k1 = st.k1;
    a.k2 = st.k2;
    a.out = st.out;
+   for (int q = 0; q < 4; q++) a.wz[q] = reinterpret_cast<const float2*>(st.w2[8 + q]);
    a.rho = st.rho;
    a.sx = st.st[0];
    a.sy = st.st[1];
@@ -834,7 +856,7 @@ int launch_mixed_stage_tma(const MixedStage& st, cudaStream_t stream)
       }
    }
    a.kchunk = stage_kchunk((long long)gx * gy, nk, resident[corr][dev], 12);
-   const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY, 1);
+   const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY + 1, 1);
    if (corr)
       mixed_stage_tma_kernel<1><<<grid, block, smem, stream>>>(tm, a);
    else

@@ -75,3 +75,17 @@ def test_unaligned_extent_keeps_the_synchronous_kernel():
     got_u, _ = _run(shape, bc, True)
     want_u, _ = _run(shape, bc, False)
     assert np.array_equal(got_u, want_u)
+
+
+@pytest.mark.parametrize("chunks", [1, 7, 40])
+def test_marches_of_any_length_agree(chunks):
+    """The copies' ring, barriers and the z weights carried from plane to plane restart with
+    each march: one march, ragged ones and one plane each give the same bits."""
+    shape, bc = (60, 21, 40), (2, 2, 2, 2, 0, 2)
+    want = _run(shape, bc, True, nsteps=2)
+    sg.set_stage_chunks(chunks)
+    try:
+        got = _run(shape, bc, True, nsteps=2)
+    finally:
+        sg.set_stage_chunks(0)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
