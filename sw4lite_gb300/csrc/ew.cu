@@ -1017,6 +1017,7 @@ int EW::mixed_piece(int piece, int ip, int iq)
          ms.co[q] = prof32_[6 + q];
       }
       ms.h = g_.h;
+      ms.alone = cv_ == nullptr;
       ms.dt = dt;
       ms.u = u;
       ms.um = um;

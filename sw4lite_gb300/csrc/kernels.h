@@ -92,6 +92,9 @@ struct MixedStage {
    // corrector 0 predictor, 1 corrector, 2 adjoint form (stage_mixed.cu); coef != 0
    // replaces the stage's dt^2 (predictor, adjoint) or dt^2/12 (corrector)
    double coef = 0;
+   // no other stage or persistent grid of topography runs meanwhile: the planes per CTA
+   // may count on the whole GPU (stage_mixed.cu)
+   bool alone = false;
    // device status word: the tensor-copy kernels or in 1 << kTimeout when an
    // mbarrier wait gives up (may be null)
    int* status = nullptr;

@@ -648,7 +648,13 @@ int launch_mixed_stage(const MixedStage& st, cudaStream_t stream)
       resident[st.corrector][dev] = resident_ctas(kern, NTHREADS, smem);
       attr_set[st.corrector][dev] = true;
    }
-   a.kchunk = stage_kchunk((long long)gx * gy, nk, resident[st.corrector][dev], 12);
+   // Alone, marches as planes_per_cta has them (two steps of 157 x 90 x 75 points 712 -> 648 us
+   // a call).  Beside the curvilinear grid's rows, whose persistent CTAs take a share of each
+   // SM, and beside a second sweep of the gradient, many short ones (a topography grid's two
+   // steps 2.02 ms a call; 2.43 with planes_per_cta's few long ones).
+   const long long cols = (long long)gx * gy;
+   a.kchunk = st.alone ? planes_per_cta(cols, nk, 152 * resident[st.corrector][dev])
+                       : stage_kchunk(cols, nk, resident[st.corrector][dev], 12);
    const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY, 1);
    if (st.corrector == 1)
       mixed_stage_kernel<1><<<grid, block, smem, stream>>>(a);
