@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(NTHREADS, 3) curv_mixed_kernel(MArgs a)
          return d1(vm2 + o, vm1 + o, vp1 + o, vp2 + o, LOFF, s, s, s, s);
       };
       // p-outer products over the x-extended rows
-      for (int idx = tid; idx < TY * PX; idx += NTHREADS) {
+      auto x_outer = [&](int idx) {
          const int li = idx % PX, ljr = idx / PX;
          const int s = (ljr + HALO) * PX + li;
          const int gi = i0 - HALO + li, gj = j0 + ljr;
@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(NTHREADS, 3) curv_mixed_kernel(MArgs a)
          GX[idx] = g0;
          GX[TY * PX + idx] = g1;
          GX[2 * TY * PX + idx] = g2;
-      }
+      };
       // q-outer products over the y-extended columns
-      for (int idx = tid; idx < PY * TX; idx += NTHREADS) {
+      auto y_outer = [&](int idx) {
          const int lic = idx % TX, lj = idx / TX;
          const int s = lj * PX + lic + HALO;
          const int gi = i0 + lic, gj = j0 - HALO + lj;
@@ -263,6 +263,12 @@ __global__ void __launch_bounds__(NTHREADS, 3) curv_mixed_kernel(MArgs a)
          GY[idx] = g0;
          GY[PY * TX + idx] = g1;
          GY[2 * PY * TX + idx] = g2;
+      };
+      // 9 + 12 warps' work, dealt to the 8 warps together (three rounds; two after two took four)
+#pragma unroll 1
+      for (int w = ty; w < (TY * PX + PY * TX) / 32; w += TY) {
+         if (w < TY * PX / 32) x_outer(32 * w + tx);
+         else y_outer(32 * w + tx - TY * PX);
       }
       __syncthreads();
 
