@@ -16,7 +16,10 @@
 // Each cross term D_a(C D_b u) is an outer difference of per-point products
 // G = C D_b u: G for the p (q) outer difference is staged in shared memory over
 // the x (y) halo, G for the r outer difference rides a register queue, as in the
-// Cartesian kernel.  The kernel covers the rows k = 7..nz under an SBP top; the six
+// Cartesian kernel.  The FP64 pipe bounds it, so each instruction counts: reciprocals
+// of the stretching once per tile, its factors on the differences, sums by fused
+// multiply-adds, the damping's inputs only where a layer reaches (192 x 192 columns: predictor
+// 656 -> 569 us, corrector 866 -> 737).  The kernel covers the rows k = 7..nz under an SBP top; the six
 // top rows and the ghost shell are done by curv_edge_kernel from the one-sided
 // operator of curv.cu.
 #include <algorithm>
@@ -128,8 +131,8 @@ struct StageArgs {
 
 __host__ __device__ constexpr int stage_smem(int corr)
 {
-   // V ring (5 x 3 planes) + [D plane (3) + RJ plane] + GX + GY
-   return 15 * PLANE + (corr ? 4 * PLANE : 0) + 3 * TY * PX + 3 * PY * TX;
+   // V ring (5 x 3 planes) + [D plane (3) + RJ plane] + GX + GY + 1/sx, 1/sy of the tile
+   return 15 * PLANE + (corr ? 4 * PLANE : 0) + 3 * TY * PX + 3 * PY * TX + PX + PY;
 }
 
 __device__ __forceinline__ int m5(int k) { return ((k % 5) + 5) % 5; }
@@ -143,6 +146,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
    double* RJ = DP + (CORR ? 3 * PLANE : 0);    // [PLANE]    (corrector, plane k)
    double* GX = RJ + (CORR ? PLANE : 0);        // [3][TY][PX]
    double* GY = GX + 3 * TY * PX;               // [3][PY][TX]
+   double* ISX = GY + 3 * PY * TX;              // [PX] 1/sx
+   double* ISY = ISX + PX;                      // [PY] 1/sy
    const Box& b = a.b;
    const long long n = b.npts;
    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + TX * ty;
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                if (!CORR) v[c] = __ldg(a.u + p + c * n);
-               else v[c] = (__ldg(a.up + p + c * n) - 2 * __ldg(a.u + p + c * n)) + __ldg(a.um + p + c * n);
+               else v[c] = fma(-2.0, __ldg(a.u + p + c * n), __ldg(a.up + p + c * n)) + __ldg(a.um + p + c * n);
             }
          }
 #pragma unroll
@@ -190,7 +195,17 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
    };
    const double sxi = active ? __ldg(a.sx + (i - b.ib)) : 1.0;
    const double syj = active ? __ldg(a.sy + (j - b.jb)) : 1.0;
-   const double isxi = 1 / sxi, isyj = 1 / syj;
+   if (tid < PX && i0 - HALO + tid <= b.ie) ISX[tid] = 1 / __ldg(a.sx + (i0 - HALO + tid - b.ib));
+   if (tid < PY && j0 - HALO + tid <= b.je) ISY[tid] = 1 / __ldg(a.sy + (j0 - HALO + tid - b.jb));
+   __syncthreads();
+   const double isxi = active ? ISX[HALO + tx] : 1.0, isyj = active ? ISY[HALO + ty] : 1.0;
+   const double sxy = sxi * isyj, syx = syj * isxi;
+   // does a damping layer reach into the CTA's columns?
+   int layer = 0;
+   if (CORR && active && a.beta != 0)
+      for (int m = -1; m <= 1; m++)
+         layer |= nonzero_bits(__ldg(a.dcx + (i + m - b.ib))) || nonzero_bits(__ldg(a.dcy + (j + m - b.jb)));
+   if (CORR) layer = __syncthreads_or(layer);
    auto P = [&](int t, long long p) { return __ldg(a.cc.prod[t] + p); };
 
    // r-outer products of the own column at plane kk (inner p and q differences)
@@ -206,11 +221,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
       const long long p = gidx(i, j, kk);
       const double p21m = P(2, p), p21l = P(3, p), p31m = P(4, p), p31l = P(5, p), p41m = P(6, p),
                    p41l = P(7, p);
-      g[0] = (2 * p21m + p21l) * sxi * isyj * dp[0] + p31m * dp[1] + p41m * isyj * dp[2] +
-             p31m * syj * isxi * dq[0] + p21l * dq[1];
-      g[1] = p31l * dp[0] + p21m * sxi * isyj * dp[1] + p21m * dq[0] +
-             (2 * p31m + p31l) * syj * isxi * dq[1] + p41m * isxi * dq[2];
-      g[2] = isyj * (p41l * dp[0] + p21m * sxi * dp[2]) + isxi * (p31m * syj * dq[2] + p41l * dq[1]);
+      g[0] = fma(2.0, p21m, p21l) * (sxy * dp[0]) + p31m * (dp[1] + syx * dq[0]) + p41m * (isyj * dp[2]) +
+             p21l * dq[1];
+      g[1] = p31l * dp[0] + p21m * (dq[0] + sxy * dp[1]) + fma(2.0, p31m, p31l) * (syx * dq[1]) +
+             p41m * (isxi * dq[2]);
+      g[2] = p41l * (isyj * dp[0] + isxi * dq[1]) + p21m * (sxy * dp[2]) + p31m * (syx * dq[2]);
    };
 
    double gz[5][3];
@@ -222,7 +237,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
 
    for (int k = kbeg; k <= kend; k++) {
       load_plane(k + 2);
-      if (CORR) load_damping(k);
+      if (CORR && layer) load_damping(k);
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < 4; q++)
@@ -246,8 +261,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
          double g0 = 0, g1 = 0, g2 = 0;
          if (gi <= b.ie && gj <= b.je) {
             const long long p = gidx(gi, gj, k);
-            const double sxx = __ldg(a.sx + (gi - b.ib)), syy = __ldg(a.sy + (gj - b.jb));
-            const double isy = 1 / syy;
+            const double isy = ISY[ljr + HALO], sxy = __ldg(a.sx + (gi - b.ib)) * isy;
             double dq[3], drr[3];
 #pragma unroll
             for (int c = 0; c < 3; c++) {
@@ -257,9 +271,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
             }
             const double p11m = P(0, p), p11l = P(1, p), p21m = P(2, p), p21l = P(3, p),
                          p31m = P(4, p), p31l = P(5, p), p41m = P(6, p), p41l = P(7, p);
-            g0 = p11l * dq[1] + isy * ((2 * p21m + p21l) * sxx * drr[0] + p31l * syy * drr[1] + p41l * drr[2]);
-            g1 = p11m * dq[0] + p31m * drr[0] + p21m * sxx * isy * drr[1];
-            g2 = isy * (p41m * drr[0] + p21m * sxx * drr[2]);
+            g0 = p11l * dq[1] + fma(2.0, p21m, p21l) * (sxy * drr[0]) + p31l * drr[1] + p41l * (isy * drr[2]);
+            g1 = p11m * dq[0] + p31m * drr[0] + p21m * (sxy * drr[1]);
+            g2 = p41m * (isy * drr[0]) + p21m * (sxy * drr[2]);
          }
          GX[idx] = g0;
          GX[TY * PX + idx] = g1;
@@ -273,8 +287,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
          double g0 = 0, g1 = 0, g2 = 0;
          if (gi <= b.ie && gj <= b.je) {
             const long long p = gidx(gi, gj, k);
-            const double sxx = __ldg(a.sx + (gi - b.ib)), syy = __ldg(a.sy + (gj - b.jb));
-            const double isx = 1 / sxx;
+            const double isx = ISX[lic + HALO], syx = __ldg(a.sy + (gj - b.jb)) * isx;
             double dpp[3], drr[3];
 #pragma unroll
             for (int c = 0; c < 3; c++) {
@@ -284,9 +297,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
             }
             const double p11m = P(0, p), p11l = P(1, p), p21m = P(2, p), p21l = P(3, p),
                          p31m = P(4, p), p31l = P(5, p), p41m = P(6, p), p41l = P(7, p);
-            g0 = p11m * dpp[1] + p31m * syy * isx * drr[0] + p21m * drr[1];
-            g1 = p11l * dpp[0] + p21l * drr[0] + (2 * p31m + p31l) * syy * isx * drr[1] + p41l * isx * drr[2];
-            g2 = isx * (p31m * syy * drr[2] + p41m * drr[1]);
+            g0 = p11m * dpp[1] + p31m * (syx * drr[0]) + p21m * drr[1];
+            g1 = p11l * dpp[0] + p21l * drr[0] + fma(2.0, p31m, p31l) * (syx * drr[1]) + p41l * (isx * drr[2]);
+            g2 = p31m * (syx * drr[2]) + p41m * (isx * drr[1]);
          }
          GY[idx] = g0;
          GY[PY * TX + idx] = g1;
@@ -314,8 +327,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
                   if (!use) continue;
                   const double* f = v0 + c * PLANE + own;
                   const int st = ax == 0 ? 1 : PX;
-                  s3[c] += w0 * (f[-2 * st] - f[0]) + w1 * (f[-st] - f[0]) + w2 * (f[st] - f[0]) +
-                           w3 * (f[2 * st] - f[0]);
+                  s3[c] = fma(w3, f[2 * st] - f[0], fma(w2, f[st] - f[0], fma(w1, f[-st] - f[0], fma(w0, f[-2 * st] - f[0], s3[c]))));
                }
             }
          }
@@ -327,13 +339,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
             const int dd = t < 7 ? t - 4 : (t == 7 ? 1 : 2);
             const double w0 = __ldg(a.cc.w[2 * t] + p), w1 = __ldg(a.cc.w[2 * t + 1] + p),
                          w2 = __ldg(a.cc.w[2 * t + 1] + p + o), w3 = __ldg(a.cc.w[2 * t] + p + 2 * o);
-            auto rr = [&](int comp) {
+            auto rr = [&](int comp, double t0) {
                const int s = comp * PLANE + own;
                const double f0 = v0[s];
-               return w0 * (vm2[s] - f0) + w1 * (vm1[s] - f0) + w2 * (vp1[s] - f0) + w3 * (vp2[s] - f0);
+               return fma(w3, vp2[s] - f0, fma(w2, vp1[s] - f0, fma(w1, vm1[s] - f0, fma(w0, vm2[s] - f0, t0))));
             };
-            s3[cc] += rr(dd);
-            if (cc != dd) s3[dd] += rr(cc);
+            s3[cc] = rr(dd, s3[cc]);
+            if (cc != dd) s3[dd] = rr(cc, s3[dd]);
          }
          // cross terms: outer differences of the staged products
 #pragma unroll
@@ -350,33 +362,32 @@ __global__ void __launch_bounds__(NTHREADS, 2) curv_stage_kernel(StageArgs a)
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                const long long q = p + c * n;
-               a.out[q] = 2 * v0[c * PLANE + own] - __ldg(a.um + q) + kk * s3[c];
+               a.out[q] = fma(2.0, v0[c * PLANE + own], -__ldg(a.um + q)) + kk * s3[c];
             }
          } else {
             double sg[3] = {0, 0, 0};
-            if (a.beta != 0) {
+            if (layer) {
                const double cxi = __ldg(a.cox + (i - b.ib)), cyj = __ldg(a.coy + (j - b.jb));
                const double dx0 = __ldg(a.dcx + (i - 1 - b.ib)), dx1 = __ldg(a.dcx + (i - b.ib)),
                             dx2 = __ldg(a.dcx + (i + 1 - b.ib));
                if (nonzero_bits(dx0) || nonzero_bits(dx1) || nonzero_bits(dx2)) {  // integer pipe
-                  const double e0 = RJ[own - 1] * dx0, e1 = RJ[own] * dx1, e2 = RJ[own + 1] * dx2;
+                  const double e0 = RJ[own - 1] * dx0, e1 = 2 * (RJ[own] * dx1), e2 = RJ[own + 1] * dx2, wx = sxi * cyj;
 #pragma unroll
                   for (int c = 0; c < 3; c++) {
                      const double* d = DP + c * PLANE + own;
-                     sg[c] += sxi * cyj * (e2 * (d[2] - 2 * d[1] + d[0]) - 2 * e1 * (d[1] - 2 * d[0] + d[-1]) +
-                                           e0 * (d[0] - 2 * d[-1] + d[-2]));
+                     sg[c] += wx * (e2 * (fma(-2.0, d[1], d[2]) + d[0]) - e1 * (fma(-2.0, d[0], d[1]) + d[-1]) +
+                                    e0 * (fma(-2.0, d[-1], d[0]) + d[-2]));
                   }
                }
                const double dy0 = __ldg(a.dcy + (j - 1 - b.jb)), dy1 = __ldg(a.dcy + (j - b.jb)),
                             dy2 = __ldg(a.dcy + (j + 1 - b.jb));
                if (nonzero_bits(dy0) || nonzero_bits(dy1) || nonzero_bits(dy2)) {
-                  const double e0 = RJ[own - PX] * dy0, e1 = RJ[own] * dy1, e2 = RJ[own + PX] * dy2;
+                  const double e0 = RJ[own - PX] * dy0, e1 = 2 * (RJ[own] * dy1), e2 = RJ[own + PX] * dy2, wy = syj * cxi;
 #pragma unroll
                   for (int c = 0; c < 3; c++) {
                      const double* d = DP + c * PLANE + own;
-                     sg[c] += syj * cxi * (e2 * (d[2 * PX] - 2 * d[PX] + d[0]) -
-                                           2 * e1 * (d[PX] - 2 * d[0] + d[-PX]) +
-                                           e0 * (d[0] - 2 * d[-PX] + d[-2 * PX]));
+                     sg[c] += wy * (e2 * (fma(-2.0, d[PX], d[2 * PX]) + d[0]) - e1 * (fma(-2.0, d[0], d[PX]) + d[-PX]) +
+                                    e0 * (fma(-2.0, d[-PX], d[0]) + d[-2 * PX]));
                   }
                }
             }
@@ -499,7 +510,7 @@ struct TopArgs {
    WR out;
    CurvCoef cc;
    const double* __restrict__ topw;
-   // per column: one-sided r derivatives DR[(k-1)*3 + c] and r-outer sums
+   // per column: 12 times the one-sided r derivatives DR[(k-1)*3 + c] and r-outer sums
    // RO[(k-1)*3 + c] of rows k = 1..6 (curv_top_pre_kernel), 18 x ncol each
    const double* __restrict__ dr;
    const double* __restrict__ ro;
@@ -525,8 +536,6 @@ __global__ void __launch_bounds__(128) curv_top_pre_kernel(Box b, Box fb, SF f, 
    const long long ncol = b.nij;
    auto F = [&](int c, int ii, int jj, int kk) { return f.get(c * fb.npts + pidx(fb, ii, jj, kk)); };
    auto Pr = [&](int t, long long q) { return __ldg(cc.prod[t] + q); };
-   const double i12 = 1.0 / 12;
-   auto cd = [&](double fm2, double fm1, double fp1, double fp2) { return i12 * d1c(fm2, fm1, fp1, fp2); };
    for (long long col = blockIdx.x * (long long)blockDim.x + threadIdx.x; col < ncol;
         col += (long long)gridDim.x * blockDim.x) {
       const int i = b.ib + (int)(col % b.ni), j = b.jb + (int)(col / b.ni);
@@ -540,12 +549,12 @@ __global__ void __launch_bounds__(128) curv_top_pre_kernel(Box b, Box fb, SF f, 
             double s = 0;
 #pragma unroll
             for (int q = 1; q <= 8; q++) s += t_bope[(k - 1) + 6 * (q - 1)] * fq[q - 1];
-            dr[((k - 1) * 3 + c) * ncol + col] = s;
+            dr[((k - 1) * 3 + c) * ncol + col] = 12 * s;
          }
       }
       if (i < b.ib + 2 || i > b.ie - 2 || j < b.jb + 2 || j > b.je - 2) continue;
       const double sxc = __ldg(sx + (i - b.ib)), syc = __ldg(sy + (j - b.jb));
-      const double istrx = 1 / sxc, istry = 1 / syc;
+      const double istrx = 1 / sxc, istry = 1 / syc, sxy = sxc * istry, syx = syc * istrx;
       double acc[6][3];
 #pragma unroll
       for (int k = 0; k < 6; k++) acc[k][0] = acc[k][1] = acc[k][2] = 0;
@@ -555,16 +564,16 @@ __global__ void __launch_bounds__(128) curv_top_pre_kernel(Box b, Box fb, SF f, 
          double dp[3], dq[3];
 #pragma unroll
          for (int c = 0; c < 3; c++) {
-            dp[c] = cd(F(c, i - 2, j, qq), F(c, i - 1, j, qq), F(c, i + 1, j, qq), F(c, i + 2, j, qq));
-            dq[c] = cd(F(c, i, j - 2, qq), F(c, i, j - 1, qq), F(c, i, j + 1, qq), F(c, i, j + 2, qq));
+            dp[c] = d1c(F(c, i - 2, j, qq), F(c, i - 1, j, qq), F(c, i + 1, j, qq), F(c, i + 2, j, qq));
+            dq[c] = d1c(F(c, i, j - 2, qq), F(c, i, j - 1, qq), F(c, i, j + 1, qq), F(c, i, j + 2, qq));
          }
          const double p21m = Pr(2, q), p21l = Pr(3, q), p31m = Pr(4, q), p31l = Pr(5, q),
                       p41m = Pr(6, q), p41l = Pr(7, q);
-         const double g0 = (2 * p21m + p21l) * sxc * istry * dp[0] + p31m * dp[1] + p41m * istry * dp[2] +
-                           p31m * syc * istrx * dq[0] + p21l * dq[1];
-         const double g1 = p31l * dp[0] + p21m * sxc * istry * dp[1] + p21m * dq[0] +
-                           (2 * p31m + p31l) * syc * istrx * dq[1] + p41m * istrx * dq[2];
-         const double g2 = istry * (p41l * dp[0] + p21m * sxc * dp[2]) + istrx * (p31m * syc * dq[2] + p41l * dq[1]);
+         const double g0 = fma(2.0, p21m, p21l) * (sxy * dp[0]) + p31m * (dp[1] + syx * dq[0]) + p41m * (istry * dp[2]) +
+                           p21l * dq[1];
+         const double g1 = p31l * dp[0] + p21m * (dq[0] + sxy * dp[1]) + fma(2.0, p31m, p31l) * (syx * dq[1]) +
+                           p41m * (istrx * dq[2]);
+         const double g2 = p41l * (istry * dp[0] + istrx * dq[1]) + p21m * (sxy * dp[2]) + p31m * (syx * dq[2]);
 #pragma unroll
          for (int k = 0; k < 6; k++) {
             const double bw = t_bope[k + 6 * (qq - 1)];
@@ -576,26 +585,82 @@ __global__ void __launch_bounds__(128) curv_top_pre_kernel(Box b, Box fb, SF f, 
 #pragma unroll
       for (int k = 0; k < 6; k++)
 #pragma unroll
-         for (int c = 0; c < 3; c++) ro[(k * 3 + c) * ncol + col] = acc[k][c];
+         for (int c = 0; c < 3; c++) ro[(k * 3 + c) * ncol + col] = (1.0 / 12) * acc[k][c];
    }
 }
 
 // Rows k = 1..6 under the SBP top: the one-sided operator from precomputed
 // coefficients, with the stage update (and the corrector's x/y damping) fused.
-// FP64 throughout; the levels are FP64 or double-float (RD, WR).
+// FP64 throughout; the levels are FP64 or double-float (RD, WR).  A block of 32 x 4 points
+// of a row forms the products of the p and q outer differences, 12 G, over its 36 x 4 and
+// 32 x 8 points in shared memory (at four neighbours of every point anew, and with four
+// divisions a point, they were two thirds of the kernel's FP64 work, which bounds it: 192 x 192 columns,
+// predictor 162 -> 111 us, corrector 187 -> 137).
+constexpr int RX = 32, RY = 4, RPX = RX + 4, RPY = RY + 4;
+
+struct TopSmem {
+   double gx[3][RY * RPX], gy[3][RPY * RX];
+   double isx[RX], isy[RY];
+};
+
+template <class RD, class WR, class SF>
+__device__ __forceinline__ void curv_top_products(const TopArgs<RD, WR, SF>& a, TopSmem& sm, int i0, int j0, int k)
+{
+   const Box& b = a.b;
+   const Box& fb = a.fb;
+   const long long ncol = b.nij;
+   auto F = [&](int c, int ii, int jj) { return a.f.get(c * fb.npts + pidx(fb, ii, jj, k)); };
+   auto DR = [&](int c, int ii, int jj) { return __ldg(a.dr + ((k - 1) * 3 + c) * ncol + pidx(b, ii, jj, b.kb)); };
+   const int tid = threadIdx.x + RX * threadIdx.y;
+   if (tid < RX) sm.isx[tid] = i0 + tid <= b.ie ? 1 / __ldg(a.sx + (i0 + tid - b.ib)) : 0;
+   else if (tid < RX + RY) sm.isy[tid - RX] = j0 + tid - RX <= b.je ? 1 / __ldg(a.sy + (j0 + tid - RX - b.jb)) : 0;
+   __syncthreads();
+   for (int idx = tid; idx < RY * RPX + RPY * RX; idx += RX * RY) {
+      if (idx < RY * RPX) {  // p-outer: QP (central) + RP (one-sided r)
+         const int lj = idx / RPX, ii = i0 - 2 + idx % RPX, jj = j0 + lj;
+         if (ii > b.ie || jj > b.je - 2) continue;
+         const long long q = pidx(b, ii, jj, k);
+         const double isy = sm.isy[lj], sxy = __ldg(a.sx + (ii - b.ib)) * isy;
+         double dq[2], dr[3];
+#pragma unroll
+         for (int c = 0; c < 3; c++) {
+            if (c < 2) dq[c] = d1c(F(c, ii, jj - 2), F(c, ii, jj - 1), F(c, ii, jj + 1), F(c, ii, jj + 2));
+            dr[c] = DR(c, ii, jj);
+         }
+         const double p21m = __ldg(a.cc.prod[2] + q), p21l = __ldg(a.cc.prod[3] + q);
+         sm.gx[0][idx] = __ldg(a.cc.prod[1] + q) * dq[1] + fma(2.0, p21m, p21l) * (sxy * dr[0]) +
+                         __ldg(a.cc.prod[5] + q) * dr[1] + __ldg(a.cc.prod[7] + q) * (isy * dr[2]);
+         sm.gx[1][idx] = __ldg(a.cc.prod[0] + q) * dq[0] + __ldg(a.cc.prod[4] + q) * dr[0] + p21m * (sxy * dr[1]);
+         sm.gx[2][idx] = __ldg(a.cc.prod[6] + q) * (isy * dr[0]) + p21m * (sxy * dr[2]);
+      } else {  // q-outer: PQ (central) + RQ (one-sided r)
+         const int id = idx - RY * RPX, li = id % RX, ii = i0 + li, jj = j0 - 2 + id / RX;
+         if (ii > b.ie - 2 || jj > b.je) continue;
+         const long long q = pidx(b, ii, jj, k);
+         const double isx = sm.isx[li], syx = __ldg(a.sy + (jj - b.jb)) * isx;
+         double dp[2], dr[3];
+#pragma unroll
+         for (int c = 0; c < 3; c++) {
+            if (c < 2) dp[c] = d1c(F(c, ii - 2, jj), F(c, ii - 1, jj), F(c, ii + 1, jj), F(c, ii + 2, jj));
+            dr[c] = DR(c, ii, jj);
+         }
+         const double p31m = __ldg(a.cc.prod[4] + q), p31l = __ldg(a.cc.prod[5] + q);
+         sm.gy[0][id] = __ldg(a.cc.prod[0] + q) * dp[1] + p31m * (syx * dr[0]) + __ldg(a.cc.prod[2] + q) * dr[1];
+         sm.gy[1][id] = __ldg(a.cc.prod[1] + q) * dp[0] + __ldg(a.cc.prod[3] + q) * dr[0] +
+                        fma(2.0, p31m, p31l) * (syx * dr[1]) + __ldg(a.cc.prod[7] + q) * (isx * dr[2]);
+         sm.gy[2][id] = p31m * (syx * dr[2]) + __ldg(a.cc.prod[6] + q) * (isx * dr[1]);
+      }
+   }
+   __syncthreads();
+}
+
 template <int CORR, class RD, class WR, class SF>
-__device__ __forceinline__ void curv_top_point(const TopArgs<RD, WR, SF>& a, int i, int j, int k)
+__device__ __forceinline__ void curv_top_point(const TopArgs<RD, WR, SF>& a, const TopSmem& sm, int i, int j, int k)
 {
    const Box& b = a.b;
    const Box& fb = a.fb;
    const long long n = b.npts, ncol = b.nij;
    const long long p = pidx(b, i, j, k), col = pidx(b, i, j, b.kb);
    auto F = [&](int c, int ii, int jj, int kk) { return a.f.get(c * fb.npts + pidx(fb, ii, jj, kk)); };
-   auto Pr = [&](int t, long long q) { return __ldg(a.cc.prod[t] + q); };
-   const double sxc = __ldg(a.sx + (i - b.ib)), syc = __ldg(a.sy + (j - b.jb));
-   const double istrx = 1 / sxc, istry = 1 / syc;
-   const double i12 = 1.0 / 12;
-   auto cd = [&](double fm2, double fm1, double fp1, double fp2) { return i12 * d1c(fm2, fm1, fp1, fp2); };
    double s3[3] = {0, 0, 0};
    // same-axis p and q (precomputed weights, as the interior)
    {
@@ -614,8 +679,9 @@ __device__ __forceinline__ void curv_top_point(const TopArgs<RD, WR, SF>& a, int
                if (!use) continue;
                const int di = ax == 0, dj = ax == 1;
                const double f0 = F(c, i, j, k);
-               s3[c] += w0 * (F(c, i - 2 * di, j - 2 * dj, k) - f0) + w1 * (F(c, i - di, j - dj, k) - f0) +
-                        w2 * (F(c, i + di, j + dj, k) - f0) + w3 * (F(c, i + 2 * di, j + 2 * dj, k) - f0);
+               s3[c] = fma(w3, F(c, i + 2 * di, j + 2 * dj, k) - f0,
+                           fma(w2, F(c, i + di, j + dj, k) - f0,
+                               fma(w1, F(c, i - di, j - dj, k) - f0, fma(w0, F(c, i - 2 * di, j - 2 * dj, k) - f0, s3[c]))));
             }
          }
    }
@@ -641,53 +707,12 @@ __device__ __forceinline__ void curv_top_point(const TopArgs<RD, WR, SF>& a, int
          if (cc[t] != dd[t]) s3[dd[t]] += sc;
       }
    }
-   // one-sided r derivative of component c at column (ii, jj), row k
-   auto drb = [&](int c, int ii, int jj) {
-      return __ldg(a.dr + ((k - 1) * 3 + c) * ncol + pidx(b, ii, jj, b.kb));
-   };
-   // p-outer: QP (central) + RP (one-sided r)
-   {
-      double G[3][4];
+   // p- and q-outer differences of the products
 #pragma unroll
-      for (int mm = 0; mm < 4; mm++) {
-         const int ii = i + (mm < 2 ? mm - 2 : mm - 1);
-         const long long q = pidx(b, ii, j, k);
-         const double sxx = __ldg(a.sx + (ii - b.ib));
-         double dq[3], dr[3];
-#pragma unroll
-         for (int c = 0; c < 3; c++) {
-            dq[c] = cd(F(c, ii, j - 2, k), F(c, ii, j - 1, k), F(c, ii, j + 1, k), F(c, ii, j + 2, k));
-            dr[c] = drb(c, ii, j);
-         }
-         G[0][mm] = Pr(1, q) * dq[1] + istry * ((2 * Pr(2, q) + Pr(3, q)) * sxx * dr[0] +
-                                                 Pr(5, q) * syc * dr[1] + Pr(7, q) * dr[2]);
-         G[1][mm] = Pr(0, q) * dq[0] + Pr(4, q) * dr[0] + Pr(2, q) * sxx * istry * dr[1];
-         G[2][mm] = istry * (Pr(6, q) * dr[0] + Pr(2, q) * sxx * dr[2]);
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++) s3[c] += cd(G[c][0], G[c][1], G[c][2], G[c][3]);
-   }
-   // q-outer: PQ (central) + RQ (one-sided r)
-   {
-      double G[3][4];
-#pragma unroll
-      for (int mm = 0; mm < 4; mm++) {
-         const int jj = j + (mm < 2 ? mm - 2 : mm - 1);
-         const long long q = pidx(b, i, jj, k);
-         const double syy = __ldg(a.sy + (jj - b.jb));
-         double dp[3], dr[3];
-#pragma unroll
-         for (int c = 0; c < 3; c++) {
-            dp[c] = cd(F(c, i - 2, jj, k), F(c, i - 1, jj, k), F(c, i + 1, jj, k), F(c, i + 2, jj, k));
-            dr[c] = drb(c, i, jj);
-         }
-         G[0][mm] = Pr(0, q) * dp[1] + Pr(4, q) * syy * istrx * dr[0] + Pr(2, q) * dr[1];
-         G[1][mm] = Pr(1, q) * dp[0] + Pr(3, q) * dr[0] + (2 * Pr(4, q) + Pr(5, q)) * syy * istrx * dr[1] +
-                    Pr(7, q) * istrx * dr[2];
-         G[2][mm] = istrx * (Pr(4, q) * syy * dr[2] + Pr(6, q) * dr[1]);
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++) s3[c] += cd(G[c][0], G[c][1], G[c][2], G[c][3]);
+   for (int c = 0; c < 3; c++) {
+      const double* gx = sm.gx[c] + threadIdx.y * RPX + threadIdx.x;
+      const double* gy = sm.gy[c] + threadIdx.y * RX + threadIdx.x;
+      s3[c] += (1.0 / 144) * (d1c(gx[0], gx[1], gx[3], gx[4]) + d1c(gy[0], gy[RX], gy[3 * RX], gy[4 * RX]));
    }
    // r-outer (one-sided): PR + QR products at planes 1..8 of this column
 #pragma unroll
@@ -697,13 +722,14 @@ __device__ __forceinline__ void curv_top_point(const TopArgs<RD, WR, SF>& a, int
 #pragma unroll
       for (int c = 0; c < 3; c++) {
          const long long q = p + c * n;
-         a.out.set(q, 2 * a.u.get(q) - a.um.get(q) + kk * s3[c]);
+         a.out.set(q, fma(2.0, a.u.get(q), -a.um.get(q)) + kk * s3[c]);
       }
    } else {
       double sg[3] = {0, 0, 0};
       if (a.beta != 0) {
          const long long st[2] = {1, b.ni};
-         const double w[2] = {sxc * __ldg(a.coy + (j - b.jb)), syc * __ldg(a.cox + (i - b.ib))};
+         const double w[2] = {__ldg(a.sx + (i - b.ib)) * __ldg(a.coy + (j - b.jb)),
+                              __ldg(a.sy + (j - b.jb)) * __ldg(a.cox + (i - b.ib))};
          const double* dcp[2] = {a.dcx + (i - b.ib), a.dcy + (j - b.jb)};
 #pragma unroll
          for (int ax = 0; ax < 2; ax++) {
@@ -719,8 +745,8 @@ __device__ __forceinline__ void curv_top_point(const TopArgs<RD, WR, SF>& a, int
 #pragma unroll
                for (int m = -2; m <= 2; m++)
                   d[m + 2] = a.dd ? __ldg(a.dd + qs + m * s) : a.u.get(q + m * s) - a.um.get(q + m * s);
-               sg[c] += w[ax] * (e2 * (d[4] - 2 * d[3] + d[2]) - 2 * e1 * (d[3] - 2 * d[2] + d[1]) +
-                                 e0 * (d[2] - 2 * d[1] + d[0]));
+               sg[c] += w[ax] * (e2 * (fma(-2.0, d[3], d[4]) + d[2]) - 2 * e1 * (fma(-2.0, d[2], d[3]) + d[1]) +
+                                 e0 * (fma(-2.0, d[1], d[2]) + d[0]));
             }
          }
       }
@@ -736,14 +762,16 @@ __device__ __forceinline__ void curv_top_point(const TopArgs<RD, WR, SF>& a, int
 // The gx x gy x 6 blocks of 32 x 4 points, strided over by the grid (one CTA per
 // block, or a persistent grid beside the stage kernels).
 template <int CORR, class RD, class WR, class SF>
-__global__ void __launch_bounds__(128) curv_top_kernel(TopArgs<RD, WR, SF> a, int gx, int gy)
+__global__ void __launch_bounds__(RX * RY) curv_top_kernel(TopArgs<RD, WR, SF> a, int gx, int gy)
 {
+   __shared__ TopSmem sm;
    const int nvb = gx * gy * 6;
    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      const int i = a.b.ib + 2 + (vb % gx) * blockDim.x + threadIdx.x;
-      const int j = a.b.jb + 2 + ((vb / gx) % gy) * blockDim.y + threadIdx.y;
-      if (i > a.b.ie - 2 || j > a.b.je - 2) continue;
-      curv_top_point<CORR>(a, i, j, 1 + vb / (gx * gy));
+      const int i0 = a.b.ib + 2 + (vb % gx) * RX, j0 = a.b.jb + 2 + ((vb / gx) % gy) * RY, k = 1 + vb / (gx * gy);
+      curv_top_products(a, sm, i0, j0, k);
+      const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+      if (i <= a.b.ie - 2 && j <= a.b.je - 2) curv_top_point<CORR>(a, sm, i, j, k);
+      __syncthreads();
    }
 }
 
@@ -781,12 +809,14 @@ int launch_top(const ST& st, RD u, RD um, RD up, WR out, SF f, cudaStream_t s, c
    t.coef = CORR ? st.dt * st.dt / 12 : st.dt * st.dt;
    t.beta = st.beta;
    if (!st.scratch) return kBadArgument;
-   curv_top_pre_kernel<<<ctas > 0 ? ctas : gsb(b.nij, 128), 128, 0, s>>>(b, st.fbox, f, st.cc, st.sx, st.sy,
+   curv_top_pre_kernel<<<ctas > 0 ? 2 * ctas : gsb(b.nij, 128), 128, 0, s>>>(b, st.fbox, f, st.cc, st.sx, st.sy,
                                                                          st.scratch, st.scratch + 18 * b.nij);
    SW4G_TRY(launch_status());
    const int ni = b.ie - b.ib - 3, nj = b.je - b.jb - 3;
-   const int gx = (ni + 31) / 32, gy = (nj + 3) / 4;
-   const dim3 blk(32, 4), g(ctas > 0 ? std::min(ctas, gx * gy * 6) : gx * gy * 6);
+   const int gx = blocks_for(ni, RX), gy = blocks_for(nj, RY);
+   // beside the stages two CTAs of 128 threads find room on an SM (topography in the mixed
+   // form, two steps of 150 x 131 columns: one per SM 1.95 ms, two 1.89)
+   const dim3 blk(RX, RY), g(ctas > 0 ? std::min(2 * ctas, gx * gy * 6) : gx * gy * 6);
    curv_top_kernel<CORR><<<g, blk, 0, s>>>(t, gx, gy);
    return launch_status();
 }

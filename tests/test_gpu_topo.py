@@ -205,3 +205,21 @@ def test_topo_steps_with_curvilinear_sources(mode):
     quiet = TopoCase(nx, ny, ncart, h, zmax_topo=1.0, amp=0.2, xc=1.4, yc=1.3, lx=0.6, ly=0.5, gp=5)
     base = quiet.oracle(dt).run(*fields, 0.0, 8)
     assert _rel(ref[2], base[2]) > 1e-3
+
+
+@pytest.mark.parametrize("nx,ny", [(75, 33), (33, 41)])
+def test_topo_tiles_with_and_without_layers(nx, ny):
+    """Remainders of the stage's 32 x 8 and the top rows' 32 x 4 tiles, and tiles that no
+    damping layer reaches beside ones that it does: both forms of the step against the oracle
+    at the bar of the tests above (the rounding of six steps' sums)."""
+    h = 0.1
+    src = [sg.source_desc(0.5 * nx * h, 0.45 * ny * h, 2.0, force=(1.0, -0.5, 0.3), freq=8.0, t0=0.1,
+                          kind=sg.GAUSSIAN)]
+    c = TopoCase(nx, ny, 22, h, zmax_topo=1.0, amp=0.2, xc=0.45 * nx * h, yc=0.55 * ny * h, lx=0.6, ly=0.5,
+                 gp=5, sources=src)
+    dt = c.time_step(1.3)
+    fields = smooth_topo_fields(c, seed=9)
+    ref = c.oracle(dt).run(*fields, 0.0, 6)
+    got, _ = _gpu(c, fields, dt, 6, sg.MODE_FUSED)
+    for a, b in zip(got, ref):
+        assert _rel(a, b) <= 1e-12
