@@ -69,39 +69,40 @@ struct PtT {
 
 using Pt = PtT<false>;
 
+// d1c of the products cf * f
+__device__ __forceinline__ double d1p(const double cf[5], const double f[5])
+{
+   return fma(8.0, fma(cf[3], f[3], -(cf[1] * f[1])), fma(-cf[4], f[4], cf[0] * f[0]));
+}
+
 // (coef * f_ai)_ao times 144 h^2 with f = component c (src/rhs4sg_rev.C:221-347).
 template <class P_>
 __device__ __forceinline__ double mixed(const P_& P, bool la_coef, int ao, int ai, int c, int i,
                                         int j, int k)
 {
-   double s = 0;
+   double cf[5], in[5];
 #pragma unroll
    for (int m = -2; m <= 2; m++) {
       if (m == 0) continue;
       const int io = i + (ao == 0) * m, jo = j + (ao == 1) * m, ko = k + (ao == 2) * m;
       const int di = (ai == 0), dj = (ai == 1), dk = (ai == 2);
-      const double inner =
+      in[m + 2] =
           d1c(P.u(c, io - 2 * di, jo - 2 * dj, ko - 2 * dk), P.u(c, io - di, jo - dj, ko - dk),
               P.u(c, io + di, jo + dj, ko + dk), P.u(c, io + 2 * di, jo + 2 * dj, ko + 2 * dk));
-      const double cf = la_coef ? P.la(io, jo, ko) : P.mu(io, jo, ko);
-      const double w = (m == -2) ? 1.0 : (m == -1) ? -8.0 : (m == 1) ? 8.0 : -1.0;
-      s += w * cf * inner;
+      cf[m + 2] = la_coef ? P.la(io, jo, ko) : P.mu(io, jo, ko);
    }
-   return s;
+   return d1p(cf, in);
 }
 
-// s_ax-stretched coefficient stencils along axis ax at (i,j,k): a = mu*s, b = (2mu+la)*s.
+// s_ax-stretched coefficient stencil along axis ax at (i,j,k): mu*s, or (2mu+la)*s.
 template <class P_>
-__device__ __forceinline__ void coef_stencil(const P_& P, int ax, int i, int j, int k, double am[5],
-                                             double bm[5])
+__device__ __forceinline__ void coef_stencil(const P_& P, bool normal, int ax, int i, int j, int k, double cf[5])
 {
 #pragma unroll
    for (int m = -2; m <= 2; m++) {
       const int ii = i + (ax == 0) * m, jj = j + (ax == 1) * m, kk = k + (ax == 2) * m;
-      const double mu = P.mu(ii, jj, kk), la = P.la(ii, jj, kk);
-      const double s = P.s(ax, ax == 0 ? ii : ax == 1 ? jj : kk);
-      am[m + 2] = mu * s;
-      bm[m + 2] = (2 * mu + la) * s;
+      const double mu = P.mu(ii, jj, kk);
+      cf[m + 2] = (normal ? fma(2.0, mu, P.la(ii, jj, kk)) : mu) * P.s(ax, ax == 0 ? ii : ax == 1 ? jj : kk);
    }
 }
 
@@ -119,8 +120,11 @@ __device__ __forceinline__ void field_stencil(const P_& P, int ax, int c, int i,
 // k=q (top) or nk-q+1 (bottom), with the first-derivative weights negated at the
 // bottom (src/rhs4sg_rev.C:602-856).  strz is not applied on these rows.
 // PRE: the per-column terms come from rows_pre_kernel (a.dzc, a.roc).
+// A thread forms one component (the same in its block): a point's three in one thread are
+// 320 FP64 instructions in a row, and on small grids, whose rows are what a step waits for, a
+// warp's chain is the time (48 x 40 x 36 points: 38 us for all three, 20 us).
 template <bool TOP, bool DF = false, bool PRE = false>
-__device__ __forceinline__ void lu_bndry_point(const OpArgs& a, int i, int j, int k, double r[3])
+__device__ __forceinline__ double lu_bndry_point(const OpArgs& a, int i, int j, int k, int c)
 {
    const int nk = a.nk;
    const int kk = TOP ? k : nk - k + 1;
@@ -133,14 +137,15 @@ __device__ __forceinline__ void lu_bndry_point(const OpArgs& a, int i, int j, in
       return TOP ? w : -w;
    };
 
-   double am[2][5], bm[2][5];
-   for (int ax = 0; ax < 2; ax++) coef_stencil(P, ax, i, j, k, am[ax], bm[ax]);
-   for (int c = 0; c < 3; c++) {
-      double f[5], acc = 0;
-      for (int ax = 0; ax < 2; ax++) {
-         field_stencil(P, ax, c, i, j, k, f);
-         acc += (ax == 0 ? sx : sy) * d2var(ax == c ? bm[ax] : am[ax], f);
-      }
+   double r, acc = 0;
+#pragma unroll
+   for (int ax = 0; ax < 2; ax++) {
+      double f[5], cf[5];
+      coef_stencil(P, ax == c, ax, i, j, k, cf);
+      field_stencil(P, ax, c, i, j, k, f);
+      acc += (ax == 0 ? sx : sy) * d2var(cf, f);
+   }
+   {
       // z: sum_q (sum_m acof(kk,q,m) coef(m)) u(q) + ghcof(kk) coef(bnd) u(ghost)
       const int t = c == 2 ? 1 : 0;
       double zz = 0;
@@ -163,15 +168,13 @@ __device__ __forceinline__ void lu_bndry_point(const OpArgs& a, int i, int j, in
       const double mub = P.mu(i, j, TOP ? 1 : nk);
       const double cb = t ? 2 * mub + P.la(i, j, TOP ? 1 : nk) : mub;
       zz += k_ghcof[kk - 1] * cb * P.u(c, i, j, TOP ? 0 : nk + 1);
-      r[c] = i6 * acc + zz;
+      r = i6 * acc + zz;
    }
-   // centred mixed x-y terms
-   r[0] += sx * sy * i144 * (mixed(P, true, 0, 1, 1, i, j, k) + mixed(P, false, 1, 0, 1, i, j, k));
-   r[1] += sx * sy * i144 * (mixed(P, false, 0, 1, 0, i, j, k) + mixed(P, true, 1, 0, 0, i, j, k));
 
    // (coef * Dz f)_a: outer centred difference along a of a one-sided z derivative
    auto outer_of_dz = [&](bool la_coef, int ax, int c) {
-      double s = 0;
+      double cf[5], dzm[5];
+#pragma unroll
       for (int m = -2; m <= 2; m++) {
          if (m == 0) continue;
          const int ii = i + (ax == 0) * m, jj = j + (ax == 1) * m;
@@ -182,11 +185,10 @@ __device__ __forceinline__ void lu_bndry_point(const OpArgs& a, int i, int j, in
          else
 #pragma unroll 1
             for (int q = 1; q <= 8; q++) dz += wz(q) * P.u(c, ii, jj, kq(q));
-         const double cf = la_coef ? P.la(ii, jj, k) : P.mu(ii, jj, k);
-         const double w = (m == -2) ? 1.0 : (m == -1) ? -8.0 : (m == 1) ? 8.0 : -1.0;
-         s += w * cf * dz;
+         cf[m + 2] = la_coef ? P.la(ii, jj, k) : P.mu(ii, jj, k);
+         dzm[m + 2] = dz;
       }
-      return s * i12;
+      return d1p(cf, dzm) * i12;
    };
    // Dz(coef * f_a): one-sided z difference of a centred derivative along a
    auto dz_of_inner = [&](bool la_coef, int ax, int c) {
@@ -207,14 +209,22 @@ __device__ __forceinline__ void lu_bndry_point(const OpArgs& a, int i, int j, in
       }
       return s;
    };
-   r[0] += sx * outer_of_dz(true, 0, 2);
-   r[0] += sx * dz_of_inner(false, 0, 2);
-   r[1] += sy * outer_of_dz(true, 1, 2);
-   r[1] += sy * dz_of_inner(false, 1, 2);
-   r[2] += sx * outer_of_dz(false, 0, 0);
-   r[2] += sy * outer_of_dz(false, 1, 1);
-   r[2] += sx * dz_of_inner(true, 0, 0);
-   r[2] += sy * dz_of_inner(true, 1, 1);
+   // with the centred mixed x-y terms
+   if (c == 0) {
+      r += sx * sy * i144 * (mixed(P, true, 0, 1, 1, i, j, k) + mixed(P, false, 1, 0, 1, i, j, k));
+      r += sx * outer_of_dz(true, 0, 2);
+      r += sx * dz_of_inner(false, 0, 2);
+   } else if (c == 1) {
+      r += sx * sy * i144 * (mixed(P, false, 0, 1, 0, i, j, k) + mixed(P, true, 1, 0, 0, i, j, k));
+      r += sy * outer_of_dz(true, 1, 2);
+      r += sy * dz_of_inner(false, 1, 2);
+   } else {
+      r += sx * outer_of_dz(false, 0, 0);
+      r += sy * outer_of_dz(false, 1, 1);
+      r += sx * dz_of_inner(true, 0, 0);
+      r += sy * dz_of_inner(true, 1, 1);
+   }
+   return r;
 }
 
 // Per column, the parts of the one-sided rows that do not depend on the row's own
@@ -222,7 +232,8 @@ __device__ __forceinline__ void lu_bndry_point(const OpArgs& a, int i, int j, in
 // (the outer x/y differences of the rows read them at four neighbours), and for
 // interior columns the z-differences sum_q wz(kk,q) coef(q) D_a u_c(q)/12 of the four
 // centred products (mu D_x w, mu D_y w, la D_x u, la D_y v) of all six rows
-// (src/rhs4sg_rev.C:349-600).
+// (src/rhs4sg_rev.C:349-600).  A thread has one of the seven kinds (blockIdx.y): all in one
+// are 500 FP64 instructions in a row (48 x 40 columns: 26 us for all seven, 10 us).
 template <bool TOP>
 __global__ void __launch_bounds__(128) rows_pre_kernel(OpArgs a, double* __restrict__ dzc,
                                                        double* __restrict__ roc)
@@ -235,12 +246,12 @@ __global__ void __launch_bounds__(128) rows_pre_kernel(OpArgs a, double* __restr
       const double w = k_bope[(kk - 1) + 6 * (q - 1)];
       return TOP ? w : -w;
    };
-   const double i12 = 1.0 / 12;
+   const int piece = blockIdx.y;  // 0..2: the z derivatives of a component; 3..6: a product t
    for (long long col = blockIdx.x * (long long)blockDim.x + threadIdx.x; col < nij;
         col += (long long)gridDim.x * blockDim.x) {
       const int i = a.b.ib + (int)(col % a.b.ni), j = a.b.jb + (int)(col / a.b.ni);
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
+      if (piece < 3) {
+         const int c = piece;
          double f[8];
 #pragma unroll
          for (int q = 1; q <= 8; q++) f[q - 1] = P.u(c, i, j, kq(q));
@@ -251,34 +262,23 @@ __global__ void __launch_bounds__(128) rows_pre_kernel(OpArgs a, double* __restr
             for (int q = 1; q <= 8; q++) dz += wz(kk, q) * f[q - 1];
             dzc[((long long)(kk - 1) * 3 + c) * nij + col] = dz;
          }
+         continue;
       }
       if (i < a.b.ib + 2 || i > a.b.ie - 2 || j < a.b.jb + 2 || j > a.b.je - 2) continue;
       // t: 0 mu D_x w, 1 mu D_y w, 2 la D_x u, 3 la D_y v
-      double acc[6][4];
+      const int t = piece - 3, ax = t & 1, c = t < 2 ? 2 : ax, di = ax == 0, dj = ax == 1;
+      double acc[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
-      for (int kk = 0; kk < 6; kk++) acc[kk][0] = acc[kk][1] = acc[kk][2] = acc[kk][3] = 0;
-#pragma unroll 1
       for (int q = 1; q <= 8; q++) {
          const int kz = kq(q);
-         const double mu = P.mu(i, j, kz), la = P.la(i, j, kz);
-         double g[4];
+         const double g = (t < 2 ? P.mu(i, j, kz) : P.la(i, j, kz)) *
+                          d1c(P.u(c, i - 2 * di, j - 2 * dj, kz), P.u(c, i - di, j - dj, kz),
+                              P.u(c, i + di, j + dj, kz), P.u(c, i + 2 * di, j + 2 * dj, kz));
 #pragma unroll
-         for (int t = 0; t < 4; t++) {
-            const int ax = t & 1, c = t < 2 ? 2 : ax;
-            const int di = ax == 0, dj = ax == 1;
-            const double inner = d1c(P.u(c, i - 2 * di, j - 2 * dj, kz), P.u(c, i - di, j - dj, kz),
-                                     P.u(c, i + di, j + dj, kz), P.u(c, i + 2 * di, j + 2 * dj, kz));
-            g[t] = (t < 2 ? mu : la) * inner * i12;
-         }
-#pragma unroll
-         for (int kk = 1; kk <= 6; kk++)
-#pragma unroll
-            for (int t = 0; t < 4; t++) acc[kk - 1][t] += wz(kk, q) * g[t];
+         for (int kk = 1; kk <= 6; kk++) acc[kk - 1] += wz(kk, q) * g;
       }
 #pragma unroll
-      for (int kk = 0; kk < 6; kk++)
-#pragma unroll
-         for (int t = 0; t < 4; t++) roc[((long long)kk * 4 + t) * nij + col] = acc[kk][t];
+      for (int kk = 0; kk < 6; kk++) roc[((long long)kk * 4 + t) * nij + col] = (1.0 / 12) * acc[kk];
    }
 }
 
@@ -288,10 +288,8 @@ __global__ void __launch_bounds__(256) rhs4_bndry_kernel(OpArgs a)
    const int i = a.b.ib + 2 + blockIdx.x * blockDim.x + threadIdx.x;
    const int j = a.b.jb + 2 + blockIdx.y * blockDim.y + threadIdx.y;
    if (i > a.b.ie - 2 || j > a.b.je - 2) return;
-   const int k = TOP ? 1 + (int)blockIdx.z : a.nk - 5 + (int)blockIdx.z;
-   double r[3];
-   lu_bndry_point<TOP>(a, i, j, k, r);
-   for (int c = 0; c < 3; c++) a.lu[cidx(a.b, c, i, j, k)] = a.cof * r[c];
+   const int k = (TOP ? 1 : a.nk - 5) + (int)blockIdx.z / 3, c = blockIdx.z % 3;
+   a.lu[cidx(a.b, c, i, j, k)] = a.cof * lu_bndry_point<TOP>(a, i, j, k, c);
 }
 
 // Fused update on the one-sided rows (SoA fields):
@@ -340,6 +338,8 @@ __device__ __forceinline__ double sg4_point(const Box& b, const RowUpdate& w, in
 #pragma unroll
    for (int ax = 0; ax < 3; ax++) {
       const int di = ax == 0, dj = ax == 1, dk = ax == 2;
+      const double* dcp = w.dc[ax] + (ax == 0 ? i - b.ib : ax == 1 ? j - b.jb : k - b.kb);
+      if (!nonzero_bits(__ldg(dcp - 1)) && !nonzero_bits(__ldg(dcp)) && !nonzero_bits(__ldg(dcp + 1))) continue;
       double d[5];
 #pragma unroll
       for (int m = -2; m <= 2; m++) {
@@ -354,11 +354,10 @@ __device__ __forceinline__ double sg4_point(const Box& b, const RowUpdate& w, in
 #pragma unroll
       for (int m = -1; m <= 1; m++) {
          const int ii = i + di * m, jj = j + dj * m, kk = k + dk * m;
-         const int off = ax == 0 ? ii - b.ib : ax == 1 ? jj - b.jb : kk - b.kb;
-         e[m + 1] = __ldg(w.rho + pidx(b, ii, jj, kk)) * __ldg(w.dc[ax] + off);
+         e[m + 1] = __ldg(w.rho + pidx(b, ii, jj, kk)) * __ldg(dcp + m);
       }
-      const double s = e[2] * (d[4] - 2 * d[3] + d[2]) - 2 * e[1] * (d[3] - 2 * d[2] + d[1]) +
-                       e[0] * (d[2] - 2 * d[1] + d[0]);
+      const double s = e[2] * (fma(-2.0, d[3], d[4]) + d[2]) - 2 * e[1] * (fma(-2.0, d[2], d[3]) + d[1]) +
+                       e[0] * (fma(-2.0, d[1], d[2]) + d[0]);
       const double wgt = ax == 0 ? w.st[0][i - b.ib] * w.co[1][j - b.jb] * w.co[2][k - b.kb]
                        : ax == 1 ? w.st[1][j - b.jb] * w.co[0][i - b.ib] * w.co[2][k - b.kb]
                                  : w.st[2][k - b.kb] * w.co[0][i - b.ib] * w.co[1][j - b.jb];
@@ -368,42 +367,39 @@ __device__ __forceinline__ double sg4_point(const Box& b, const RowUpdate& w, in
 }
 
 // DF: the levels (and, when the stage field is not an FP64 slab, the field) are
-// double-float pairs; FDF: the stage field is double-float.  The gx x gy x 6 blocks
-// of 32 x 8 or 32 x 4 points are strided over by the grid (one CTA per block, or fewer CTAs,
+// double-float pairs; FDF: the stage field is double-float.  The gx x gy x 18
+// blocks of 32 x 4 points, of a row and component, are strided over by the grid (one CTA per block, or fewer CTAs,
 // each taking several: a persistent grid beside a stage kernel).
 template <bool TOP, bool DF, bool FDF, bool PRE>
-__global__ void __launch_bounds__(256, 2) stage_rows_kernel(OpArgs a, RowUpdate w, int gx, int gy)
+__global__ void __launch_bounds__(128, 4) stage_rows_kernel(OpArgs a, RowUpdate w, int gx, int gy)
 {
-   const int nvb = gx * gy * 6;
+   const int nvb = gx * gy * 18;
    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
       const int i = a.b.ib + 2 + (vb % gx) * blockDim.x + threadIdx.x;
       const int j = a.b.jb + 2 + ((vb / gx) % gy) * blockDim.y + threadIdx.y;
       if (i > a.b.ie - 2 || j > a.b.je - 2) continue;
-      const int bz = vb / (gx * gy);
-      const int k = TOP ? 1 + bz : a.nk - 5 + bz;
-      double r[3];
-      lu_bndry_point<TOP, FDF, PRE>(a, i, j, k, r);
+      const int bz = vb / (gx * gy), c = bz % 3;
+      const int k = (TOP ? 1 : a.nk - 5) + bz / 3;
+      const double r = lu_bndry_point<TOP, FDF, PRE>(a, i, j, k, c);
       const long long p = pidx(a.b, i, j, k);
       const double ir = w.irho ? __ldg(w.irho + p) : 1.0 / __ldg(w.rho + p);
       const double cr = w.coef * ir;
       const double birho = w.beta * ir;
-      for (int c = 0; c < 3; c++) {
-         const long long q = cidx(a.b, c, i, j, k);
-         const double lu = a.cof * r[c];
-         double v;
-         if (w.corrector != 1)
-            v = fma(2.0, lvl<DF>(w.u, w.udf, q, w.lo), -lvl<DF>(w.um, w.umdf, q, w.lo)) + cr * lu;
-         else
-            v = lvl<DF>(w.up, w.updf, q, w.lo) + cr * lu;
-         if (w.corrector != 0 && w.beta != 0) v -= birho * sg4_point<DF>(a.b, w, c, i, j, k);
-         if (DF) {
-            float hh, ll;
-            df_split(v, hh, ll);
-            w.outdf[q] = hh;
-            w.outdf[q + w.lo] = ll;
-         } else {
-            w.out[q] = v;
-         }
+      const long long q = cidx(a.b, c, i, j, k);
+      const double lu = a.cof * r;
+      double v;
+      if (w.corrector != 1)
+         v = fma(2.0, lvl<DF>(w.u, w.udf, q, w.lo), -lvl<DF>(w.um, w.umdf, q, w.lo)) + cr * lu;
+      else
+         v = lvl<DF>(w.up, w.updf, q, w.lo) + cr * lu;
+      if (w.corrector != 0 && w.beta != 0) v -= birho * sg4_point<DF>(a.b, w, c, i, j, k);
+      if (DF) {
+         float hh, ll;
+         df_split(v, hh, ll);
+         w.outdf[q] = hh;
+         w.outdf[q + w.lo] = ll;
+      } else {
+         w.out[q] = v;
       }
    }
 }
@@ -458,11 +454,11 @@ int launch_rhs4sg_direct(int soa, int ifirst, int ilast, int jfirst, int jlast, 
       SW4G_TRY(launch_operator_fixed(a.b, k1, k2, lu, u, mu, la, h, strx, stry, strz, stream));
    }
    if (onesided[4] == 1) {
-      const dim3 grid(blocks_for(ni, 32), blocks_for(nj, 8), 6);
+      const dim3 grid(blocks_for(ni, 32), blocks_for(nj, 8), 18);
       rhs4_bndry_kernel<true><<<grid, block, 0, stream>>>(a);
    }
    if (onesided[5] == 1) {
-      const dim3 grid(blocks_for(ni, 32), blocks_for(nj, 8), 6);
+      const dim3 grid(blocks_for(ni, 32), blocks_for(nj, 8), 18);
       rhs4_bndry_kernel<false><<<grid, block, 0, stream>>>(a);
    }
    return launch_status();
@@ -515,12 +511,12 @@ int launch_stage_rows(int corrector, bool top, const Box& b, int nk, const doubl
    }
    const int ni = b.ie - b.ib - 3, nj = b.je - b.jb - 3;
    if (ni <= 0 || nj <= 0) return kOk;
-   const int gx = blocks_for(ni, 32), gy = blocks_for(nj, 8);
-   const dim3 block(32, 8, 1), grid(ctas > 0 ? std::min(ctas, gx * gy * 6) : gx * gy * 6);
+   const int gx = blocks_for(ni, 32), gy = blocks_for(nj, 4);
+   const dim3 block(32, 4, 1), grid(ctas > 0 ? std::min(ctas, gx * gy * 18) : gx * gy * 18);
    if (rscr) {  // the per-column terms once, then the rows read them
       a.dzc = rscr;
       a.roc = rscr + 18 * b.nij;
-      const int nb = ctas > 0 ? ctas : (int)std::min<long long>((b.nij + 127) / 128, 152LL * 16);
+      const dim3 nb(ctas > 0 ? (ctas + 6) / 7 : (int)std::min<long long>((b.nij + 127) / 128, 152LL * 16), 7);
       if (top) rows_pre_kernel<true><<<nb, 128, 0, stream>>>(a, rscr, rscr + 18 * b.nij);
       else rows_pre_kernel<false><<<nb, 128, 0, stream>>>(a, rscr, rscr + 18 * b.nij);
       const int st = launch_status();
@@ -585,17 +581,15 @@ int launch_stage_rows_df(int corrector, bool top, const Box& b, int nz, const do
    }
    const int ni = b.ie - b.ib - 3, nj = b.je - b.jb - 3;
    if (ni <= 0 || nj <= 0) return kOk;
-   // Beside the stage kernel fed by tensor copies (i extents that are multiples of 4), whose
-   // nine warps leave registers for four more on an SM: CTAs of four (CTAs of eight waited for
-   // the stage to end; steps of 320^3 11.4 -> 9.8 ms a call of two).  Beside the other one,
-   // which leaves room for eight, CTAs of eight (steps at ragged sizes 727 -> 715 us a call).
-   const int by = ctas > 0 && b.ni % 4 == 0 ? 4 : 8;
-   const int gx = blocks_for(ni, 32), gy = blocks_for(nj, by);
-   const dim3 block(32, by, 1), grid(ctas > 0 ? std::min(ctas, gx * gy * 6) : gx * gy * 6);
+   // CTAs of four warps: as many as the nine warps of the stage kernel fed by tensor copies
+   // leave registers for on an SM (CTAs of eight waited for the stage to end; steps of 320^3
+   // 11.4 -> 9.8 ms a call of two), and twice as many CTAs on small grids.
+   const int gx = blocks_for(ni, 32), gy = blocks_for(nj, 4);
+   const dim3 block(32, 4, 1), grid(ctas > 0 ? std::min(ctas, gx * gy * 18) : gx * gy * 18);
    if (rscr) {  // the per-column terms once, then the rows read them
       a.dzc = rscr;
       a.roc = rscr + 18 * b.nij;
-      const int nb = ctas > 0 ? ctas : (int)std::min<long long>((b.nij + 127) / 128, 152LL * 16);
+      const dim3 nb(ctas > 0 ? (ctas + 6) / 7 : (int)std::min<long long>((b.nij + 127) / 128, 152LL * 16), 7);
       if (top) rows_pre_kernel<true><<<nb, 128, 0, stream>>>(a, rscr, rscr + 18 * b.nij);
       else rows_pre_kernel<false><<<nb, 128, 0, stream>>>(a, rscr, rscr + 18 * b.nij);
       const int st = launch_status();

@@ -85,3 +85,30 @@ def test_corr_rows(side):
     assert sg.lib().sw4g_corr_rows(*g.bounds, g.nz, side, out.data_ptr(),
                                    *[t.data_ptr() for t in d], g.h, dt, beta,
                                    scratch.data_ptr(), n - 1, stream()) == 1
+
+
+@pytest.mark.parametrize("side", [0, 1])
+@pytest.mark.parametrize("lo,hi", [(0, 25), (7, 9), (6, 21), (30, 31)])
+def test_corr_rows_where_layers_end(side, lo, hi):
+    """Profiles that vanish on part of each axis (or all of it): a point adds an axis' damping
+    when any of the three values its term reads is nonzero.  The bar of test_corr_rows."""
+    g, u, um, up, rho, mu, la, st, dc, co = _problem(60 + side)
+    dt, beta = 0.011, 0.02
+    dc = tuple(np.where((np.arange(a.size) >= lo) & (np.arange(a.size) < hi), 0.0, a) for a in dc)
+    if lo == 30:
+        dc = tuple(np.zeros_like(a) for a in dc)
+    uacc, lu = np.zeros_like(u), np.zeros_like(u)
+    O.dpdmtfort(g.bounds, up, u, um, uacc, 1 / dt ** 2)
+    O.rhs4sg(1, g.bounds, g.nz, [0, 0, 0, 0, 1, 1], lu, uacc, mu, la, g.h, *st)
+    ref = up.copy()
+    O.corrfort(1, g.bounds, ref, lu, np.zeros_like(u), rho, dt ** 4)
+    O.addsgd(4, 1, g.bounds, ref, u, um, rho, dc, st, co, beta)
+    n = sg.lib().sw4g_corr_rows_scratch_len(g.ib, g.ie, g.jb, g.je)
+    scratch = dev(np.zeros(n))
+    d = [dev(a) for a in (up, u, um, mu, la, rho, *st, *dc, *co)]
+    out = dev(np.zeros_like(u))
+    sg.check(sg.lib().sw4g_corr_rows(*g.bounds, g.nz, side, out.data_ptr(),
+                                     *[t.data_ptr() for t in d], g.h, dt, beta,
+                                     scratch.data_ptr(), n, stream()), "corr_rows")
+    m = _rows_mask(g, side)
+    assert rel_err((host(out) - up)[m], (ref - up)[m]) <= 1e-13
