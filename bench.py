@@ -83,15 +83,16 @@ def measured_peaks():
 # algorithmic bytes per interior point of one corrector stage: reads Up, U, Um (9
 # words) and mu, lambda, rho (3), writes the new level (3): 15 FP64 words
 CORR_STAGE_WORDS = 15
-# DRAM bytes per interior point of the FP64 corrector stage kernel, from one ncu
-# capture of the 192^3 case (dram__bytes_read.sum + dram__bytes_write.sum = 2.1133e9 B
-# over 7,077,888 interior points); traffic grows with the point count, so a launch
-# moves this many bytes per point at any size
-CORR_STAGE_DRAM_BYTES_PER_PT = 298.6
-# FP64-pipe warp instructions per interior point of the FP64 stage kernels on the
-# 512^3 workload (smsp__inst_executed_pipe_fp64.sum, single-pass ncu captures of the
-# full-size run: corrector 830,809,640 and predictor 671,186,048 over 512^3 points).  The pipe issues
-# 2 FP64 thread instructions per clock per SM, i.e. one warp instruction per 16 clocks.
+# DRAM bytes and warp instructions per interior point of the fixed-point FP64 stage kernels
+# (ncu captures at 256^3, profiles/fixed_stage_c2_256.md: corrector 5.590e9 B and
+# 1,187,100,000 warp instructions, predictor 1,143,807,280, over 256^3 points); both grow
+# with the point count.  An SM issues at most 4 warp instructions a clock.
+CORR_STAGE_DRAM_BYTES_PER_PT = 333.2
+WARP_INST_PER_PT = {"corr": 1187100000 / 256 ** 3, "pred": 1143807280 / 256 ** 3}
+WARP_INST_PER_CLK_PER_SM = 4
+# FP64-pipe warp instructions per interior point of the same stages in FP64 arithmetic
+# (profiles/fp64_pipe_c2_512.md): what the fixed-point form avoids.  The pipe issues 2 FP64
+# thread instructions per clock per SM, i.e. one warp instruction per 16 clocks.
 FP64_WARP_INST_PER_PT = {"corr": 830809640 / 512 ** 3, "pred": 671186048 / 512 ** 3}
 FP64_THREAD_INST_PER_CLK_PER_SM = 2
 # mixed form, corrector stage: reads Up, U, Um as double-float pairs (9 x 8 B), mu,
@@ -823,9 +824,10 @@ def run_ours(args, rank, world):
     nsm = torch.cuda.get_device_properties(local).multi_processor_count
     mhz = fp64["clocks"]["sm_mhz"] or 2070.0
     fp64_peak = FP64_THREAD_INST_PER_CLK_PER_SM * nsm * mhz * 1e6 / 1e9
-    fp64_rate = 32 * FP64_WARP_INST_PER_PT["corr"] * npts_int / (corr_ms * 1e-3) / 1e9
+    issue_peak = WARP_INST_PER_CLK_PER_SM * nsm * mhz * 1e6 / 1e9
+    issue_rate = WARP_INST_PER_PT["corr"] * npts_int / (corr_ms * 1e-3) / 1e9
     pred_ms = fp64["kernel_ms"]["pred_stage"]
-    fp64_rate_pred = 32 * FP64_WARP_INST_PER_PT["pred"] * npts_int / (pred_ms * 1e-3) / 1e9
+    issue_rate_pred = WARP_INST_PER_PT["pred"] * npts_int / (pred_ms * 1e-3) / 1e9
     if mixed is not None:
         mixed["roofline"]["peak"] = peak_hbm
         mixed["roofline"]["frac"] = mixed["roofline"]["achieved"] / peak_hbm
@@ -870,21 +872,23 @@ def run_ours(args, rank, world):
                        "l2": "inputs larger than L2 (3.3 GB per field), no flush",
                        "parallelism": "replicas" if world > 1 else "single"},
             "roofline": {
-                "bound": "fp64", "kernel": "fused corrector stage (fused_stage_kernel<1>)",
-                "achieved": fp64_rate, "peak": fp64_peak, "unit": "G FP64 thread-instructions/s",
-                "frac": fp64_rate / fp64_peak,
+                "bound": "issue", "kernel": "fixed-point corrector stage (fixed_stage_kernel<1>)",
+                "achieved": issue_rate, "peak": issue_peak, "unit": "G warp instructions/s",
+                "frac": issue_rate / issue_peak,
                 "traffic": CORR_STAGE_DRAM_BYTES_PER_PT * npts_int,
-                "basis": f"{32 * FP64_WARP_INST_PER_PT['corr']:.2f} FP64-pipe thread instructions "
-                         "per interior point (ncu smsp__inst_executed_pipe_fp64 x 32 at 512^3) x points "
-                         f"/ launch_ms; peak = {FP64_THREAD_INST_PER_CLK_PER_SM} per clock per SM x "
-                         f"{nsm} SMs x the median sampled SM clock ({mhz:.0f} MHz)",
+                "basis": f"{WARP_INST_PER_PT['corr']:.2f} warp instructions per interior point (ncu "
+                         "inst_executed at 256^3) x points / launch_ms, which includes the damping of the "
+                         f"layers; peak = {WARP_INST_PER_CLK_PER_SM} per clock per SM x {nsm} SMs x the median "
+                         f"sampled SM clock ({mhz:.0f} MHz)",
                 "launch_ms": corr_ms,
-                "predictor": {"achieved": fp64_rate_pred, "frac": fp64_rate_pred / fp64_peak,
+                "predictor": {"achieved": issue_rate_pred, "frac": issue_rate_pred / issue_peak,
                               "launch_ms": pred_ms},
+                "fp64_form_floor_ms": {
+                    k: 32 * v * npts_int / (fp64_peak * 1e9) * 1e3 for k, v in FP64_WARP_INST_PER_PT.items()},
                 "hbm": {"achieved": achieved, "peak": peak_hbm, "unit": "GB/s",
                         "frac": achieved / peak_hbm, "peak_source": peak_kind,
                         "algorithmic_bytes_per_launch": corr_bytes,
-                        "traffic_source": "ncu capture at 192^3 scaled per point"}},
+                        "traffic_source": "ncu capture at 256^3 scaled per point"}},
             "kernel_ms": fp64["kernel_ms"],
             "clocks": fp64["clocks"],
             "e2e": fp64.get("e2e"),
