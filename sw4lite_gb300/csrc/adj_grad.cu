@@ -236,10 +236,11 @@ __global__ void grad_profiles_kernel(int n, const double* __restrict__ st, const
 }
 
 // The step kernels: one thread per array point, kGradThreads consecutive points of
-// a k plane (rows of i) per CTA, blockIdx.y the plane.  They run beside the FP64
-// stage kernels, in the registers those leave free: the predictor-form stage (96
-// registers x 512 threads per SM) leaves 16K, room for three 64-thread CTAs of
-// grad_df_kernel (72 registers) but one of 128 threads.
+// a k plane (rows of i) per CTA, blockIdx.y the plane.  Small CTAs fit in the registers
+// that other kernels leave: beside the damping, the closures and the last CTAs of a stage
+// (the fixed-point stages themselves leave none while they fill the SMs), or beside the
+// predictor form of the FP64 stages (16K of an SM's: three of grad_df_kernel's CTAs at 72
+// registers, but one of 128 threads).  Issue slots bound them: 62 and 67 % busy alone.
 constexpr int kGradThreads = 64;
 
 // w1 = up - 2u + um; the pairs of b1, mt (adjoint shift) and w1, u, um (forward

@@ -1100,8 +1100,10 @@ int EW::side_stream()
    SW4G_TRY(cuda_ok(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev)));
    // FP32-mixed form: the highest priority, so that the rows' persistent CTAs take
    // their place on every SM beside the (FP32, issue-bound) stage kernel's as soon as
-   // they are launched.  FP64 form: the stage kernels and the rows both load the FP64
-   // pipe, and the rows' own full grid at the default priority measured best.
+   // they are launched.  FP64 form: two CTAs of the fixed-point stages leave no registers
+   // for a rows CTA on an SM, and displacing them costs more than running the rows as they
+   // drain: a step of 512^3 43.4 ms with the rows' full grid at the default priority, 44.0
+   // at the highest, 44.7 with a persistent grid.
    SW4G_TRY(cuda_ok(cudaDeviceGetStreamPriorityRange(&lo, &hi)));
    SW4G_TRY(cuda_ok(cudaStreamCreateWithPriority(&side_, cudaStreamNonBlocking, mixed_ ? hi : lo)));
    SW4G_TRY(cuda_ok(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming)));
