@@ -80,7 +80,9 @@ struct FreeSurf {
    double sbop[5];
 };
 
-// Ghost plane of a flat free surface (src/ew-cfromfort.C:415-476, :686-744).
+// Ghost plane of a flat free surface (src/ew-cfromfort.C:415-476, :686-744), a component per
+// thread (blockIdx.z): its divisions make all three a chain of some 200 FP64 instructions,
+// which is the kernel's time on small planes (48 x 40 points 11.8 -> 5.1 us).
 template <class Field>
 __global__ void free_surface_kernel(Box b, Field u, const double* __restrict__ mu,
                                     const double* __restrict__ la,
@@ -96,30 +98,27 @@ __global__ void free_surface_kernel(Box b, Field u, const double* __restrict__ m
    const long long qq = (i - b.ib) + b.ni * (j - b.jb);
    const long long p = pidx(b, i, j, k);
    auto U = [&](int c, int ii, int jj, int kk) { return u.get(cidx(b, c, ii, jj, kk)); };
-   const double sx = strx[i - b.ib], sy = stry[j - b.jb];
-   const double wx = sx * (d4a * (U(2, i + 1, j, k) - U(2, i - 1, j, k)) +
-                           d4b * (U(2, i + 2, j, k) - U(2, i - 2, j, k)));
-   const double ux = sx * (d4a * (U(0, i + 1, j, k) - U(0, i - 1, j, k)) +
-                           d4b * (U(0, i + 2, j, k) - U(0, i - 2, j, k)));
-   const double wy = sy * (d4a * (U(2, i, j + 1, k) - U(2, i, j - 1, k)) +
-                           d4b * (U(2, i, j + 2, k) - U(2, i, j - 2, k)));
-   const double vy = sy * (d4a * (U(1, i, j + 1, k) - U(1, i, j - 1, k)) +
-                           d4b * (U(1, i, j + 2, k) - U(1, i, j - 2, k)));
-   double uz = 0, vz = 0, wz = 0;
+   const int c = blockIdx.z;
+   double dz = 0;
 #pragma unroll
-   for (int q = 1; q <= 4; q++) {
-      const int kq = k + kl * (q - 1);
-      uz += fs.sbop[q] * U(0, i, j, kq);
-      vz += fs.sbop[q] * U(1, i, j, kq);
-      wz += fs.sbop[q] * U(2, i, j, kq);
+   for (int q = 1; q <= 4; q++) dz += fs.sbop[q] * U(c, i, j, k + kl * (q - 1));
+   const double f = bforce ? bforce[3 * qq + c] : 0.0;
+   const double sx = strx[i - b.ib], sy = stry[j - b.jb];
+   auto dx = [&](int e) {
+      return sx * (d4a * (U(e, i + 1, j, k) - U(e, i - 1, j, k)) + d4b * (U(e, i + 2, j, k) - U(e, i - 2, j, k)));
+   };
+   auto dy = [&](int e) {
+      return sy * (d4a * (U(e, i, j + 1, k) - U(e, i, j - 1, k)) + d4b * (U(e, i, j + 2, k) - U(e, i, j - 2, k)));
+   };
+   const double m = mu[p];
+   double g;
+   if (c < 2) {
+      g = -dz - kl * (c == 0 ? dx(2) : dy(2)) + kl * h * f / m;
+   } else {
+      const double l = la[p];
+      g = -dz + (-kl * l * (dx(0) + dy(1)) + kl * h * f) / (2 * m + l);
    }
-   const double f0 = bforce ? bforce[3 * qq] : 0.0;
-   const double f1 = bforce ? bforce[3 * qq + 1] : 0.0;
-   const double f2 = bforce ? bforce[3 * qq + 2] : 0.0;
-   const double m = mu[p], l = la[p];
-   u.set(cidx(b, 0, i, j, k - kl), (-uz - kl * wx + kl * h * f0 / m) / fs.sbop[0]);
-   u.set(cidx(b, 1, i, j, k - kl), (-vz - kl * wy + kl * h * f1 / m) / fs.sbop[0]);
-   u.set(cidx(b, 2, i, j, k - kl), (-wz + (-kl * l * (ux + vy) + kl * h * f2) / (2 * m + l)) / fs.sbop[0]);
+   u.set(cidx(b, c, i, j, k - kl), g / fs.sbop[0]);
 }
 
 int small_grid(long long n)
@@ -181,7 +180,7 @@ int bc_sides(int soa, int ib, int ie, int jb, int je, int kb, int ke, const int 
          FreeSurf fs;
          for (int q = 0; q < 5; q++) fs.sbop[q] = sbop[q];
          const int k = side == 4 ? 1 : nz, kl = side == 4 ? 1 : -1;
-         const dim3 block(32, 8), grid(blocks_for(ie - ib - 3, 32), blocks_for(je - jb - 3, 8));
+         const dim3 block(32, 4), grid(blocks_for(ie - ib - 3, 32), blocks_for(je - jb - 3, 4), 3);
          free_surface_kernel<<<grid, block, 0, s>>>(b, u, mu, la, bforce ? bforce[side] : nullptr,
                                                     strx, stry, h, k, kl, fs);
       }
@@ -199,7 +198,7 @@ int launch_free_surface_ghosts(const Box& b, int nz, int side, bool df, void* u,
    FreeSurf fs;
    for (int q = 0; q < 5; q++) fs.sbop[q] = sbop[q];
    const int k = side == 4 ? 1 : nz, kl = side == 4 ? 1 : -1;
-   const dim3 block(32, 8), grid(blocks_for(b.ie - b.ib - 3, 32), blocks_for(b.je - b.jb - 3, 8));
+   const dim3 block(32, 4), grid(blocks_for(b.ie - b.ib - 3, 32), blocks_for(b.je - b.jb - 3, 4), 3);
    if (df)
       free_surface_kernel<<<grid, block, 0, s>>>(b, DFField{static_cast<float*>(u), 3 * b.npts}, mu, la,
                                                  nullptr, strx, stry, h, k, kl, fs);
