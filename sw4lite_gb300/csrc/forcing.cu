@@ -80,20 +80,22 @@ __global__ void force_update_kernel(Box b, S* __restrict__ up, const double* __r
    const int r = blockIdx.x * blockDim.x + threadIdx.x;
    if (r >= src.npoints) return;
    if (clk) t = clk[0];  // the device clock of a captured time loop
+   // the point's values first: their loads, a chain of four, overlap the time functions (one source,
+   // 7.5 -> 5.4 us)
+   const int s0 = src.start[r], s1 = src.start[r + 1];
+   const int i = src.ijk[3 * s0], j = src.ijk[3 * s0 + 1], k = src.ijk[3 * s0 + 2];
+   const double rp = rho[pidx(b, i, j, k)];
+   double old[3];
+   for (int c = 0; c < 3; c++) old[c] = (double)up[cidx(b, c, i, j, k)];
    double acc[3] = {0, 0, 0};
-   for (int s = src.start[r]; s < src.start[r + 1]; s++) {
+   for (int s = s0; s < s1; s++) {
       const double g = timefunc(src.kind[s], src.freq[s], t - src.t0[s], tt != 0);
       acc[0] += src.amp[3 * s] * g;
       acc[1] += src.amp[3 * s + 1] * g;
       acc[2] += src.amp[3 * s + 2] * g;
    }
-   const int s0 = src.start[r];
-   const int i = src.ijk[3 * s0], j = src.ijk[3 * s0 + 1], k = src.ijk[3 * s0 + 2];
-   const double c0 = coef / rho[pidx(b, i, j, k)];
-   for (int c = 0; c < 3; c++) {
-      const long long q = cidx(b, c, i, j, k);
-      up[q] = (S)((double)up[q] + c0 * acc[c]);
-   }
+   const double c0 = coef / rp;
+   for (int c = 0; c < 3; c++) up[cidx(b, c, i, j, k)] = (S)(old[c] + c0 * acc[c]);
 }
 
 // Same as force_update_kernel for a double-float level: the add runs in FP64.
@@ -104,20 +106,22 @@ __global__ void force_update_df_kernel(Box b, DFField up, const double* __restri
    const int r = blockIdx.x * blockDim.x + threadIdx.x;
    if (r >= src.npoints) return;
    if (clk) t = clk[0];
+   // the point's values first: their loads, a chain of four, overlap the time functions (one source,
+   // 7.5 -> 5.4 us)
+   const int s0 = src.start[r], s1 = src.start[r + 1];
+   const int i = src.ijk[3 * s0], j = src.ijk[3 * s0 + 1], k = src.ijk[3 * s0 + 2];
+   const double rp = rho[pidx(b, i, j, k)];
+   double old[3];
+   for (int c = 0; c < 3; c++) old[c] = up.get(cidx(b, c, i, j, k));
    double acc[3] = {0, 0, 0};
-   for (int s = src.start[r]; s < src.start[r + 1]; s++) {
+   for (int s = s0; s < s1; s++) {
       const double g = timefunc(src.kind[s], src.freq[s], t - src.t0[s], tt != 0);
       acc[0] += src.amp[3 * s] * g;
       acc[1] += src.amp[3 * s + 1] * g;
       acc[2] += src.amp[3 * s + 2] * g;
    }
-   const int s0 = src.start[r];
-   const int i = src.ijk[3 * s0], j = src.ijk[3 * s0 + 1], k = src.ijk[3 * s0 + 2];
-   const double c0 = coef / rho[pidx(b, i, j, k)];
-   for (int c = 0; c < 3; c++) {
-      const long long q = cidx(b, c, i, j, k);
-      up.set(q, up.get(q) + c0 * acc[c]);
-   }
+   const double c0 = coef / rp;
+   for (int c = 0; c < 3; c++) up.set(cidx(b, c, i, j, k), old[c] + c0 * acc[c]);
 }
 
 // The device clock of a captured time loop: [0] time of the next stage's forcing,
