@@ -63,6 +63,8 @@ struct FixedArgs {
    const int4* __restrict__ c;    // lambda and mu coefficients of the mixed terms
    const int* __restrict__ e;     // exponents of both: weights << 16 | coefficients
    const int* __restrict__ bad;   // nonzero: the material is not finite everywhere
+   const double* __restrict__ mu;  // read where the material is not finite
+   const double* __restrict__ la;
    int wbx, wny;                  // blocks per row and rows per plane of w
    const double* __restrict__ sx;
    const double* __restrict__ sy;
@@ -71,7 +73,7 @@ struct FixedArgs {
    int* emax;
 };
 
-// Exponent of coefficients that are not finite
+// Exponent of coefficients beyond the range
 constexpr int kCoefBad = 0x7fff;
 
 struct Smem {
@@ -130,7 +132,8 @@ __device__ __forceinline__ double stage_value(const FixedArgs& a, long long q)
 // The points of a column whose sums read a value that is not finite, set to NaN after the
 // march: the sums themselves took it as zero.  A component's second differences read the
 // component along the three axes; its mixed terms read another component at the points
-// off both axes in the plane of the two; the coefficients are those of the same points.
+// off both axes in the plane of the two.  Of the material a component reads mu at every
+// point of the three axes, lambda at its own point and along its own axis.
 // Returns the exponent field of NaN if there was such a point.
 template <int FORM>
 __device__ int mark_not_finite(const FixedArgs& a, int i, int j, int kbeg, int kend)
@@ -142,15 +145,18 @@ __device__ int mark_not_finite(const FixedArgs& a, int i, int j, int kbeg, int k
       auto bad = [&](int c, long long q) {
          return !isfinite(stage_value<FORM>(a, q + c * a.npts));
       };
-      auto coef_bad = [&](long long q) { return (short)(a.e[q] & 0xffff) == kCoefBad; };
-      const bool all = (a.e[p] >> 16) == kCoefBad;
-      bool nan[3] = {all || bad(0, p), all || bad(1, p), all || bad(2, p)};
+      bool coef = !isfinite(a.mu[p]) || !isfinite(a.la[p]), all = coef;
+      bool nan[3] = {bad(0, p), bad(1, p), bad(2, p)};
       for (int ax = 0; ax < 3; ax++)
          for (int m = -2; m <= 2; m++) {
             if (m == 0) continue;
             const long long q = p + m * st[ax];
+            const bool mu = !isfinite(a.mu[q]), la = !isfinite(a.la[q]);
+            all = all || mu;
+            nan[ax] = nan[ax] || la;
+            coef = coef || mu || la;
             for (int c = 0; c < 3; c++) {
-               nan[c] = nan[c] || bad(c, q) || coef_bad(q);
+               nan[c] = nan[c] || bad(c, q);
                if (c == ax) continue;
                for (int n = -2; n <= 2; n++)
                   if (n != 0 && bad(c, q + n * st[c])) nan[ax] = true;  // c_c of another component ...
@@ -158,8 +164,9 @@ __device__ int mark_not_finite(const FixedArgs& a, int i, int j, int kbeg, int k
                   if (n != 0 && bad(ax, q + n * st[c])) nan[c] = true;  // ... in both of the plane's
             }
          }
+      if (!coef && (a.e[p] >> 16) == kCoefBad) all = true;  // weights beyond the range
       for (int c = 0; c < 3; c++)
-         if (nan[c]) {
+         if (all || nan[c]) {
             a.out[p + c * a.npts] = __longlong_as_double(0x7ff8000000000000LL);
             em = 0x7ff;
          }
@@ -564,7 +571,15 @@ __global__ void fixed_coef_kernel(Box b, const double* __restrict__ mu, const do
       const int i = b.ib + (int)(p % b.ni);
       const int j = b.jb + (int)((p / b.ni) % (b.je - b.jb + 1));
       const int k = b.kb + (int)(p / b.nij);
-      const double m = mu[p] * cof144, l = la[p] * cof144;
+      // a coefficient that is not finite counts as zero; the points that read it are marked
+      // after the march
+      bool finite = true;
+      auto clean = [&](double v) {
+         if (isfinite(v)) return v;
+         finite = false;
+         return 0.0;
+      };
+      const double m = clean(mu[p] * cof144), l = clean(la[p] * cof144);
       int ec = max(exponent_above(fmax(fabs(m), fabs(l))), -900);
       const int2 cm = to_coef(m, ec), cl = to_coef(l, ec);
       c[p] = make_int4(cm.x, cm.y, cl.x, cl.y);
@@ -592,6 +607,8 @@ __global__ void fixed_coef_kernel(Box b, const double* __restrict__ mu, const do
                wt[ax][t][1] = f * (v[0] + v[3] + 3 * (v[2] + v[1]));
                wt[ax][t][2] = f * (v[1] + v[4] + 3 * (v[3] + v[2]));
                wt[ax][t][3] = f * (v[3] - 0.75 * (v[2] + v[4]));
+#pragma unroll
+               for (int q = 0; q < 4; q++) wt[ax][t][q] = clean(wt[ax][t][q]);
                sum[ax][t] = fabs(wt[ax][t][0]) + fabs(wt[ax][t][1]) + fabs(wt[ax][t][2]) + fabs(wt[ax][t][3]);
             }
          }
@@ -620,7 +637,7 @@ __global__ void fixed_coef_kernel(Box b, const double* __restrict__ mu, const do
                   o[((ax * 2 + t) * 4 + q) * kFixedBlock] = make_int2((int)hi, (int)(v - (hi << kSplit)));
                }
       }
-      if (ew == kCoefBad || ec == kCoefBad) *bad = 1;
+      if (!finite || ew == kCoefBad || ec == kCoefBad) *bad = 1;
       e[p] = (int)((unsigned)ew << 16 | ((unsigned)ec & 0xffffu));
    }
 }
@@ -687,6 +704,8 @@ int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
    a.c = st.fc.c;
    a.e = st.fc.e;
    a.bad = st.fc.bad;
+   a.mu = st.mu;
+   a.la = st.la;
    a.sx = st.st[0];
    a.sy = st.st[1];
    a.sz = st.st[2];

@@ -1,0 +1,66 @@
+"""Material values that are not finite, in one stage of the FP64 time step: the predicted
+level is NaN or infinite exactly where the same sums in FP64 are, and elsewhere within the
+rounding of two sums of 80 products (2 x 80 x 2^-53 < 2^-45 of the largest value).  A
+subdomain that is the whole grid steps part by part; after its first part the two interior
+planes next to a side can be read as a halo, so the planted point lies there.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import sw4lite_gb300 as sg
+from oracle import oracle as O
+from tests.gpu_util import dev, host, smooth_fields, smooth_material
+
+pytestmark = pytest.mark.gpu
+SHAPE = (40, 17, 21)
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _lib():
+    sg.build()
+    O.lib()
+
+
+def _predicted(mat, u, um, dt, h):
+    """Planes i = 1, 2 of the predicted level, (3, nz + 4, ny + 4, 2)."""
+    nx, ny, nz = SHAPE
+    g = sg.grid_desc(nx, ny, nz, h, bc=(2,) * 6, sg_gp=6)
+    lib, ew = sg.lib(), C.c_void_p()
+    sg.check(lib.sw4g_ew_create_subdomain(C.byref(g), 1, nx, 1, ny, None, C.byref(ew)))
+    keep = [dev(a) for a in (*mat, u, um)]
+    sg.check(lib.sw4g_ew_set_material(ew, *[a.data_ptr() for a in keep[:3]], 1))
+    sg.check(lib.sw4g_ew_set_time_step(ew, dt, 0.0))
+    sg.check(lib.sw4g_ew_set_fields(ew, keep[3].data_ptr(), keep[4].data_ptr(), 1))
+    sg.check(lib.sw4g_ew_step_part(ew, 0))
+    buf = dev(np.zeros(lib.sw4g_ew_halo_bytes(ew, 0) // 8))
+    sg.check(lib.sw4g_ew_halo_pack(ew, 0, 0, buf.data_ptr()))
+    out = host(buf).reshape(3, nz + 4, ny + 4, 2)
+    sg.check(lib.sw4g_ew_destroy(ew))
+    prof = []
+    for ax, n in enumerate(SHAPE):
+        arr = [np.zeros(n + 4) for _ in range(3)]
+        sg.check(lib.sw4g_supergrid_profile(C.byref(g), ax, *[a.ctypes.data_as(sg._D) for a in arr]))
+        prof.append(arr[1])
+    return out, prof
+
+
+@pytest.mark.parametrize("which", ["mu", "lambda"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("i", [1, 2, 4])
+def test_predicted_level_is_not_finite_where_fp64_sums_are_not(which, bad, i):
+    nx, ny, nz = SHAPE
+    h = 0.05
+    mat = smooth_material(nx, ny, nz, seed=2)
+    dt = 0.3 * h / float(np.sqrt(np.max((4 * mat[1] + mat[2]) / mat[0])))
+    mat[1 if which == "mu" else 2].reshape(nz + 4, ny + 4, nx + 4)[12, 9, i + 1] = bad
+    u, um = smooth_fields(nx, ny, nz, seed=7)
+    got, st = _predicted(mat, u, um, dt, h)
+    lu = np.zeros_like(u)
+    O.rhs4sg(1, (-1, nx + 2, -1, ny + 2, -1, nz + 2), nz, [0] * 6, lu, u, mat[1], mat[2], h, *st)
+    want = (2 * u - um + dt * dt / np.tile(mat[0], 3) * lu).reshape(3, nz + 4, ny + 4, nx + 4)[..., 2:4]
+    m = (slice(None), slice(2, -2), slice(2, -2))
+    assert np.array_equal(np.isfinite(got[m]), np.isfinite(want[m]))
+    ok = np.isfinite(want[m])
+    assert np.max(np.abs(got[m] - want[m])[ok]) <= 2.0 ** -45 * np.max(np.abs(u))
