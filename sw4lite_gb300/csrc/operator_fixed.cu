@@ -86,7 +86,9 @@ __device__ __forceinline__ int upper(int e) { return e >> 16; }
 __device__ __forceinline__ int lower(int e) { return (short)(e & 0xffff); }
 
 // The points of a column whose sums read a field or material value or a stretching factor
-// that is not finite, set to NaN after the march (see stage_fixed.cu).
+// that is not finite, set to NaN after the march (see stage_fixed.cu: of the material a
+// component reads mu at every point of the three axes, lambda at its own point and along
+// its own axis).
 __device__ void mark_not_finite(const OpFixed& a, int i, int j, int kbeg, int kend)
 {
    const Box& b = a.b;
@@ -95,14 +97,14 @@ __device__ void mark_not_finite(const OpFixed& a, int i, int j, int kbeg, int ke
    for (int k = kbeg; k <= kend; k++) {
       const long long p = pidx(b, i, j, k);
       auto bad = [&](int c, long long q) { return !isfinite(a.u[c * b.cs + b.ps * q]); };
-      auto coef = [&](long long q) { return !isfinite(a.mu[q]) || !isfinite(a.la[q]); };
-      bool nan[3] = {bad(0, p), bad(1, p), bad(2, p)}, all = coef(p);
+      bool nan[3] = {bad(0, p), bad(1, p), bad(2, p)}, all = !isfinite(a.mu[p]) || !isfinite(a.la[p]);
       for (int ax = 0; ax < 3; ax++)
          for (int m = -2; m <= 2; m++) {
             all = all || !isfinite(str[ax][(ax == 2 ? k : 0) + m]);
             if (m == 0) continue;
             const long long q = p + m * st[ax];
-            all = all || coef(q);
+            all = all || !isfinite(a.mu[q]);
+            nan[ax] = nan[ax] || !isfinite(a.la[q]);
             for (int c = 0; c < 3; c++) {
                nan[c] = nan[c] || bad(c, q);
                if (c == ax) continue;

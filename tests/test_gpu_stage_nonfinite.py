@@ -1,5 +1,5 @@
-"""Material values that are not finite, in one stage of the FP64 time step: the predicted
-level is NaN or infinite exactly where the same sums in FP64 are, and elsewhere within the
+"""Material values that are not finite, in the kernel-level operator and in one stage of
+the FP64 time step.  The predicted level is NaN or infinite exactly where the same sums in FP64 are, and elsewhere within the
 rounding of two sums of 80 products (2 x 80 x 2^-53 < 2^-45 of the largest value).  A
 subdomain that is the whole grid steps part by part; after its first part the two interior
 planes next to a side can be read as a halo, so the planted point lies there.
@@ -64,3 +64,27 @@ def test_predicted_level_is_not_finite_where_fp64_sums_are_not(which, bad, i):
     assert np.array_equal(np.isfinite(got[m]), np.isfinite(want[m]))
     ok = np.isfinite(want[m])
     assert np.max(np.abs(got[m] - want[m])[ok]) <= 2.0 ** -45 * np.max(np.abs(u))
+
+
+@pytest.mark.parametrize("soa", [1, 0])
+@pytest.mark.parametrize("bad", [np.nan, -np.inf])
+def test_operator_lambda_not_finite(soa, bad):
+    """The kernel-level operator: lambda enters all components at its own point and one
+    component along each axis.  The bar is that of the operator's tile tests."""
+    nx, ny, nz = SHAPE
+    _, mu, la = smooth_material(nx, ny, nz, seed=4)
+    u, _ = smooth_fields(nx, ny, nz, seed=5)
+    la.reshape(nz + 4, ny + 4, nx + 4)[11, 8, 30] = bad
+    st = [np.ones(n + 4) for n in SHAPE]
+    b = (-1, nx + 2, -1, ny + 2, -1, nz + 2)
+    want = np.zeros_like(u)
+    O.rhs4sg(soa, b, nz, [0] * 6, want, u, mu, la, 0.3, *st)
+    lu = dev(np.zeros_like(u))
+    d = [dev(a) for a in (u, mu, la, *st)]
+    sg.check(sg.lib().sw4g_rhs4sg(soa, *b, nz, (C.c_int * 6)(), lu.data_ptr(), *[t.data_ptr() for t in d[:3]], 0.3,
+                                  *[t.data_ptr() for t in d[3:]], None))
+    got = host(lu)
+    assert np.array_equal(np.isfinite(got), np.isfinite(want))
+    ok = np.isfinite(want)
+    scale = 64 * np.max((2 * mu + la)[np.isfinite(la)]) * np.max(np.abs(u)) / 0.3 ** 2
+    assert np.max(np.abs(got - want)[ok]) <= 2.0 ** -46 * scale
