@@ -155,7 +155,7 @@ int EW::init()
    return kOk;
 }
 
-// The fixed-point stages' coefficients take 212 bytes a point, the FP64 stages' weights
+// The fixed-point stages' coefficients take 224 bytes a point, the FP64 stages' weights
 // 144.  The fixed-point stages run where their coefficients fit and leave room for the
 // phase order's work arrays (72 bytes a point, allocated when first used), so a grid that
 // fits with the FP64 stages alone runs on those: at 512^3 a step takes 95 ms on the FP64
@@ -166,12 +166,13 @@ int EW::alloc_stage_coefficients()
    const size_t n = (size_t)npts_;
    const Box b = make_box(1, b_.ib, b_.ie, b_.jb, b_.je, b_.kb, b_.ke);
    const size_t wbytes = (size_t)fixed_weight_len(b) * sizeof(int2);
-   const size_t need = wbytes + n * (sizeof(int4) + sizeof(int) + 9 * sizeof(double));
+   const size_t need = wbytes + n * (sizeof(int4) + 4 * sizeof(int) + 9 * sizeof(double));
    size_t free = 0, total = 0;
    SW4G_TRY(cuda_ok(cudaMemGetInfo(&free, &total)));
    if (free >= need + (size_t)(64 << 20)) {
       if (cudaMalloc(&fc_.w, wbytes) == cudaSuccess && cudaMalloc(&fc_.c, n * sizeof(int4)) == cudaSuccess &&
-          cudaMalloc(&fc_.e, n * sizeof(int)) == cudaSuccess && cudaMalloc(&fc_.bad, sizeof(int)) == cudaSuccess)
+          cudaMalloc(&fc_.e, n * sizeof(int)) == cudaSuccess && cudaMalloc(&fc_.ew, 3 * n * sizeof(int)) == cudaSuccess &&
+          cudaMalloc(&fc_.bad, sizeof(int)) == cudaSuccess)
          return kOk;
       cudaGetLastError();
       free_fixed_coefficients();
@@ -187,6 +188,7 @@ void EW::free_fixed_coefficients()
    if (fc_.w) cudaFree(fc_.w);
    if (fc_.c) cudaFree(fc_.c);
    if (fc_.e) cudaFree(fc_.e);
+   if (fc_.ew) cudaFree(fc_.ew);
    if (fc_.bad) cudaFree(fc_.bad);
    fc_ = FixedCoef{};
 }

@@ -2,16 +2,18 @@
 //
 // GB300 issues FP64 at 1/64 of its FP32 and integer rate: measured per SM and clock,
 // 1.7 FP64 operations against 59 multiply-accumulates of 32 x 32 -> 64 bits, 64 funnel
-// shifts and about 110 simple integer operations.  A stencil sum in FP64 aligns,
-// rounds and normalises every term; here the values a point's stencil reads are aligned
-// once, to the largest exponent among them, as 57-bit integers (4 bits more than an
-// FP64 significand), the differences are exact integer sums, the products are
-// accumulated in 64-bit integers, and only the finished sum is normalised.
+// shifts and about 110 simple integer operations.  A stencil sum in FP64 aligns, rounds and
+// normalises every term; here the values that enter one sum are aligned once, to the largest
+// exponent among them, as 57-bit integers (4 bits more than an FP64 significand), the
+// differences are exact integer sums, the products are accumulated in 64-bit integers, and
+// only the finished sum is normalised.
 //
-// The error of a sum is a few units of 2^-57 of its largest term, against 2^-53 for each
-// FP64 operation.  Exponents belong to points, never to tiles: a result depends on the
-// values of the point's own stencil alone, so it does not change with the tiling, the
-// launch shape or a decomposition of the grid.
+// Every value, coefficient and product carries an exponent of its own, and only what is
+// added is aligned: the error of a sum is a few units of 2^-57 of its largest term, against
+// 2^-53 for each FP64 operation.  The components of a field, the coefficients of a point and
+// the axes of an operator may differ by any power of two.  A result depends on the values of
+// the point's own stencil alone, so it does not change with the tiling, the launch shape or a
+// decomposition of the grid.
 #pragma once
 
 #include <cstdint>
@@ -20,7 +22,6 @@ namespace sw4g {
 
 typedef long long i64;
 
-constexpr int kExpNone = -0x10000000;  // below any exponent
 constexpr int kSplit = 26;  // low limb of values and weights
 constexpr int kMask = (1 << kSplit) - 1;
 
@@ -51,6 +52,17 @@ struct Round {
    }
 };
 
+// x / 2^d to an integer beside it, the odd one unless it is exact, for any d >= 0: without a
+// bias, for fewer instructions than Round takes and an error of up to 1 against 1/2, where
+// the integers have bits to spare.
+__device__ __forceinline__ i64 to_odd(i64 x, int d)
+{
+   const i64 y = sar(x, d);
+   i64 z;
+   asm("shl.b64 %0, %1, %2;" : "=l"(z) : "l"(y), "r"(d));
+   return y | (i64)(z != x);
+}
+
 __device__ __forceinline__ i64 madw(int a, int b, i64 c)
 {
    i64 r;
@@ -59,6 +71,58 @@ __device__ __forceinline__ i64 madw(int a, int b, i64 c)
 }
 
 __device__ __forceinline__ int max4(int a, int b, int c, int d) { return max(max(a, b), max(c, d)); }
+
+// An FP64 value as an integer m with value m * 2^(e - 1079), |m| < 2^57, exact: its 53 bits
+// and four below; e is its biased exponent (at least 1, the subnormals').  True if it is not
+// finite; it counts as less than the smallest normal number.
+__device__ __forceinline__ bool to_fixed(double v, i64& m, int& e)
+{
+   const int hi = __double2hiint(v), eb = (hi >> 20) & 0x7ff;
+   const unsigned mh = (unsigned)(hi & 0xfffff) | (unsigned)(min(eb, 1) << 20);
+   const i64 t = (i64)(((unsigned long long)mh << 32) | (unsigned)__double2loint(v)) << 4;
+   const i64 s = (i64)(hi >> 31);
+   m = (t ^ s) - s;
+   e = eb == 2047 ? 1 : max(eb, 1);
+   return eb == 2047;
+}
+
+// An integer with an exponent of its own
+struct Num {
+   i64 m;
+   int e;
+};
+
+constexpr int kNone = -20000;  // below any exponent, in 16 bits: that of zero
+
+// How far |m| < 2^(top + 1) is from reaching bit `top`, from its upper word alone: less than
+// the distance where |m| < 2^32
+template <int top>
+__device__ __forceinline__ int headroom(i64 m)
+{
+   const int hi = (int)(m >> 32);
+   return max(__clz(hi ^ (hi >> 31)) - (63 - top), 0);
+}
+
+// m * 2^e with the leading bit of m brought to bit 60 (left at bit 61 if it is there): what is
+// formed from a difference keeps its accuracy, however small it is against its terms.  A
+// difference below 2^32 is left for `rest`.
+__device__ __forceinline__ Num normal(i64 m, int e)
+{
+   const int n = headroom<60>(m);
+   return Num{m << n, e - n};
+}
+__device__ __forceinline__ bool small(const Num& d) { return __clz((int)(d.m >> 32) ^ (int)(d.m >> 63)) > 3; }
+__device__ __forceinline__ void rest(Num& d)
+{
+   const int n = max(__clzll(d.m ^ (d.m >> 63)) - 3, 0);
+   d = Num{d.m << n, d.m == 0 ? kNone : d.e - n};
+}
+
+// The difference d1i(x) of values |x| < 2^57 aligned to the exponent e of the largest
+__device__ __forceinline__ Num difference(i64 x0, i64 x1, i64 x2, i64 x3, int e0, int e1, int e2, int e3, int e)
+{
+   return normal(((sar(x2, e - e2) - sar(x1, e - e1)) << 3) + (sar(x0, e - e0) - sar(x3, e - e3)), e);
+}
 
 // Three FP64 values as integers m[c] with value m[c] * 2^(e - 1079), |m[c]| < 2^57, e the
 // largest of their biased exponents (at least 1, the subnormals' exponent); bits below
@@ -104,30 +168,7 @@ __device__ __forceinline__ i64 mulc(i64 x, int2 c)
    return madw(xh, c.x, cross >> 31);
 }
 
-// x * f for |x| < 2^61 and a factor 0 < f <= 1 with its full relative precision, rounded
-// to nearest (the supergrid stretching, which falls to 1e-4 at the sides).
-struct Factor {
-   int hi, lo, down;
-   bool on;
-   __device__ __forceinline__ explicit Factor(double f)
-   {
-      on = __double_as_longlong(f) != 0x3ff0000000000000LL;
-      const int h = __double2hiint(f), e = ((h >> 20) & 0x7ff) - 1022;
-      const i64 c = (i64)(((unsigned long long)((h & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(f)) << 4;
-      hi = (int)(c >> kSplit);
-      lo = (int)(c & kMask) << 5;
-      down = -e;
-   }
-   __device__ __forceinline__ i64 operator()(i64 x) const
-   {
-      if (!on) return x;
-      const int xh = (int)(x >> 31), xl = (int)x & 0x7fffffff;
-      const i64 cross = madw(xl, hi, madw(xh, lo, (madw(xl, lo, 1LL << 30) >> 31) + (1LL << 30)));
-      return Round(down)(madw(xh, hi, cross >> 31));
-   }
-};
-
-// x * f / 2^e for |x| < 2^61 and any finite factor f, with its full relative precision,
+// x * f / 2^e for |x| < 2^62 and any finite factor f, with its full relative precision,
 // rounded to nearest; f / 2^e is below 1 in magnitude.
 struct Scale {
    int hi, lo, e;
@@ -150,13 +191,6 @@ struct Scale {
       return neg ? -r : r;
    }
 };
-
-// A value |v| < 2^e as such a coefficient, C = v * 2^(57 - e) rounded.
-__device__ __forceinline__ int2 to_coef(double v, int e)
-{
-   const i64 c = min(__double2ll_rn(scalbn(v, 57 - e)), (1LL << 57) - 1);
-   return make_int2((int)(c >> kSplit), (int)(c & kMask) << 5);
-}
 
 // p * 2^e as FP64, rounded once; below the normal range 0, above it infinite.
 __device__ __forceinline__ double from_block(i64 p, int e)

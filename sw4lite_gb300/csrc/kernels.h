@@ -21,13 +21,14 @@ struct WeightPtrs {
 
 // Coefficients of the fixed-point stage kernels (stage_fixed.cu): the weights of every
 // interior point's second differences, stored by blocks of kFixedBlock points along x
-// (24 lines of a block in a row; fixed_weight_len entries), the coefficients of the
-// mixed terms and the exponents of both at every array point.
+// (24 lines of a block in a row; fixed_weight_len entries) with exponents for each axis and
+// coefficient, and the coefficients of the mixed terms with theirs at every array point.
 constexpr int kFixedBlock = 32;
 struct FixedCoef {
    int2* w = nullptr;
    int4* c = nullptr;
    int* e = nullptr;
+   int* ew = nullptr;
    int* bad = nullptr;  // one flag: the material is not finite everywhere
 };
 long long fixed_weight_len(const Box& b);

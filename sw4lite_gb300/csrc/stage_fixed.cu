@@ -11,28 +11,33 @@
 // alone (damping_layers.cu).
 //
 //  * CTA = 32 x 6 columns marching up z through a 5-plane ring of the stage field in
-//    shared memory, 2-point halo: per point three 57-bit integers with one exponent.
+//    shared memory, 2-point halo: three 57-bit integers and their exponents a point.
 //    Two CTAs per SM at 168 registers: the 128 registers of 2 x 256 threads spill into an
-//    L1 that the shared memory leaves at a few KB (predictor at 512^3 19.6 ms, 32 x 6
-//    15.2 ms, one CTA of 32 x 12 18.3 ms).
-//  * Every sum has the exponent of the largest value it reads: per axis for the centred
-//    differences and the second differences along it, their largest for the point's sum.
-//  * The second differences' 24 weights per point (stretching folded in) are integers
-//    with one exponent per point, prepared once per material and stored by blocks of 32
-//    points, so that a warp reads 24 contiguous lines; each warp copies its own
-//    asynchronously, two axes ahead of their use.
+//    L1 that the shared memory leaves at a few KB (measured with one exponent a point:
+//    predictor at 512^3 19.6 ms, 32 x 6 15.2 ms, one CTA of 32 x 12 18.3 ms).
+//  * A value, a difference, a product and a weight each have their own exponent, so a
+//    component keeps its digits beside one that is any power of two larger.  A component's
+//    second differences are sums over w (x - x_0) on all three axes, aligned to the largest
+//    w x among them; the products of the mixed terms are aligned by the outer difference
+//    that reads them.
+//  * The second differences' 24 weights per point (stretching folded in) are integers with
+//    an exponent for each axis and coefficient, prepared once per material and stored by
+//    blocks of 32 points, so that a warp reads 24 contiguous lines; each warp copies its own
+//    asynchronously, three axes' and coefficients' lines ahead of their use.
 //  * A mixed derivative is the outer difference of a product G = c * D f formed once per
 //    point.  The nine first differences of a point serve its second differences' values
 //    and all three of its products: those for the x and y outer differences go to shared
 //    memory, those for the z outer difference into a register queue, so a plane is
 //    finished two planes later, when the last product along z is known.
 //  * FP64 remains in forming up - 2u + um and in the update.
-// What bounds them: the integer pipes (about 2300 instructions a warp of 32 points, half of
-// them at half rate), the corrector also the FP64 operations of its stage field.  At 512^3
-// the predictor takes 15.2 ms and the corrector 22.5 ms with the damping (28.2 ms with the
-// damping inside the kernel), against 40.6 and 53.8 ms with the sums in FP64 (stage_fused.cu), whose 160 and 198 FP64 operations a point saturate the
-// 1.7 that an SM completes per clock.  Against quad precision the levels after 50 steps are off
-// by 0.5 to 0.65 times what they were.
+// What bounds them: the latency of twelve warps an SM and the integer pipes (about 2900
+// instructions a warp of 32 points, half of them at half rate), the corrector also the FP64
+// operations of its stage field.  At 512^3 the predictor takes 17.9 ms and the corrector 25.5 ms
+// with the damping, against 40.6 and 53.8 ms with the sums in FP64 (stage_fused.cu), whose 160
+// and 198 FP64 operations a point saturate the 1.7 that an SM completes per clock.  (One
+// exponent for a point's three components, and one for all its weights, took 15.2 and 22.5 ms,
+// and cost a component below the others its digits.)  Against quad precision the levels after 50
+// steps are off by 0.47 to 0.69 times what they are with the sums in FP64.
 #include <algorithm>
 
 #include "common.cuh"
@@ -61,10 +66,9 @@ struct FixedArgs {
    const double* __restrict__ irho;
    const int2* __restrict__ w;    // second-difference weights, by blocks of 32 points
    const int4* __restrict__ c;    // lambda and mu coefficients of the mixed terms
-   const int* __restrict__ e;     // exponents of both: weights << 16 | coefficients
+   const int* __restrict__ e;     // exponents of both: lambda << 16 | mu
+   const int* __restrict__ ew;    // of the weights, npts for each axis: (2 mu + lambda) << 16 | mu
    const int* __restrict__ bad;   // nonzero: the material is not finite everywhere
-   const double* __restrict__ mu;  // read where the material is not finite
-   const double* __restrict__ la;
    int wbx, wny;                  // blocks per row and rows per plane of w
    const double* __restrict__ sx;
    const double* __restrict__ sy;
@@ -73,45 +77,64 @@ struct FixedArgs {
    int* emax;
 };
 
-// Exponent of coefficients beyond the range
+// Exponent of weights and coefficients that are not finite
 constexpr int kCoefBad = 0x7fff;
+
+constexpr int kStages = 3;     // of weights, four lines each
+constexpr int kLimb = 27;      // low limb of the second differences' factors
 
 struct Smem {
    i64 v[5][3][PLANE];         // stage field, ring of planes
    i64 gx[3][NX];              // products for the x outer difference: la (v_y + w_z), mu u_y, mu u_z
    i64 gy[3][NY];              // for the y outer difference: mu v_x, la (u_x + w_z), mu v_z
-   int2 w[TY][2][8][TX];       // weights of one axis for a row of points, two stages per warp
+   int2 w[TY][kStages][4][TX]; // weights of one axis and coefficient for a row of points
    i64 gz[4][3][NTHREADS];     // products for the z outer difference: mu w_x, mu w_y, la (u_x + v_y)
-   int gze[4][NTHREADS];       // of the four planes before, each thread its own column
-   int ve[5][PLANE];
-   int gxe[NX], gye[NY];
+                               // of the four planes before, each thread its own column
+   short ve[5][3][PLANE];      // exponents of all these
+   short gxe[3][NX], gye[3][NY], gze[4][3][NTHREADS];
    int bad;                    // a value of the stage field or of the material is not finite
 };
 
 __device__ __forceinline__ bool is_one(double x) { return __double_as_longlong(x) == 0x3ff0000000000000LL; }
 
-// Products of one point for one outer direction; la multiplies the sum of the two
-// differences s0, s1 (exponents es0, es1; stretching factors f0, f1), mu the differences
-// m0 (exponent es0) and m1 (exponent es1); value g * 2^(e - 1078).
+// times a stretching factor
+__device__ __forceinline__ Num stretched(const Num& d, double s)
+{
+   const Scale f(s);
+   return Num{f(d.m), d.e + f.e};
+}
+
+// Products of one point for one outer direction, value m * 2^(e - 1078): la times the sum of
+// the differences s0, s1 with stretching factors f0, f1, and mu times m0 and m1.  c, ec:
+// limbs and exponents of mu and lambda.
 struct Triple {
-   i64 la, m0, m1;
-   int e;
+   Num la, m0, m1;
 };
 
-__device__ __forceinline__ Triple products(i64 s0, i64 s1, i64 m0, i64 m1, int es0, int es1, int4 c, int ec,
-                                           double f0, double f1)
+__device__ __forceinline__ Num times(const Num& d, int x, int y, int ec)
 {
-   const int es = max(es0, es1);
-   const int d0 = es - es0 + 1, d1 = es - es1 + 1;
-   i64 a = sar(s0, d0), b = sar(s1, d1);
-   if (!is_one(f0)) a = Factor(f0)(a);
-   if (!is_one(f1)) b = Factor(f1)(b);
+   return Num{mulc(d.m, make_int2(x, y)), d.e + ec - 1};
+}
+
+__device__ __forceinline__ Triple products(Num s0, Num s1, const Num& m0, const Num& m1, int4 c, int ec, double f0, double f1)
+{
+   if (!is_one(f0)) s0 = stretched(s0, f0);
+   if (!is_one(f1)) s1 = stretched(s1, f1);
+   const int es = max(s0.e, s1.e), emu = (int)(short)(ec & 0xffff);
    Triple t;
-   t.la = mulc(a + b, make_int2(c.z, c.w));
-   t.m0 = mulc(sar(m0, d0), make_int2(c.x, c.y));
-   t.m1 = mulc(sar(m1, d1), make_int2(c.x, c.y));
-   t.e = es + ec;
+   t.la = Num{mulc(sar(s0.m, es - s0.e + 1) + sar(s1.m, es - s1.e + 1), make_int2(c.z, c.w)), es + (ec >> 16)};
+   t.m0 = times(m0, c.x, c.y, emu);
+   t.m1 = times(m1, c.x, c.y, emu);
    return t;
+}
+
+// The outer difference of four products, e the largest of their exponents, value
+// m * 2^(e - 1074).  Equal products leave zero, which has no exponent: a component that they do
+// not reach keeps its own.
+__device__ __forceinline__ Num outer(i64 g0, i64 g1, i64 g2, i64 g3, int e0, int e1, int e2, int e3, int e)
+{
+   const i64 d = d1i(sar(g0, e - e0 + 4), sar(g1, e - e1 + 4), sar(g2, e - e2 + 4), sar(g3, e - e3 + 4));
+   return Num{d, d == 0 ? kNone : e};
 }
 
 __device__ __forceinline__ void copy16(void* dst, const void* src)
@@ -131,9 +154,9 @@ __device__ __forceinline__ double stage_value(const FixedArgs& a, long long q)
 
 // The points of a column whose sums read a value that is not finite, set to NaN after the
 // march: the sums themselves took it as zero.  A component's second differences read the
-// component along the three axes; its mixed terms read another component at the points
-// off both axes in the plane of the two.  Of the material a component reads mu at every
-// point of the three axes, lambda at its own point and along its own axis.
+// component and its weights along the three axes; its mixed terms read another component at
+// the points off both axes in the plane of the two, lambda along its own axis and mu along
+// the others.
 // Returns the exponent field of NaN if there was such a point.
 template <int FORM>
 __device__ int mark_not_finite(const FixedArgs& a, int i, int j, int kbeg, int kend)
@@ -145,18 +168,17 @@ __device__ int mark_not_finite(const FixedArgs& a, int i, int j, int kbeg, int k
       auto bad = [&](int c, long long q) {
          return !isfinite(stage_value<FORM>(a, q + c * a.npts));
       };
-      bool coef = !isfinite(a.mu[p]) || !isfinite(a.la[p]), all = coef;
       bool nan[3] = {bad(0, p), bad(1, p), bad(2, p)};
-      for (int ax = 0; ax < 3; ax++)
+      for (int ax = 0; ax < 3; ax++) {
+         const int ew = a.ew[p + ax * a.npts];
+         for (int c = 0; c < 3; c++)
+            if ((c == ax ? ew >> 16 : (int)(short)(ew & 0xffff)) == kCoefBad) nan[c] = true;
          for (int m = -2; m <= 2; m++) {
             if (m == 0) continue;
             const long long q = p + m * st[ax];
-            const bool mu = !isfinite(a.mu[q]), la = !isfinite(a.la[q]);
-            all = all || mu;
-            nan[ax] = nan[ax] || la;
-            coef = coef || mu || la;
+            const bool mu = (short)(a.e[q] & 0xffff) == kCoefBad, la = (a.e[q] >> 16) == kCoefBad;
             for (int c = 0; c < 3; c++) {
-               nan[c] = nan[c] || bad(c, q);
+               nan[c] = nan[c] || bad(c, q) || (c == ax ? la : mu);
                if (c == ax) continue;
                for (int n = -2; n <= 2; n++)
                   if (n != 0 && bad(c, q + n * st[c])) nan[ax] = true;  // c_c of another component ...
@@ -164,9 +186,9 @@ __device__ int mark_not_finite(const FixedArgs& a, int i, int j, int kbeg, int k
                   if (n != 0 && bad(ax, q + n * st[c])) nan[c] = true;  // ... in both of the plane's
             }
          }
-      if (!coef && (a.e[p] >> 16) == kCoefBad) all = true;  // weights beyond the range
+      }
       for (int c = 0; c < 3; c++)
-         if (all || nan[c]) {
+         if (nan[c]) {
             a.out[p + c * a.npts] = __longlong_as_double(0x7ff8000000000000LL);
             em = 0x7ff;
          }
@@ -220,29 +242,31 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
       for (int r = 0; r < kPre; r++) {
          const int idx = tid + r * NTHREADS;
          if (idx < PLANE) {
-            i64 m[3];
-            int e;
-            if (to_block(pv[r][0], pv[r][1], pv[r][2], m, e)) sm.bad = 1;
 #pragma unroll
-            for (int c = 0; c < 3; c++) sm.v[q][c][idx] = m[c];
-            sm.ve[q][idx] = e;
+            for (int c = 0; c < 3; c++) {
+               i64 m;
+               int e;
+               if (to_fixed(pv[r][c], m, e)) sm.bad = 1;
+               sm.v[q][c][idx] = m;
+               sm.ve[q][c][idx] = (short)e;
+            }
          }
       }
    };
-   // The weights of the warp's row, axis by axis, through two stages of shared memory
-   // two axes ahead of their use; wsrc: the next ones to copy, two planes end to end
+   // The weights of the warp's row, four lines (one axis and coefficient) at a time, through
+   // three stages of shared memory; wsrc: the next ones to copy, two planes end to end
    // wstride apart
    const int2* wsrc = a.w + (((long long)(kbeg - a.kb - 2) * a.wny + (j - a.jb - 2)) * a.wbx + blockIdx.x) * (24 * TX);
-   const long long wstride = (long long)a.wny * a.wbx * (24 * TX) - 16 * TX;
-   int wax = 0, wk = kbeg;
+   const long long wstride = (long long)a.wny * a.wbx * (24 * TX) - 20 * TX;
+   int wunit = 0, wk = kbeg;
    auto copy_weights = [&](int stage) {
       if (row && wk <= kend) {
 #pragma unroll
-         for (int r = 0; r < 4; r++)
+         for (int r = 0; r < 2; r++)
             copy16(&sm.w[ty][stage][0][0] + (r * 32 + tx) * 2, wsrc + (r * 32 + tx) * 2);
-         wax = wax == 2 ? 0 : wax + 1;
-         wk += wax == 0 ? 1 : 0;
-         wsrc += wax == 0 ? wstride : 8 * TX;
+         wunit = wunit == 5 ? 0 : wunit + 1;
+         wk += wunit == 0 ? 1 : 0;
+         wsrc += wunit == 0 ? wstride : 4 * TX;
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
    };
@@ -266,12 +290,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
       }
    }
 
-   i64 pq[2][3];  // sums of planes k-2, k-1
-   int pe[2];
+   Num pq[2][3];  // sums of planes k-2, k-1, value m * 2^(e - 1072)
 #pragma unroll
-   for (int q = 0; q < 4; q++) sm.gze[q][tid] = kExpNone, sm.gz[q][0][tid] = sm.gz[q][1][tid] = sm.gz[q][2][tid] = 0;
+   for (int c = 0; c < 3; c++) {
 #pragma unroll
-   for (int q = 0; q < 2; q++) pe[q] = kExpNone, pq[q][0] = pq[q][1] = pq[q][2] = 0;
+      for (int q = 0; q < 4; q++) sm.gze[q][c][tid] = (short)kNone, sm.gz[q][c][tid] = 0;
+      pq[0][c] = pq[1][c] = Num{0, kNone};
+   }
    int em = 0;
 
    if (tid == 0) sm.bad = *a.bad;
@@ -285,7 +310,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
    fetch(kbeg);
    copy_weights(0);
    copy_weights(1);
-   int stage = 0;
+   copy_weights(2);
    for (int k = kbeg - 2; k <= kend + 2; k++) {
       const bool full = k >= kbeg && k <= kend;
       const long long plane = a.nij * (long long)(k - a.kb);
@@ -294,159 +319,147 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
       __syncthreads();
       // coefficients, used after the second differences
       int4 cc = make_int4(0, 0, 0, 0), hc = make_int4(0, 0, 0, 0);
-      int ee = 0, he = 0;
+      int ee = 0, he = 0, ew[3] = {0, 0, 0};
       if (inside) {
          cc = __ldg(a.c + plane + col);
          ee = __ldg(a.e + plane + col);
-      }
-      if (hcol >= 0) {
-         hc = __ldg(a.c + plane + hcol);
-         he = __ldg(a.e + plane + hcol);
+         if (full)
+#pragma unroll
+            for (int ax = 0; ax < 3; ax++) ew[ax] = __ldg(a.ew + plane + col + ax * npts);
       }
       const double szk = __ldg(a.sz + (k - a.kb));
       const i64* v0 = &sm.v[q0][0][0];
-      const int* e0 = sm.ve[q0];
-      const int ec = (int)(short)(ee & 0xffff), ew = ee >> 16;
+      const short* e0 = &sm.ve[q0][0][0];
+      const int qz[4] = {qm2, qm1, qp1, qp2};
+      // value and exponent of component c at the point s, m points along an axis of the plane
+      // (stride o) or, as down, planes
+      auto along = [&](int c, int s, int o) {
+         const i64* v = v0 + c * PLANE + s;
+         const short* e = e0 + c * PLANE + s;
+         const int x0 = e[-2 * o], x1 = e[-o], x2 = e[o], x3 = e[2 * o];
+         return difference(v[-2 * o], v[-o], v[o], v[2 * o], x0, x1, x2, x3, max4(x0, x1, x2, x3));
+      };
+      auto down = [&](int c, int s) {
+         const int x0 = sm.ve[qm2][c][s], x1 = sm.ve[qm1][c][s], x2 = sm.ve[qp1][c][s], x3 = sm.ve[qp2][c][s];
+         return difference(sm.v[qm2][c][s], sm.v[qm1][c][s], sm.v[qp1][c][s], sm.v[qp2][c][s], x0, x1, x2, x3, max4(x0, x1, x2, x3));
+      };
 
-      int ex[4], ey[4];
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-         const int s = m < 2 ? m - 2 : m - 1;
-         ex[m] = e0[own + s];
-         ey[m] = e0[own + s * PX];
-      }
-      const int Ex = max4(ex[0], ex[1], ex[2], ex[3]), Ey = max4(ey[0], ey[1], ey[2], ey[3]);
-      int Ez = 0;
-      i64 dx[3], dy[3], dz[3];
+      Num D[3][3];  // differences along x, y, z of the components
       i64 S[3] = {0, 0, 0};
-      int eS = kExpNone;
+      int eS[3] = {kNone, kNone, kNone};
 
       if (!full) {
+         D[0][0] = along(0, own, 1);
+         D[0][2] = along(2, own, 1);
+         D[1][1] = along(1, own, PX);
+         D[1][2] = along(2, own, PX);
+      } else {
+         // the largest exponent along each axis, and of a component's w x
+         int E[3][3], eo[3];
 #pragma unroll
          for (int c = 0; c < 3; c++) {
-            const i64* v = v0 + c * PLANE + own;
-            if (c != 1) dx[c] = d1i(sar(v[-2], Ex - ex[0]), sar(v[-1], Ex - ex[1]), sar(v[1], Ex - ex[2]), sar(v[2], Ex - ex[3]));
-            if (c != 0) dy[c] = d1i(sar(v[-2 * PX], Ey - ey[0]), sar(v[-PX], Ey - ey[1]), sar(v[PX], Ey - ey[2]), sar(v[2 * PX], Ey - ey[3]));
+            const short* e = e0 + c * PLANE + own;
+            eo[c] = e[0];
+            E[0][c] = max4(e[-2], e[-1], e[1], e[2]);
+            E[1][c] = max4(e[-2 * PX], e[-PX], e[PX], e[2 * PX]);
+            E[2][c] = max4(sm.ve[qm2][c][own], sm.ve[qm1][c][own], sm.ve[qp1][c][own], sm.ve[qp2][c][own]);
+#pragma unroll
+            for (int ax = 0; ax < 3; ax++)
+               eS[c] = max(eS[c], max(E[ax][c], eo[c]) + (ax == c ? ew[ax] >> 16 : (int)(short)(ew[ax] & 0xffff)));
          }
-      } else {
-         const int qz[4] = {qm2, qm1, qp1, qp2};
-         int ez[4];
+         i64 cr[3] = {0, 0, 0};  // products of high and low limbs
 #pragma unroll
-         for (int m = 0; m < 4; m++) ez[m] = sm.ve[qz[m]][own];
-         Ez = max4(ez[0], ez[1], ez[2], ez[3]);
-         const int eo = e0[own];
-         const int E = max(max(Ex, Ey), max(Ez, eo));
-         i64 cr[3] = {1 << (kSplit - 1), 1 << (kSplit - 1), 1 << (kSplit - 1)};
-         int ch[3] = {0, 0, 0}, cl[3] = {0, 0, 0};  // limb sums of the weights: the centre's
-#pragma unroll
-         for (int ax = 0; ax < 3; ax++) {
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
+         for (int unit = 0; unit < 6; unit++) {
+            const int ax = unit / 2, t = unit % 2;
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
             __syncwarp();
-            int2 w[2][4];
+            int2 w[4];
 #pragma unroll
-            for (int t = 0; t < 2; t++)
-#pragma unroll
-               for (int m = 0; m < 4; m++) w[t][m] = sm.w[ty][stage][t * 4 + m][tx];
+            for (int m = 0; m < 4; m++) w[m] = sm.w[ty][unit % kStages][m][tx];
             __syncwarp();
-            copy_weights(stage);
-            stage ^= 1;
-            const int Ea = ax == 0 ? Ex : ax == 1 ? Ey : Ez;
+            copy_weights(unit % kStages);
+            const int et = t == 1 ? ew[ax] >> 16 : (int)(short)(ew[ax] & 0xffff);
 #pragma unroll
             for (int c = 0; c < 3; c++) {
+               if ((ax == c) != (t == 1)) continue;
+               const int E_ = E[ax][c], A = eS[c] - et;
                i64 x[4];
 #pragma unroll
                for (int m = 0; m < 4; m++) {
                   const int s = m < 2 ? m - 2 : m - 1;
-                  x[m] = ax == 0 ? v0[c * PLANE + own + s] : ax == 1 ? v0[c * PLANE + own + s * PX] : sm.v[qz[m]][c][own];
+                  const int e = ax == 0 ? e0[c * PLANE + own + s] : ax == 1 ? e0[c * PLANE + own + s * PX] : sm.ve[qz[m]][c][own];
+                  x[m] = sar(ax == 0 ? v0[c * PLANE + own + s] : ax == 1 ? v0[c * PLANE + own + s * PX] : sm.v[qz[m]][c][own], E_ - e);
                }
-               const int* e = ax == 0 ? ex : ax == 1 ? ey : ez;
-               const i64 d = d1i(sar(x[0], Ea - e[0]), sar(x[1], Ea - e[1]), sar(x[2], Ea - e[2]), sar(x[3], Ea - e[3]));
-               if (ax == 0) dx[c] = d;
-               if (ax == 1) dy[c] = d;
-               if (ax == 2) dz[c] = d;
-               const int2* wc = w[ax == c ? 1 : 0];
+               D[ax][c] = normal(d1i(x[0], x[1], x[2], x[3]), E_);
+               const i64 x0 = sar(v0[c * PLANE + own], A - eo[c]);
 #pragma unroll
                for (int m = 0; m < 4; m++) {
-                  const i64 y = sar(x[m], E - e[m]);
-                  const int xh = (int)(y >> kSplit), xl = (int)y & kMask;
-                  S[c] = madw(xh, wc[m].x, S[c]);
-                  cr[c] = madw(xh, wc[m].y, cr[c]);
-                  cr[c] = madw(xl, wc[m].x, cr[c]);
+                  const i64 y = sar(x[m], A - E_) - x0;
+                  const int xh = (int)(y >> kLimb), xl = (int)y & ((1 << kLimb) - 1);
+                  S[c] = madw(xh, w[m].x, S[c]);
+                  cr[c] = madw(xh, w[m].y, cr[c]);
+                  cr[c] = madw(xl, w[m].x, cr[c]);
                }
             }
-#pragma unroll
-            for (int t = 0; t < 2; t++) {
-               const int sh = (w[t][0].x + w[t][1].x) + (w[t][2].x + w[t][3].x);
-               const int sl = (w[t][0].y + w[t][1].y) + (w[t][2].y + w[t][3].y);
-#pragma unroll
-               for (int c = 0; c < 3; c++)
-                  if ((ax == c) == (t == 1)) {
-                     ch[c] -= sh;
-                     cl[c] -= sl;
-                  }
-            }
          }
 #pragma unroll
-         for (int c = 0; c < 3; c++) {
-            const i64 x = sar(v0[c * PLANE + own], E - eo);
-            const int xh = (int)(x >> kSplit), xl = (int)x & kMask;
-            cr[c] = madw(xl, ch[c], madw(xh, cl[c], cr[c]));
-            S[c] = madw(xh, ch[c], S[c]) + (cr[c] >> kSplit);
+         for (int c = 0; c < 3; c++) {  // with as many of the lower bits as there is room for
+            const int n = min(headroom<61>(S[c]), kLimb);
+            S[c] = (S[c] << n) + to_odd(cr[c], kLimb - n);
+            eS[c] -= 9 + n;
          }
-         eS = E + ew - 11;
+      }
+
+      // differences that cancelled almost or fully
+      if (!full) {
+         rest(D[0][0]), rest(D[0][2]), rest(D[1][1]), rest(D[1][2]);
+      } else {
+         bool any = false;
+#pragma unroll
+         for (int ax = 0; ax < 3; ax++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) any = any || small(D[ax][c]);
+         if (any)
+#pragma unroll
+            for (int ax = 0; ax < 3; ax++)
+#pragma unroll
+               for (int c = 0; c < 3; c++) rest(D[ax][c]);
       }
 
       // Products of the own point
       const bool stz = !is_one(szk);
-      const Triple z = products(dx[0], dy[1], dx[2], dy[2], Ex, Ey, cc, ec, sxi, syj);
+      const Triple z = products(D[0][0], D[1][1], D[0][2], D[1][2], cc, ee, sxi, syj);
       if (full) {
-         Triple t = products(dy[1], dz[2], dy[0], dz[0], Ey, Ez, cc, ec, syj, szk);
-         const int qx = ty * PX + tx + HALO;
-         sm.gx[0][qx] = t.la;
-         sm.gx[1][qx] = t.m0;
-         sm.gx[2][qx] = t.m1;
-         sm.gxe[qx] = t.e;
-         t = products(dx[0], dz[2], dx[1], dz[1], Ex, Ez, cc, ec, sxi, szk);
-         const int qy = (ty + HALO) * TX + tx;
-         sm.gy[0][qy] = t.m0;
-         sm.gy[1][qy] = t.la;
-         sm.gy[2][qy] = t.m1;
-         sm.gye[qy] = t.e;
+         auto to_x = [&](const Triple& t, int q) {
+            sm.gx[0][q] = t.la.m;
+            sm.gx[1][q] = t.m0.m;
+            sm.gx[2][q] = t.m1.m;
+            sm.gxe[0][q] = (short)t.la.e;
+            sm.gxe[1][q] = (short)t.m0.e;
+            sm.gxe[2][q] = (short)t.m1.e;
+         };
+         auto to_y = [&](const Triple& t, int q) {
+            sm.gy[0][q] = t.m0.m;
+            sm.gy[1][q] = t.la.m;
+            sm.gy[2][q] = t.m1.m;
+            sm.gye[0][q] = (short)t.m0.e;
+            sm.gye[1][q] = (short)t.la.e;
+            sm.gye[2][q] = (short)t.m1.e;
+         };
+         to_x(products(D[1][1], D[2][2], D[1][0], D[2][0], cc, ee, syj, szk), ty * PX + tx + HALO);
+         to_y(products(D[0][0], D[2][2], D[0][1], D[2][1], cc, ee, sxi, szk), (ty + HALO) * TX + tx);
          if (halo) {
-            const int s = hrow * PX + hcl, o = yh ? 1 : PX;
-            const int qz[4] = {qm2, qm1, qp1, qp2};
-            int eh[4], ez[4];
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-               eh[m] = e0[s + (m < 2 ? m - 2 : m - 1) * o];
-               ez[m] = sm.ve[qz[m]][s];
-            }
-            const int Eh = max4(eh[0], eh[1], eh[2], eh[3]), Ezh = max4(ez[0], ez[1], ez[2], ez[3]);
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-               eh[m] = Eh - eh[m];
-               ez[m] = Ezh - ez[m];
-            }
             // y outer: mu v_x, la (u_x + w_z), mu v_z;  x outer: la (v_y + w_z), mu u_y, mu u_z
-            const int cs = (yh ? 0 : PLANE) + s, cm = (yh ? PLANE : 0) + s;
-            auto along = [&](int q) { return d1i(sar(v0[q - 2 * o], eh[0]), sar(v0[q - o], eh[1]), sar(v0[q + o], eh[2]), sar(v0[q + 2 * o], eh[3])); };
-            auto down = [&](int q) {
-               return d1i(sar(sm.v[qm2][0][q], ez[0]), sar(sm.v[qm1][0][q], ez[1]), sar(sm.v[qp1][0][q], ez[2]), sar(sm.v[qp2][0][q], ez[3]));
-            };
-            t = products(along(cs), down(2 * PLANE + s), along(cm), down(cm), Eh, Ezh, hc, (int)(short)(he & 0xffff), hst, szk);
-            if (yh) {
-               const int q = hrow * TX + tx;
-               sm.gy[0][q] = t.m0;
-               sm.gy[1][q] = t.la;
-               sm.gy[2][q] = t.m1;
-               sm.gye[q] = t.e;
-            } else {
-               const int q = (hrow - HALO) * PX + hcl;
-               sm.gx[0][q] = t.la;
-               sm.gx[1][q] = t.m0;
-               sm.gx[2][q] = t.m1;
-               sm.gxe[q] = t.e;
+            const int s = hrow * PX + hcl, o = yh ? 1 : PX, cs = yh ? 0 : 1, cm = 1 - cs;
+            if (hcol >= 0) {
+               hc = __ldg(a.c + plane + hcol);
+               he = __ldg(a.e + plane + hcol);
             }
+            Num d0 = along(cs, s, o), d1 = down(2, s), d2 = along(cm, s, o), d3 = down(cm, s);
+            if (small(d0) || small(d1) || small(d2) || small(d3)) rest(d0), rest(d1), rest(d2), rest(d3);
+            const Triple t = products(d0, d1, d2, d3, hc, he, hst, szk);
+            if (yh) to_y(t, hrow * TX + tx);
+            else to_x(t, (hrow - HALO) * PX + hcl);
          }
       }
       __syncthreads();
@@ -467,58 +480,41 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
       if (k < kend) fetch(k + 3);
 
       // plane k: second differences and the x and y outer differences
-      i64 P[3] = {0, 0, 0};
-      int eP = kExpNone;
+      Num P[3] = {{0, kNone}, {0, kNone}, {0, kNone}};
       if (full) {
-         const i64* gx = &sm.gx[0][ty * PX + tx];
-         const i64* gy = &sm.gy[0][ty * TX + tx];
-         int hx[4], hy[4];
-#pragma unroll
-         for (int m = 0; m < 4; m++) {
-            const int n = m < 2 ? m : m + 1;
-            hx[m] = sm.gxe[ty * PX + tx + n];
-            hy[m] = sm.gye[(ty + n) * TX + tx];
-         }
-         const int Eg = max(max4(hx[0], hx[1], hx[2], hx[3]), max4(hy[0], hy[1], hy[2], hy[3]));
-         eP = max(eS, Eg);
-         const Round of_s(eP - eS + 1), of_g(eP - Eg + 2);
-#pragma unroll
-         for (int m = 0; m < 4; m++) {
-            hx[m] = Eg - hx[m] + 4;
-            hy[m] = Eg - hy[m] + 4;
-         }
 #pragma unroll
          for (int c = 0; c < 3; c++) {
-            const i64* x = gx + c * NX;
-            const i64* y = gy + c * NY;
-            i64 cx = d1i(sar(x[0], hx[0]), sar(x[1], hx[1]), sar(x[3], hx[2]), sar(x[4], hx[3]));
-            i64 cy = d1i(sar(y[0], hy[0]), sar(y[TX], hy[1]), sar(y[3 * TX], hy[2]), sar(y[4 * TX], hy[3]));
+            const i64* x = &sm.gx[c][ty * PX + tx];
+            const i64* y = &sm.gy[c][ty * TX + tx];
+            const short* xe = &sm.gxe[c][ty * PX + tx];
+            const short* ye = &sm.gye[c][ty * TX + tx];
+            const int hx[4] = {xe[0], xe[1], xe[3], xe[4]}, hy[4] = {ye[0], ye[TX], ye[3 * TX], ye[4 * TX]};
+            Num cx = outer(x[0], x[1], x[3], x[4], hx[0], hx[1], hx[2], hx[3], max4(hx[0], hx[1], hx[2], hx[3]));
+            Num cy = outer(y[0], y[TX], y[3 * TX], y[4 * TX], hy[0], hy[1], hy[2], hy[3], max4(hy[0], hy[1], hy[2], hy[3]));
             if (stx || sty || stz) {
-               cx = Factor(c == 0 ? sxi : c == 1 ? sxi * syj : sxi * szk)(cx);
-               cy = Factor(c == 0 ? syj * sxi : c == 1 ? syj : syj * szk)(cy);
+               cx = stretched(cx, c == 0 ? sxi : c == 1 ? sxi * syj : sxi * szk);
+               cy = stretched(cy, c == 0 ? syj * sxi : c == 1 ? syj : syj * szk);
             }
-            P[c] = of_s(S[c]) + of_g(cx + cy);
+            P[c].e = max(eS[c], max(cx.e, cy.e));
+            P[c].m = to_odd(S[c], P[c].e - eS[c] + 1) + to_odd(cx.m, P[c].e - cx.e + 2) + to_odd(cy.m, P[c].e - cy.e + 2);
          }
       }
 
       // plane k - 2: the z outer difference, then the update
       if (finish) {
          const int z0 = k & 3, z1 = (k + 1) & 3, z3 = (k + 3) & 3;  // planes k-4, k-3, k-1
-         int h0 = sm.gze[z0][tid], h1 = sm.gze[z1][tid], h3 = sm.gze[z3][tid];
-         const int Eg = max4(h0, h1, h3, z.e);
-         const int eF = max(pe[0], Eg);
-         const Round of_p(eF - pe[0]), of_z(eF - Eg + 2);
-         h0 = Eg - h0 + 4, h1 = Eg - h1 + 4, h3 = Eg - h3 + 4;
-         const int h4 = Eg - z.e + 4;
          const double szp = __ldg(a.sz + (kp - a.kb));
          const bool st = stx || sty || !is_one(szp);
-         const i64 zn[3] = {z.m0, z.m1, z.la};
+         const Num zn[3] = {z.m0, z.m1, z.la};
          const double cr = a.coef * ir;
 #pragma unroll
          for (int c = 0; c < 3; c++) {
-            i64 cz = d1i(sar(sm.gz[z0][c][tid], h0), sar(sm.gz[z1][c][tid], h1), sar(sm.gz[z3][c][tid], h3), sar(zn[c], h4));
-            if (st) cz = Factor(c == 0 ? szp * sxi : c == 1 ? szp * syj : szp)(cz);
-            const double lu = from_block(of_p(pq[0][c]) + of_z(cz), eF - 1072);
+            const int h0 = sm.gze[z0][c][tid], h1 = sm.gze[z1][c][tid], h3 = sm.gze[z3][c][tid], h4 = zn[c].e;
+            Num g = outer(sm.gz[z0][c][tid], sm.gz[z1][c][tid], sm.gz[z3][c][tid], zn[c].m, h0, h1, h3, h4, max4(h0, h1, h3, h4));
+            if (st) g = stretched(g, c == 0 ? szp * sxi : c == 1 ? szp * syj : szp);
+            const int eF = max(pq[0][c].e, g.e);
+            const i64 F = to_odd(pq[0][c].m, eF - pq[0][c].e) + to_odd(g.m, eF - g.e + 2);
+            const double lu = from_block(F, eF - 1072);
             const double v = base[c] + cr * lu;
             if (FORM != 0) em = max(em, (__double2hiint(v) >> 20) & 0x7ff);
             a.out[pp + c * npts] = v;
@@ -526,17 +522,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
       }
 
       // queues
-      sm.gz[k & 3][0][tid] = z.m0;
-      sm.gz[k & 3][1][tid] = z.m1;
-      sm.gz[k & 3][2][tid] = z.la;
-      sm.gze[k & 3][tid] = z.e;
+      const Num zn[3] = {z.m0, z.m1, z.la};
 #pragma unroll
       for (int c = 0; c < 3; c++) {
+         sm.gz[k & 3][c][tid] = zn[c].m;
+         sm.gze[k & 3][c][tid] = (short)zn[c].e;
          pq[0][c] = pq[1][c];
          pq[1][c] = P[c];
       }
-      pe[0] = pe[1];
-      pe[1] = eP;
       const int next = qm2;
       qm2 = qm1;
       qm1 = q0;
@@ -551,44 +544,44 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
    }
 }
 
-// The smallest e with x < 2^e, from the bit pattern of a positive x (-1022 for zero).
-__device__ __forceinline__ int exponent_above(double x) { return ((__double2hiint(x) >> 20) & 0x7ff) - 1022; }
-
 // Coefficients of the fixed-point stages.  For every array point: mu and lambda over
-// 144 h^2 with the exponent of the larger; for every interior point the weights of its
-// second differences (src/rhs4sg_rev.C:114-136)
+// 144 h^2; for every interior point the weights of its second differences
+// (src/rhs4sg_rev.C:114-136)
 //   a(q-1) - 3/4 (a(q) + a(q-2)),  a(q-2) + a(q+1) + 3 (a(q) + a(q-1))  and their mirrors
-// of a = mu s and a = (2 mu + lambda) s along each axis, times s / (6 h^2), with the
-// exponent of twice the largest sum of absolute values of one component's twelve.
+// of a = mu s and a = (2 mu + lambda) s along each axis, times s / (6 h^2), each four with
+// the exponent that leaves the sum of their magnitudes below 2^56.  What is not finite counts
+// as zero and has the exponent kCoefBad; the points that read it are marked after a march.
 __global__ void fixed_coef_kernel(Box b, const double* __restrict__ mu, const double* __restrict__ la,
                                   const double* __restrict__ sx, const double* __restrict__ sy,
                                   const double* __restrict__ sz, double scale, double cof144, int wbx, int wny,
                                   int2* __restrict__ w, int4* __restrict__ c, int* __restrict__ e,
-                                  int* __restrict__ bad)
+                                  int* __restrict__ ew, int* __restrict__ bad)
 {
    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < b.npts;
         p += (long long)gridDim.x * blockDim.x) {
       const int i = b.ib + (int)(p % b.ni);
       const int j = b.jb + (int)((p / b.ni) % (b.je - b.jb + 1));
       const int k = b.kb + (int)(p / b.nij);
-      // a coefficient that is not finite counts as zero; the points that read it are marked
-      // after the march
-      bool finite = true;
-      auto clean = [&](double v) {
-         if (isfinite(v)) return v;
-         finite = false;
-         return 0.0;
+      bool any = false;
+      auto coef = [&](double v, int2& limbs) {
+         i64 m;
+         int x;
+         const bool nf = to_fixed(v, m, x);
+         any = any || nf;
+         if (nf) m = 0;
+         limbs = make_int2((int)(m >> kSplit), (int)(m & kMask) << 5);
+         return nf ? kCoefBad : x - 1022;
       };
-      const double m = clean(mu[p] * cof144), l = clean(la[p] * cof144);
-      int ec = max(exponent_above(fmax(fabs(m), fabs(l))), -900);
-      const int2 cm = to_coef(m, ec), cl = to_coef(l, ec);
+      int2 cm, cl;
+      const int em = coef(mu[p] * cof144, cm), el = coef(la[p] * cof144, cl);
       c[p] = make_int4(cm.x, cm.y, cl.x, cl.y);
-      if (!(fabs(m) <= 1e300 && fabs(l) <= 1e300)) ec = kCoefBad;
-      int ew = -1022;
+      e[p] = (int)((unsigned)el << 16 | ((unsigned)em & 0xffffu));
       if (i >= b.ib + 2 && i <= b.ie - 2 && j >= b.jb + 2 && j <= b.je - 2 && k >= b.kb + 2 && k <= b.ke - 2) {
          const long long st[3] = {1, b.ni, b.nij};
          const double* sv[3] = {sx + (i - b.ib), sy + (j - b.jb), sz + (k - b.kb)};
-         double wt[3][2][4], sum[3][2];
+         const int ii = i - b.ib - 2;
+         int2* o = w + ((((long long)(k - b.kb - 2) * wny + (j - b.jb - 2)) * wbx + ii / kFixedBlock) * 24) * kFixedBlock +
+                   ii % kFixedBlock;
 #pragma unroll
          for (int ax = 0; ax < 3; ax++) {
             double av[2][5];
@@ -600,45 +593,37 @@ __global__ void fixed_coef_kernel(Box b, const double* __restrict__ mu, const do
                av[1][q + 2] = (2 * mu[pq] + la[pq]) * s;
             }
             const double f = scale * sv[ax][0];
+            int et[2];
 #pragma unroll
             for (int t = 0; t < 2; t++) {
                const double* v = av[t];
-               wt[ax][t][0] = f * (v[1] - 0.75 * (v[2] + v[0]));
-               wt[ax][t][1] = f * (v[0] + v[3] + 3 * (v[2] + v[1]));
-               wt[ax][t][2] = f * (v[1] + v[4] + 3 * (v[3] + v[2]));
-               wt[ax][t][3] = f * (v[3] - 0.75 * (v[2] + v[4]));
+               const double wt[4] = {f * (v[1] - 0.75 * (v[2] + v[0])), f * (v[0] + v[3] + 3 * (v[2] + v[1])),
+                                     f * (v[1] + v[4] + 3 * (v[3] + v[2])), f * (v[3] - 0.75 * (v[2] + v[4]))};
+               i64 m[4], sum = 0;
+               int x[4];
+               bool nf = false;
 #pragma unroll
-               for (int q = 0; q < 4; q++) wt[ax][t][q] = clean(wt[ax][t][q]);
-               sum[ax][t] = fabs(wt[ax][t][0]) + fabs(wt[ax][t][1]) + fabs(wt[ax][t][2]) + fabs(wt[ax][t][3]);
-            }
-         }
-         double most = 0;
-#pragma unroll
-         for (int q = 0; q < 3; q++) {
-            double s = 0;
-#pragma unroll
-            for (int ax = 0; ax < 3; ax++) s += sum[ax][ax == q ? 1 : 0];
-            most = fmax(most, s);
-         }
-         ew = max(exponent_above(2 * most), -900);
-         if (!(most <= 1e300)) ew = kCoefBad;
-         const int ii = i - b.ib - 2;
-         int2* o = w + ((((long long)(k - b.kb - 2) * wny + (j - b.jb - 2)) * wbx + ii / kFixedBlock) * 24) * kFixedBlock +
-                   ii % kFixedBlock;
-         const double up = ew == kCoefBad ? 0.0 : scalbn(1.0, 57 - ew);
-#pragma unroll
-         for (int ax = 0; ax < 3; ax++)
-#pragma unroll
-            for (int t = 0; t < 2; t++)
+               for (int q = 0; q < 4; q++)
+                  if (to_fixed(wt[q], m[q], x[q])) nf = true;
+               const int most = max4(x[0], x[1], x[2], x[3]);
 #pragma unroll
                for (int q = 0; q < 4; q++) {
-                  const i64 v = __double2ll_rn(wt[ax][t][q] * up);
-                  const i64 hi = (v + (1 << (kSplit - 1))) >> kSplit;
-                  o[((ax * 2 + t) * 4 + q) * kFixedBlock] = make_int2((int)hi, (int)(v - (hi << kSplit)));
+                  const i64 r = sar(m[q], most - x[q]);
+                  sum += r < 0 ? -r : r;
                }
+               const int down = nf ? 62 : max(8 - __clzll(sum), 0);  // sum < 2^(64 - clz)
+#pragma unroll
+               for (int q = 0; q < 4; q++) {
+                  const i64 r = nf ? 0 : Round(most - x[q] + down)(m[q]), hi = (r + (1 << (kLimb - 1))) >> kLimb;
+                  o[((ax * 2 + t) * 4 + q) * kFixedBlock] = make_int2((int)hi, (int)(r - (hi << kLimb)));
+               }
+               et[t] = nf ? kCoefBad : most + down - 1022;
+               any = any || nf;
+            }
+            ew[p + ax * b.npts] = (int)((unsigned)et[1] << 16 | ((unsigned)et[0] & 0xffffu));
+         }
       }
-      if (!finite || ew == kCoefBad || ec == kCoefBad) *bad = 1;
-      e[p] = (int)((unsigned)ew << 16 | ((unsigned)ec & 0xffffu));
+      if (any) *bad = 1;
    }
 }
 
@@ -657,7 +642,7 @@ int launch_fixed_coef(const Box& b, const double* mu, const double* la, const do
    const int nx = (int)(b.ie - b.ib - 3), ny = (int)(b.je - b.jb - 3);
    const long long blocks = std::min<long long>((b.npts + 127) / 128, 152LL * 32);
    fixed_coef_kernel<<<(int)blocks, 128, 0, s>>>(b, mu, la, sx, sy, sz, 1.0 / (6 * h * h), 1.0 / (144 * h * h),
-                                                 blocks_for(nx, kFixedBlock), ny, c.w, c.c, c.e, c.bad);
+                                                 blocks_for(nx, kFixedBlock), ny, c.w, c.c, c.e, c.ew, c.bad);
    return launch_status();
 }
 
@@ -703,9 +688,8 @@ int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
    a.w = st.fc.w;
    a.c = st.fc.c;
    a.e = st.fc.e;
+   a.ew = st.fc.ew;
    a.bad = st.fc.bad;
-   a.mu = st.mu;
-   a.la = st.la;
    a.sx = st.st[0];
    a.sy = st.st[1];
    a.sz = st.st[2];
