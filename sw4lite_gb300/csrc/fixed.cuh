@@ -118,44 +118,16 @@ __device__ __forceinline__ void rest(Num& d)
    d = Num{d.m << n, d.m == 0 ? kNone : d.e - n};
 }
 
-// The difference d1i(x) of values |x| < 2^57 aligned to the exponent e of the largest
-__device__ __forceinline__ Num difference(i64 x0, i64 x1, i64 x2, i64 x3, int e0, int e1, int e2, int e3, int e)
-{
-   return normal(((sar(x2, e - e2) - sar(x1, e - e1)) << 3) + (sar(x0, e - e0) - sar(x3, e - e3)), e);
-}
-
-// Three FP64 values as integers m[c] with value m[c] * 2^(e - 1079), |m[c]| < 2^57, e the
-// largest of their biased exponents (at least 1, the subnormals' exponent); bits below
-// 2^-57 of the largest are dropped toward zero.  True if one
-// is not finite; it counts as (less than) the smallest normal number.
-__device__ __forceinline__ bool to_block(double v0, double v1, double v2, i64 m[3], int& e)
-{
-   const double v[3] = {v0, v1, v2};
-   int hi[3], eb[3], any = 0;
-#pragma unroll
-   for (int c = 0; c < 3; c++) {
-      hi[c] = __double2hiint(v[c]);
-      eb[c] = (hi[c] >> 20) & 0x7ff;
-      any = max(any, eb[c]);
-      eb[c] = eb[c] == 2047 ? 0 : eb[c];
-   }
-   e = max(max(eb[0], eb[1]), max(eb[2], 1));
-#pragma unroll
-   for (int c = 0; c < 3; c++) {
-      const int lead = min(eb[c], 1) << 20;
-      const unsigned mh = (unsigned)(hi[c] & 0xfffff) | (unsigned)lead;
-      i64 t = (i64)(((unsigned long long)mh << 32) | (unsigned)__double2loint(v[c])) << 4;
-      t = sar(t, e - max(eb[c], 1));
-      const i64 s = (i64)(hi[c] >> 31);
-      m[c] = (t ^ s) - s;
-   }
-   return any == 2047;
-}
-
 // 8 (fp1 - fm1) + (fm2 - fp2)
 __device__ __forceinline__ i64 d1i(i64 fm2, i64 fm1, i64 fp1, i64 fp2)
 {
    return ((fp1 - fm1) << 3) + (fm2 - fp2);
+}
+
+// The difference d1i(x) of values |x| < 2^57 aligned to the exponent e of the largest
+__device__ __forceinline__ Num difference(i64 x0, i64 x1, i64 x2, i64 x3, int e0, int e1, int e2, int e3, int e)
+{
+   return normal(d1i(sar(x0, e - e0), sar(x1, e - e1), sar(x2, e - e2), sar(x3, e - e3)), e);
 }
 
 // x * C / 2^57 for |x| < 2^62 and a coefficient |C| < 2^57 held as c.x = C >> 26,
@@ -191,6 +163,46 @@ struct Scale {
       return neg ? -r : r;
    }
 };
+
+__device__ __forceinline__ bool is_one(double x) { return __double_as_longlong(x) == 0x3ff0000000000000LL; }
+
+// times a stretching factor
+__device__ __forceinline__ Num stretched(const Num& d, double s)
+{
+   const Scale f(s);
+   return Num{f(d.m), d.e + f.e};
+}
+
+// Products of one point for one outer direction of the mixed terms, value m * 2^(e - 1078):
+// la times the sum of the differences s0, s1 with stretching factors f0, f1, and mu times m0
+// and m1.  A coefficient is C * 2^(e - 57), its limbs as mulc takes them.
+struct Triple {
+   Num la, m0, m1;
+};
+
+__device__ __forceinline__ Num times(const Num& d, int2 c, int e) { return Num{mulc(d.m, c), d.e + e - 1}; }
+
+__device__ __forceinline__ Triple products(Num s0, Num s1, const Num& m0, const Num& m1, int2 mu, int emu, int2 la, int ela,
+                                           double f0, double f1)
+{
+   if (!is_one(f0)) s0 = stretched(s0, f0);
+   if (!is_one(f1)) s1 = stretched(s1, f1);
+   const int es = max(s0.e, s1.e);
+   Triple t;
+   t.la = Num{mulc(sar(s0.m, es - s0.e + 1) + sar(s1.m, es - s1.e + 1), la), es + ela};
+   t.m0 = times(m0, mu, emu);
+   t.m1 = times(m1, mu, emu);
+   return t;
+}
+
+// The outer difference of four products, e the largest of their exponents, value
+// m * 2^(e - 1074).  Equal products leave zero, which has no exponent: a component that they do
+// not reach keeps its own.
+__device__ __forceinline__ Num outer(i64 g0, i64 g1, i64 g2, i64 g3, int e0, int e1, int e2, int e3, int e)
+{
+   const i64 d = d1i(sar(g0, e - e0 + 4), sar(g1, e - e1 + 4), sar(g2, e - e2 + 4), sar(g3, e - e3 + 4));
+   return Num{d, d == 0 ? kNone : e};
+}
 
 // p * 2^e as FP64, rounded once; below the normal range 0, above it infinite.
 __device__ __forceinline__ double from_block(i64 p, int e)

@@ -7,13 +7,15 @@
 // a = c s of a coefficient (mu, 2 mu + lambda) and the stretching along each axis are
 // formed in FP64, aligned as integers like the field, and the weights of the second
 // differences are integer sums of five of them.  Stretching factors of the point itself
-// multiply finished sums and keep their own exponents: any finite profile is accepted.
+// multiply finished sums and keep their own exponents, as everything does that is not yet
+// added: any finite profile is accepted, and each component, coefficient and axis keeps its
+// digits beside others any power of two larger.
 //
-// What bounds it: the integer pipes, about 3500 instructions a warp of 32 points, and 20
-// FP64 operations a point, against 410 for one thread per point that forms every weight and
-// inner difference anew: 256 x 200 x 150 points 1.74 ms against 5.97 ms.  The error against
-// quad precision is 0.5 to 0.9 times that of the FP64 sums (smooth and random fields, profiles
-// random and falling to 1e-4).
+// What bounds it: the latency of twelve warps an SM and the integer pipes, about 5000
+// instructions a warp of 32 points, and 20 FP64 operations a point, against 410 for one thread
+// per point that forms every weight and inner difference anew: 256 x 200 x 150 points 2.18 ms
+// against 5.97 ms.  (One exponent for a point's components and coefficients: 1.74 ms, and the
+// smaller ones lost digits.)
 #include <algorithm>
 
 #include "common.cuh"
@@ -27,8 +29,6 @@ constexpr int TX = 32, TY = 6, HALO = 2;
 constexpr int PX = TX + 2 * HALO, PY = TY + 2 * HALO, PLANE = PX * PY;
 constexpr int NTHREADS = TX * TY;
 constexpr int NX = TY * PX, NY = PY * TX;
-constexpr int kNone = -20000;  // below any exponent, in 16 bits
-
 struct OpFixed {
    Box b;
    int k1, k2, kchunk;
@@ -50,40 +50,27 @@ struct Smem {
    i64 ax[2][NX];        // mu s_x, (2 mu + la) s_x of the plane along x,
    i64 ay[2][NY];        // ... s_y along y,
    i64 az[5][2][NTHREADS];  // ... s_z of the own column, ring of planes
-   int gxe[NX], gye[NY], gze[4][NTHREADS];  // exponents: la's product << 16 | mu's
-   short ve[5][PLANE], axe[NX], aye[NY], aze[5][NTHREADS];
+   unsigned ve[5][PLANE];   // exponents of the three components (pack)
+   short gxe[3][NX], gye[3][NY], gze[4][3][NTHREADS], axe[2][NX], aye[2][NY];
    int bad;
 };
 
-// Products of one point for one outer direction: la f0 s0 + la f1 s1, mu m0 and mu m1 (as in
-// stage_fixed.cu, the first with its own exponent).  c: mu and la as integers, ec their
-// exponent - 1022.
-struct Triple {
-   i64 la, m0, m1;
-   int el, em;
-};
+// Exponents of a point's three components in one word: 11 bits each for the first two, and the
+// third, whose integer is brought to an even one, halved.
+__device__ __forceinline__ unsigned pack(int e0, int e1, int e2) { return (unsigned)e2 << 21 | (unsigned)e1 << 11 | (unsigned)e0; }
+__device__ __forceinline__ int unpack(int c, unsigned e)
+{
+   return c == 0 ? (int)(e & 0x7ff) : c == 1 ? (int)(e >> 11 & 0x7ff) : (int)(e >> 22) << 1;
+}
 
 __device__ __forceinline__ int2 limbs(i64 c) { return make_int2((int)(c >> kSplit), (int)(c & kMask) << 5); }
 
-__device__ __forceinline__ Triple products(i64 s0, i64 s1, i64 m0, i64 m1, int es0, int es1, i64 mu, i64 la, int ec,
-                                           double f0, double f1)
+// The sum of two numbers, halved once so that sums of sums fit
+__device__ __forceinline__ Num add(const Num& a, const Num& b)
 {
-   const int es = max(es0, es1), d0 = es - es0 + 1, d1 = es - es1 + 1;
-   const int2 cm = limbs(mu);
-   Triple t;
-   t.m0 = mulc(sar(m0, d0), cm);
-   t.m1 = mulc(sar(m1, d1), cm);
-   t.em = es + ec;
-   const Scale a(f0), b(f1);
-   const int ea = es0 + a.e, eb = es1 + b.e, el = max(ea, eb);
-   t.la = mulc(sar(a(s0 >> 1), el - ea) + sar(b(s1 >> 1), el - eb), limbs(la));
-   t.el = el + ec;
-   return t;
+   const int e = max(a.e, b.e);
+   return Num{to_odd(a.m, e - a.e + 1) + to_odd(b.m, e - b.e + 1), e + 1};
 }
-
-__device__ __forceinline__ int pack(int el, int em) { return (int)((unsigned)max(el, kNone) << 16 | (unsigned)(max(em, kNone) & 0xffff)); }
-__device__ __forceinline__ int upper(int e) { return e >> 16; }
-__device__ __forceinline__ int lower(int e) { return (short)(e & 0xffff); }
 
 // The points of a column whose sums read a field or material value or a stretching factor
 // that is not finite, set to NaN after the march (see stage_fixed.cu: of the material a
@@ -155,25 +142,34 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
       for (int r = 0; r < kPre; r++) {
          const int idx = tid + r * NTHREADS;
          if (idx < PLANE) {
-            i64 m[3];
-            int e;
-            if (to_block(pv[r][0], pv[r][1], pv[r][2], m, e)) sm.bad = 1;
+            int e[3];
 #pragma unroll
-            for (int c = 0; c < 3; c++) sm.v[q][c][idx] = m[c];
-            sm.ve[q][idx] = (short)e;
+            for (int c = 0; c < 3; c++) {
+               i64 m;
+               if (to_fixed(pv[r][c], m, e[c])) sm.bad = 1;
+               if (c == 2) {
+                  m >>= e[2] & 1;
+                  e[2] += e[2] & 1;
+               }
+               sm.v[q][c][idx] = m;
+            }
+            sm.ve[q][idx] = pack(e[0], e[1], e[2]);
          }
       }
    };
    // c s of a point's two coefficients as integers
-   auto put = [&](double m, double l, double s, i64* a0, i64* a1, short* e) {
-      i64 t[3];
-      int x;
-      if (to_block(m * s, fma(2.0, m, l) * s, 0.0, t, x)) sm.bad = 1;
-      *a0 = t[0];
-      *a1 = t[1];
-      *e = (short)x;
+   auto put = [&](double m, double l, double s, i64* a0, i64* a1, int& e0, int& e1) {
+      const bool b0 = to_fixed(m * s, *a0, e0), b1 = to_fixed(fma(2.0, m, l) * s, *a1, e1);
+      if (b0 || b1) sm.bad = 1;
    };
-   // the own column's material two planes ahead (z weights)
+   auto put_xy = [&](double m, double l, double s, i64* a0, i64* a1, short* e0, short* e1) {
+      int x0, x1;
+      put(m, l, s, a0, a1, x0, x1);
+      *e0 = (short)x0;
+      *e1 = (short)x1;
+   };
+   // the own column's material two planes ahead (z weights), exponents (2 mu + la) << 16 | mu
+   int aze[5] = {0, 0, 0, 0, 0};  // of the planes k-2..k+2
    auto put_z = [&](int kk, int q) {
       double m = 0, l = 0;
       if (inside) {
@@ -181,10 +177,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
          m = __ldg(a.mu + p);
          l = __ldg(a.la + p);
       }
-      put(m, l, __ldg(a.sz + kk - b.kb), &sm.az[q][0][tid], &sm.az[q][1][tid], &sm.aze[q][tid]);
+      int e0, e1;
+      put(m, l, __ldg(a.sz + kk - b.kb), &sm.az[q][0][tid], &sm.az[q][1][tid], e0, e1);
+      return e1 << 16 | e0;
    };
 
    const double sxi = inside ? __ldg(a.sx + (i - b.ib)) : 0.0, syj = inside ? __ldg(a.sy + (j - b.jb)) : 0.0;
+
+   const bool stx = !is_one(sxi), sty = !is_one(syj);
 
    // the halo's products and x, y weights: rows -2, -1, TY, TY + 1 by the first four warps,
    // columns -2, -1, 32, 33 by the next 4 TY threads
@@ -202,14 +202,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
       }
    }
 
-   i64 pq[2][3];  // sums of planes k-2, k-1 and their exponents
-   int pe[2][3];
+   Num pq[2][3];  // sums of planes k-2, k-1, value m * 2^(e - 1072)
 #pragma unroll
-   for (int q = 0; q < 4; q++) sm.gze[q][tid] = pack(kNone, kNone), sm.gz[q][0][tid] = sm.gz[q][1][tid] = sm.gz[q][2][tid] = 0;
+   for (int c = 0; c < 3; c++) {
 #pragma unroll
-   for (int q = 0; q < 2; q++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) pe[q][c] = kNone, pq[q][c] = 0;
+      for (int q = 0; q < 4; q++) sm.gze[q][c][tid] = (short)kNone, sm.gz[q][c][tid] = 0;
+      pq[0][c] = pq[1][c] = Num{0, kNone};
+   }
 
    if (tid == 0) sm.bad = 0;
    __syncthreads();
@@ -217,265 +216,248 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
    int qm2 = 3, qm1 = 4, q0 = 0, qp1 = 1, qp2 = 2;
    fetch(kbeg - 2);
    store(q0);
-   put_z(kbeg - 2, q0);
+   aze[2] = put_z(kbeg - 2, q0);
    fetch(kbeg - 1);
    store(qp1);
-   put_z(kbeg - 1, qp1);
+   aze[3] = put_z(kbeg - 1, qp1);
    fetch(kbeg);
    for (int k = kbeg - 2; k <= kend + 2; k++) {
       const bool full = k >= kbeg && k <= kend;
       const long long plane = b.nij * (long long)(k - b.kb);
       // material of the plane, own point and halo
-      i64 cm[3];
-      int ec;
+      i64 cm[2];
+      int ec[2];
       {
          double m = 0, l = 0;
          if (inside) {
             m = __ldg(a.mu + plane + col);
             l = __ldg(a.la + plane + col);
          }
-         if (to_block(m, l, 0.0, cm, ec)) sm.bad = 1;
-         ec -= 1022;
+         const bool b0 = to_fixed(m, cm[0], ec[0]), b1 = to_fixed(l, cm[1], ec[1]);
+         if (b0 || b1) sm.bad = 1;
          if (full) {
             const int qx = ty * PX + tx + HALO, qy = (ty + HALO) * TX + tx;
-            put(m, l, sxi, &sm.ax[0][qx], &sm.ax[1][qx], &sm.axe[qx]);
-            put(m, l, syj, &sm.ay[0][qy], &sm.ay[1][qy], &sm.aye[qy]);
+            put_xy(m, l, sxi, &sm.ax[0][qx], &sm.ax[1][qx], &sm.axe[0][qx], &sm.axe[1][qx]);
+            put_xy(m, l, syj, &sm.ay[0][qy], &sm.ay[1][qy], &sm.aye[0][qy], &sm.aye[1][qy]);
          }
       }
-      i64 hm[3] = {0, 0, 0};
-      int he = 0;
+      i64 hm[2] = {0, 0};
+      int he[2] = {0, 0};
       if (full && halo) {
          double m = 0, l = 0;
          if (hcol >= 0) {
             m = __ldg(a.mu + plane + hcol);
             l = __ldg(a.la + plane + hcol);
          }
-         if (to_block(m, l, 0.0, hm, he)) sm.bad = 1;
-         he -= 1022;
+         const bool b0 = to_fixed(m, hm[0], he[0]), b1 = to_fixed(l, hm[1], he[1]);
+         if (b0 || b1) sm.bad = 1;
          if (yh) {
             const int q = hrow * TX + tx;
-            put(m, l, hst, &sm.ay[0][q], &sm.ay[1][q], &sm.aye[q]);
+            put_xy(m, l, hst, &sm.ay[0][q], &sm.ay[1][q], &sm.aye[0][q], &sm.aye[1][q]);
          } else {
             const int q = (hrow - HALO) * PX + hcl;
-            put(m, l, hst, &sm.ax[0][q], &sm.ax[1][q], &sm.axe[q]);
+            put_xy(m, l, hst, &sm.ax[0][q], &sm.ax[1][q], &sm.axe[0][q], &sm.axe[1][q]);
          }
       }
       if (k <= kend) {
          store(qp2);
-         put_z(k + 2, qp2);
+         aze[4] = put_z(k + 2, qp2);
       }
       __syncthreads();
       if (k < kend) fetch(k + 3);
       const double szk = __ldg(a.sz + (k - b.kb));
       const i64* v0 = &sm.v[q0][0][0];
-      const short* e0 = sm.ve[q0];
-      int ex[4], ey[4], ez[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-         const int s = m < 2 ? m - 2 : m - 1;
-         ex[m] = e0[own + s];
-         ey[m] = e0[own + s * PX];
-      }
-      const int Ex = max4(ex[0], ex[1], ex[2], ex[3]), Ey = max4(ey[0], ey[1], ey[2], ey[3]);
-      int Ez = 0;
-      i64 dx[3], dy[3], dz[3], S[3] = {0, 0, 0};
-      int eS = kNone;
+      const unsigned* e0 = sm.ve[q0];
       const int qz[4] = {qm2, qm1, qp1, qp2};
+      // differences of component c at the point s along an axis of the plane (stride o) or
+      // across the planes
+      auto along = [&](int c, int s, int o) {
+         const i64* v = v0 + c * PLANE + s;
+         const int x0 = unpack(c, e0[s - 2 * o]), x1 = unpack(c, e0[s - o]), x2 = unpack(c, e0[s + o]), x3 = unpack(c, e0[s + 2 * o]);
+         return difference(v[-2 * o], v[-o], v[o], v[2 * o], x0, x1, x2, x3, max4(x0, x1, x2, x3));
+      };
+      auto down = [&](int c, int s) {
+         const int x0 = unpack(c, sm.ve[qm2][s]), x1 = unpack(c, sm.ve[qm1][s]), x2 = unpack(c, sm.ve[qp1][s]), x3 = unpack(c, sm.ve[qp2][s]);
+         return difference(sm.v[qm2][c][s], sm.v[qm1][c][s], sm.v[qp1][c][s], sm.v[qp2][c][s], x0, x1, x2, x3, max4(x0, x1, x2, x3));
+      };
+
+      Num D[3][3];  // differences along x, y, z of the components
+      Num S[3] = {{0, kNone}, {0, kNone}, {0, kNone}};
       if (!full) {
-#pragma unroll
-         for (int c = 0; c < 3; c++) {
-            const i64* v = v0 + c * PLANE + own;
-            if (c != 1) dx[c] = d1i(sar(v[-2], Ex - ex[0]), sar(v[-1], Ex - ex[1]), sar(v[1], Ex - ex[2]), sar(v[2], Ex - ex[3]));
-            if (c != 0) dy[c] = d1i(sar(v[-2 * PX], Ey - ey[0]), sar(v[-PX], Ey - ey[1]), sar(v[PX], Ey - ey[2]), sar(v[2 * PX], Ey - ey[3]));
-         }
+         D[0][0] = along(0, own, 1);
+         D[0][2] = along(2, own, 1);
+         D[1][1] = along(1, own, PX);
+         D[1][2] = along(2, own, PX);
+         rest(D[0][0]), rest(D[0][2]), rest(D[1][1]), rest(D[1][2]);
       } else {
-#pragma unroll
-         for (int m = 0; m < 4; m++) ez[m] = sm.ve[qz[m]][own];
-         Ez = max4(ez[0], ez[1], ez[2], ez[3]);
-         const int eo = e0[own], E = max(max(Ex, Ey), max(Ez, eo));
-         i64 x0[3];
-#pragma unroll
-         for (int c = 0; c < 3; c++) x0[c] = sar(v0[c * PLANE + own], E - eo);
+         const int qx = ty * PX + tx, qy = ty * TX + tx;
 #pragma unroll
          for (int ax = 0; ax < 3; ax++) {
-            // weights: 4 a(q-1) - 3 (a(q) + a(q-2)) and 4 (a(q-2) + a(q+1)) + 12 (a(q) + a(q-1)) and
-            // their mirrors, below 2^62, kept to 2^-5 and split at bit 30, so that an axis'
-            // sums of products fit.  The centre's is minus the sum of the limbs.
-            int ae[5];
-            i64 av[2][5];
-            const int qx = ty * PX + tx, qy = ty * TX + tx;
+            unsigned en[4];  // exponents of the four neighbours
 #pragma unroll
-            for (int m = 0; m < 5; m++) {
-               const int zq = m == 0 ? qm2 : m == 1 ? qm1 : m == 2 ? q0 : m == 3 ? qp1 : qp2;
-               ae[m] = ax == 0 ? sm.axe[qx + m] : ax == 1 ? sm.aye[qy + m * TX] : sm.aze[zq][tid];
-#pragma unroll
-               for (int t = 0; t < 2; t++) av[t][m] = ax == 0 ? sm.ax[t][qx + m] : ax == 1 ? sm.ay[t][qy + m * TX] : sm.az[zq][t][tid];
+            for (int m = 0; m < 4; m++) {
+               const int s = m < 2 ? m - 2 : m - 1;
+               en[m] = ax == 0 ? e0[own + s] : ax == 1 ? e0[own + s * PX] : sm.ve[qz[m]][own];
             }
-            const int ea = max(max4(ae[0], ae[1], ae[2], ae[3]), ae[4]);
-            int2 w[2][4];
-            int ch[2], cl[2];
+            const double f = ax == 0 ? sxi : ax == 1 ? syj : szk;
 #pragma unroll
             for (int t = 0; t < 2; t++) {
+               // weights: 4 a(q-1) - 3 (a(q) + a(q-2)) and 4 (a(q-2) + a(q+1)) + 12 (a(q) + a(q-1)) and
+               // their mirrors, four times the operator's, below 2^62, kept to 2^-5 and split at bit
+               // 30; each with the exponent of the largest a that it reads
                i64 A[5];
-#pragma unroll
-               for (int m = 0; m < 5; m++) A[m] = sar(av[t][m], ea - ae[m]);
-               const i64 o0 = A[2] + A[0], o1 = A[2] + A[4], i0s = A[2] + A[1], i1s = A[3] + A[2];
-               const i64 W[4] = {(A[1] << 2) - (o0 + (o0 << 1)), (A[0] + A[3] + i0s + (i0s << 1)) << 2,
-                                 (A[1] + A[4] + i1s + (i1s << 1)) << 2, (A[3] << 2) - (o1 + (o1 << 1))};
-               i64 lows = 0;
-               ch[t] = 0;
-#pragma unroll
-               for (int m = 0; m < 4; m++) {
-                  const i64 r = (W[m] + 16) >> 5, h = (r + (1 << 29)) >> 30;
-                  w[t][m] = make_int2((int)h, (int)(r - (h << 30)));
-                  ch[t] -= w[t][m].x;
-                  lows -= w[t][m].y;
-               }
-               const i64 h = (lows + (1 << 29)) >> 30;
-               ch[t] += (int)h;
-               cl[t] = (int)(lows - (h << 30));
-            }
-            const int Ea = ax == 0 ? Ex : ax == 1 ? Ey : Ez;
-            i64 hh[3], xw[3], wx[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-               i64 x[4];
-#pragma unroll
-               for (int m = 0; m < 4; m++) {
-                  const int o = m < 2 ? m - 2 : m - 1;
-                  x[m] = ax == 0 ? v0[c * PLANE + own + o] : ax == 1 ? v0[c * PLANE + own + o * PX] : sm.v[qz[m]][c][own];
-               }
-               const int* e = ax == 0 ? ex : ax == 1 ? ey : ez;
-               const i64 d = d1i(sar(x[0], Ea - e[0]), sar(x[1], Ea - e[1]), sar(x[2], Ea - e[2]), sar(x[3], Ea - e[3]));
-               if (ax == 0) dx[c] = d;
-               if (ax == 1) dy[c] = d;
-               if (ax == 2) dz[c] = d;
-               const int t = ax == c ? 1 : 0;
-               hh[c] = xw[c] = wx[c] = 0;
+               int ae[5];
 #pragma unroll
                for (int m = 0; m < 5; m++) {
-                  const i64 y = m < 4 ? sar(x[m], E - e[m]) : x0[c];
-                  const int wh = m < 4 ? w[t][m].x : ch[t], wl = m < 4 ? w[t][m].y : cl[t];
-                  const int xh = (int)(y >> kSplit), xl = (int)y & kMask;
-                  hh[c] = madw(xh, wh, hh[c]);
-                  xw[c] = madw(xh, wl, xw[c]);
-                  wx[c] = madw(xl, wh, wx[c]);
+                  const int zq = m == 0 ? qm2 : m == 1 ? qm1 : m == 2 ? q0 : m == 3 ? qp1 : qp2;
+                  ae[m] = ax == 0 ? sm.axe[t][qx + m] : ax == 1 ? sm.aye[t][qy + m * TX] : t == 1 ? aze[m] >> 16 : aze[m] & 0xffff;
+                  A[m] = ax == 0 ? sm.ax[t][qx + m] : ax == 1 ? sm.ay[t][qy + m * TX] : sm.az[zq][t][tid];
+               }
+               int2 w[4];
+               int we[4];
+#pragma unroll
+               for (int m = 0; m < 4; m++) {
+                  const int far = m == 0 ? 0 : 4;
+                  i64 W;
+                  if (m == 0 || m == 3) {
+                     const int e = max(max(ae[2], ae[far]), ae[m == 0 ? 1 : 3]);
+                     const i64 o = sar(A[2], e - ae[2]) + sar(A[far], e - ae[far]);
+                     W = (sar(A[m == 0 ? 1 : 3], e - ae[m == 0 ? 1 : 3]) << 2) - (o + (o << 1));
+                     we[m] = e;
+                  } else {
+                     const int q = m - 1;  // a(q), a(q + 3) with weight 1, the two between with 3
+                     const int e = max4(ae[q], ae[q + 1], ae[q + 2], ae[q + 3]);
+                     const i64 i = sar(A[q + 1], e - ae[q + 1]) + sar(A[q + 2], e - ae[q + 2]);
+                     W = (sar(A[q], e - ae[q]) + sar(A[q + 3], e - ae[q + 3]) + i + (i << 1)) << 2;
+                     we[m] = e;
+                  }
+                  const i64 r = (W + 16) >> 5, h = (r + (1 << 29)) >> 30;
+                  w[m] = make_int2((int)h, (int)(r - (h << 30)));
+               }
+#pragma unroll
+               for (int c = 0; c < 3; c++) {
+                  if ((ax == c) != (t == 1)) continue;
+                  int e[4];
+#pragma unroll
+                  for (int m = 0; m < 4; m++) e[m] = unpack(c, en[m]);
+                  const int E = max4(e[0], e[1], e[2], e[3]), eo = unpack(c, e0[own]), Ec = max(E, eo);
+                  i64 x[4];
+#pragma unroll
+                  for (int m = 0; m < 4; m++) {
+                     const int s = m < 2 ? m - 2 : m - 1;
+                     x[m] = sar(ax == 0 ? v0[c * PLANE + own + s] : ax == 1 ? v0[c * PLANE + own + s * PX] : sm.v[qz[m]][c][own], E - e[m]);
+                  }
+                  D[ax][c] = normal(d1i(x[0], x[1], x[2], x[3]), E);
+                  // differences to the own value, aligned by the size of their products with the weights,
+                  // the largest brought to bit 57
+                  const i64 x0 = sar(v0[c * PLANE + own], Ec - eo);
+                  int pe[4];
+                  bool tiny = false;
+#pragma unroll
+                  for (int m = 0; m < 4; m++) {
+                     const i64 d = sar(x[m], Ec - E) - x0;
+                     const int n = headroom<57>(d);
+                     x[m] = d << n;
+                     pe[m] = we[m] - n;
+                     tiny = tiny || (unsigned)((int)(d >> 32) + 1) < 2u;  // its upper word is sign
+                  }
+                  if (tiny)
+#pragma unroll
+                     for (int m = 0; m < 4; m++) {
+                        const int n = max(__clzll(x[m] ^ (x[m] >> 63)) - 6, 0);
+                        pe[m] = x[m] == 0 ? kNone : pe[m] - n;
+                        x[m] <<= n;
+                     }
+                  const int ep = max4(pe[0], pe[1], pe[2], pe[3]);
+                  i64 hh = 0, xw = 0, wx = 0;
+#pragma unroll
+                  for (int m = 0; m < 4; m++) {
+                     const i64 y = sar(x[m], ep - pe[m]);
+                     const int xh = (int)(y >> 27), xl = (int)y & ((1 << 27) - 1);
+                     hh = madw(xh, w[m].x, hh);
+                     xw = madw(xh, w[m].y, xw);
+                     wx = madw(xl, w[m].x, wx);
+                  }
+                  // the sum of a smooth field is a small part of its terms: with as many of the
+                  // lower bits as there is room for
+                  const int up = min(headroom<60>(hh), 27);  // |s| < 2^62, as Scale takes it
+                  const i64 s = (hh << up) + to_odd((xw >> 3) + wx, 27 - up);
+                  // times the point's own factor
+                  Num T = {s, s == 0 ? kNone : Ec + ep - up};
+                  if (!is_one(f)) T = stretched(T, f);
+                  S[c] = ax == 0 ? T : add(S[c], T);
                }
             }
-            // the sum of a smooth field is a small part of its terms: shifted up to keep
-            // its low bits
-            auto top = [](i64 x) { return (unsigned)((int)(x >> 32) ^ (int)(x >> 63)); };
-            const int up = min(max(__clz((int)(top(hh[0]) | top(hh[1]) | top(hh[2]))) - 3, 0), 24);
-            i64 s[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) s[c] = (hh[c] << up) + sar(xw[c], 30 - up) + sar(wx[c], kSplit - up);
-            // times the point's own factor; running sums to the larger exponent
-            const Scale f(ax == 0 ? sxi : ax == 1 ? syj : szk);
-            const int es = E + ea + f.e - up;
-            if (ax == 0) {
-               eS = es;
-#pragma unroll
-               for (int c = 0; c < 3; c++) S[c] = f(s[c]);
-            } else {
-               const int en = max(eS, es);
-               const Round down(en - eS), add(en - es);
-#pragma unroll
-               for (int c = 0; c < 3; c++) S[c] = down(S[c]) + add(f(s[c]));
-               eS = en;
-            }
          }
-         eS -= 1021;
+#pragma unroll
+         for (int c = 0; c < 3; c++) S[c].e = max(S[c].e - 1020, kNone);
       }
 
-      // products of the own point
-      const Triple z = products(dx[0], dy[1], dx[2], dy[2], Ex, Ey, cm[0], cm[1], ec, sxi, syj);
       if (full) {
-         Triple t = products(dy[1], dz[2], dy[0], dz[0], Ey, Ez, cm[0], cm[1], ec, syj, szk);
-         const int qx = ty * PX + tx + HALO;
-         sm.gx[0][qx] = t.la;
-         sm.gx[1][qx] = t.m0;
-         sm.gx[2][qx] = t.m1;
-         sm.gxe[qx] = pack(t.el, t.em);
-         t = products(dx[0], dz[2], dx[1], dz[1], Ex, Ez, cm[0], cm[1], ec, sxi, szk);
-         const int qy = (ty + HALO) * TX + tx;
-         sm.gy[0][qy] = t.m0;
-         sm.gy[1][qy] = t.la;
-         sm.gy[2][qy] = t.m1;
-         sm.gye[qy] = pack(t.el, t.em);
+         bool any = false;
+#pragma unroll
+         for (int ax = 0; ax < 3; ax++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) any = any || small(D[ax][c]);
+         if (any)
+#pragma unroll
+            for (int ax = 0; ax < 3; ax++)
+#pragma unroll
+               for (int c = 0; c < 3; c++) rest(D[ax][c]);
+      }
+      // products of the own point
+      const int2 lm = limbs(cm[0]), ll = limbs(cm[1]);
+      const int emu = ec[0] - 1022, ela = ec[1] - 1022;
+      const Triple z = products(D[0][0], D[1][1], D[0][2], D[1][2], lm, emu, ll, ela, sxi, syj);
+      if (full) {
+         auto to_x = [&](const Triple& t, int q) {
+            sm.gx[0][q] = t.la.m;
+            sm.gx[1][q] = t.m0.m;
+            sm.gx[2][q] = t.m1.m;
+            sm.gxe[0][q] = (short)max(t.la.e, kNone);
+            sm.gxe[1][q] = (short)max(t.m0.e, kNone);
+            sm.gxe[2][q] = (short)max(t.m1.e, kNone);
+         };
+         auto to_y = [&](const Triple& t, int q) {
+            sm.gy[0][q] = t.m0.m;
+            sm.gy[1][q] = t.la.m;
+            sm.gy[2][q] = t.m1.m;
+            sm.gye[0][q] = (short)max(t.m0.e, kNone);
+            sm.gye[1][q] = (short)max(t.la.e, kNone);
+            sm.gye[2][q] = (short)max(t.m1.e, kNone);
+         };
+         to_x(products(D[1][1], D[2][2], D[1][0], D[2][0], lm, emu, ll, ela, syj, szk), ty * PX + tx + HALO);
+         to_y(products(D[0][0], D[2][2], D[0][1], D[2][1], lm, emu, ll, ela, sxi, szk), (ty + HALO) * TX + tx);
          if (halo) {
-            const int s = hrow * PX + hcl, o = yh ? 1 : PX;
-            int eh[4], ezh[4];
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-               eh[m] = e0[s + (m < 2 ? m - 2 : m - 1) * o];
-               ezh[m] = sm.ve[qz[m]][s];
-            }
-            const int Eh = max4(eh[0], eh[1], eh[2], eh[3]), Ezh = max4(ezh[0], ezh[1], ezh[2], ezh[3]);
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-               eh[m] = Eh - eh[m];
-               ezh[m] = Ezh - ezh[m];
-            }
-            const int cs = (yh ? 0 : PLANE) + s, cc = (yh ? PLANE : 0) + s;
-            auto along = [&](int q) { return d1i(sar(v0[q - 2 * o], eh[0]), sar(v0[q - o], eh[1]), sar(v0[q + o], eh[2]), sar(v0[q + 2 * o], eh[3])); };
-            auto down = [&](int q) {
-               return d1i(sar(sm.v[qm2][0][q], ezh[0]), sar(sm.v[qm1][0][q], ezh[1]), sar(sm.v[qp1][0][q], ezh[2]), sar(sm.v[qp2][0][q], ezh[3]));
-            };
-            t = products(along(cs), down(2 * PLANE + s), along(cc), down(cc), Eh, Ezh, hm[0], hm[1], he, hin, szk);
-            if (yh) {
-               const int q = hrow * TX + tx;
-               sm.gy[0][q] = t.m0;
-               sm.gy[1][q] = t.la;
-               sm.gy[2][q] = t.m1;
-               sm.gye[q] = pack(t.el, t.em);
-            } else {
-               const int q = (hrow - HALO) * PX + hcl;
-               sm.gx[0][q] = t.la;
-               sm.gx[1][q] = t.m0;
-               sm.gx[2][q] = t.m1;
-               sm.gxe[q] = pack(t.el, t.em);
-            }
+            const int s = hrow * PX + hcl, o = yh ? 1 : PX, cs = yh ? 0 : 1, cc = 1 - cs;
+            Num d0 = along(cs, s, o), d1 = down(2, s), d2 = along(cc, s, o), d3 = down(cc, s);
+            if (small(d0) || small(d1) || small(d2) || small(d3)) rest(d0), rest(d1), rest(d2), rest(d3);
+            const Triple t = products(d0, d1, d2, d3, limbs(hm[0]), he[0] - 1022, limbs(hm[1]), he[1] - 1022, hin, szk);
+            if (yh) to_y(t, hrow * TX + tx);
+            else to_x(t, (hrow - HALO) * PX + hcl);
          }
       }
       __syncthreads();
 
       // plane k: second differences and the x and y outer differences
-      i64 P[3] = {0, 0, 0};
-      int eP[3] = {kNone, kNone, kNone};
+      Num P[3] = {{0, kNone}, {0, kNone}, {0, kNone}};
       if (full) {
-         const i64* gx = &sm.gx[0][ty * PX + tx];
-         const i64* gy = &sm.gy[0][ty * TX + tx];
-         int hx[2][4], hy[2][4], Gx[2], Gy[2];  // mu's products, la's
-#pragma unroll
-         for (int m = 0; m < 4; m++) {
-            const int n = m < 2 ? m : m + 1, x = sm.gxe[ty * PX + tx + n], y = sm.gye[(ty + n) * TX + tx];
-            hx[0][m] = lower(x);
-            hx[1][m] = upper(x);
-            hy[0][m] = lower(y);
-            hy[1][m] = upper(y);
-         }
-#pragma unroll
-         for (int q = 0; q < 2; q++) {
-            Gx[q] = max4(hx[q][0], hx[q][1], hx[q][2], hx[q][3]);
-            Gy[q] = max4(hy[q][0], hy[q][1], hy[q][2], hy[q][3]);
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-               hx[q][m] = Gx[q] - hx[q][m] + 3;
-               hy[q][m] = Gy[q] - hy[q][m] + 3;
-            }
-         }
 #pragma unroll
          for (int c = 0; c < 3; c++) {
-            const i64* x = gx + c * NX;
-            const i64* y = gy + c * NY;
-            const int lx = c == 0, ly = c == 1;
-            const Scale fx(c == 0 ? sxi : c == 1 ? sxi * syj : sxi * szk), fy(c == 0 ? syj * sxi : c == 1 ? syj : syj * szk);
-            const i64 cx = fx(d1i(sar(x[0], hx[lx][0]), sar(x[1], hx[lx][1]), sar(x[3], hx[lx][2]), sar(x[4], hx[lx][3])) >> 1);
-            const i64 cy = fy(d1i(sar(y[0], hy[ly][0]), sar(y[TX], hy[ly][1]), sar(y[3 * TX], hy[ly][2]), sar(y[4 * TX], hy[ly][3])) >> 1);
-            const int tx_ = Gx[lx] + fx.e, ty_ = Gy[ly] + fy.e;
-            eP[c] = max(eS, max(tx_, ty_));
-            const i64 s8 = Round(eP[c] - eS + 3)(S[c]);  // second differences carry 1/6, mixed terms 1/144
-            P[c] = s8 + (s8 << 1) + Round(eP[c] - tx_ + 2)(cx) + Round(eP[c] - ty_ + 2)(cy);
+            const i64* x = &sm.gx[c][ty * PX + tx];
+            const i64* y = &sm.gy[c][ty * TX + tx];
+            const short* xe = &sm.gxe[c][ty * PX + tx];
+            const short* ye = &sm.gye[c][ty * TX + tx];
+            const int hx[4] = {xe[0], xe[1], xe[3], xe[4]}, hy[4] = {ye[0], ye[TX], ye[3 * TX], ye[4 * TX]};
+            Num cx = outer(x[0], x[1], x[3], x[4], hx[0], hx[1], hx[2], hx[3], max4(hx[0], hx[1], hx[2], hx[3]));
+            Num cy = outer(y[0], y[TX], y[3 * TX], y[4 * TX], hy[0], hy[1], hy[2], hy[3], max4(hy[0], hy[1], hy[2], hy[3]));
+            if (stx || sty || !is_one(szk)) {
+               cx = stretched(cx, c == 0 ? sxi : c == 1 ? sxi * syj : sxi * szk);
+               cy = stretched(cy, c == 0 ? syj * sxi : c == 1 ? syj : syj * szk);
+            }
+            P[c].e = max(S[c].e, max(cx.e, cy.e));
+            const i64 s8 = to_odd(S[c].m, P[c].e - S[c].e + 3);  // second differences carry 1/6, mixed terms 1/144
+            P[c].m = s8 + (s8 << 1) + to_odd(cx.m, P[c].e - cx.e + 2) + to_odd(cy.m, P[c].e - cy.e + 2);
          }
       }
 
@@ -483,34 +465,28 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
       const int kp = k - 2;
       if (kp >= kbeg && active) {
          const int z0 = k & 3, z1 = (k + 1) & 3, z3 = (k + 3) & 3;  // planes k-4, k-3, k-1
-         const int g0 = sm.gze[z0][tid], g1 = sm.gze[z1][tid], g3 = sm.gze[z3][tid];
          const double szp = __ldg(a.sz + (kp - b.kb));
-         const i64 zn[3] = {z.m0, z.m1, z.la};
+         const Num zn[3] = {z.m0, z.m1, z.la};
          const long long pp = col + b.nij * (long long)(kp - b.kb);
 #pragma unroll
          for (int c = 0; c < 3; c++) {
-            const bool l = c == 2;
-            const int h0 = l ? upper(g0) : lower(g0), h1 = l ? upper(g1) : lower(g1), h3 = l ? upper(g3) : lower(g3),
-                      h4 = l ? z.el : z.em;
-            const int Eg = max4(h0, h1, h3, h4);
-            const Scale f(c == 0 ? szp * sxi : c == 1 ? szp * syj : szp);
-            const i64 cz = f(d1i(sar(sm.gz[z0][c][tid], Eg - h0 + 3), sar(sm.gz[z1][c][tid], Eg - h1 + 3),
-                                 sar(sm.gz[z3][c][tid], Eg - h3 + 3), sar(zn[c], Eg - h4 + 3)) >> 1);
-            const int tz = Eg + f.e, eF = max(pe[0][c], tz);
-            a.lu[c * b.cs + b.ps * pp] = a.cof * from_block(Round(eF - pe[0][c])(pq[0][c]) + Round(eF - tz + 2)(cz), eF - 1072);
+            const int h0 = sm.gze[z0][c][tid], h1 = sm.gze[z1][c][tid], h3 = sm.gze[z3][c][tid], h4 = zn[c].e;
+            Num g = outer(sm.gz[z0][c][tid], sm.gz[z1][c][tid], sm.gz[z3][c][tid], zn[c].m, h0, h1, h3, h4, max4(h0, h1, h3, h4));
+            if (stx || sty || !is_one(szp)) g = stretched(g, c == 0 ? szp * sxi : c == 1 ? szp * syj : szp);
+            const int eF = max(pq[0][c].e, g.e);
+            a.lu[c * b.cs + b.ps * pp] = a.cof * from_block(to_odd(pq[0][c].m, eF - pq[0][c].e) + to_odd(g.m, eF - g.e + 2), eF - 1072);
          }
       }
-      sm.gz[k & 3][0][tid] = z.m0;
-      sm.gz[k & 3][1][tid] = z.m1;
-      sm.gz[k & 3][2][tid] = z.la;
-      sm.gze[k & 3][tid] = pack(z.el, z.em);
+      const Num zn[3] = {z.m0, z.m1, z.la};
 #pragma unroll
       for (int c = 0; c < 3; c++) {
+         sm.gz[k & 3][c][tid] = zn[c].m;
+         sm.gze[k & 3][c][tid] = (short)max(zn[c].e, kNone);
          pq[0][c] = pq[1][c];
          pq[1][c] = P[c];
-         pe[0][c] = pe[1][c];
-         pe[1][c] = eP[c];
       }
+#pragma unroll
+      for (int q = 0; q < 4; q++) aze[q] = aze[q + 1];
       const int next = qm2;
       qm2 = qm1;
       qm1 = q0;

@@ -95,48 +95,6 @@ struct Smem {
    int bad;                    // a value of the stage field or of the material is not finite
 };
 
-__device__ __forceinline__ bool is_one(double x) { return __double_as_longlong(x) == 0x3ff0000000000000LL; }
-
-// times a stretching factor
-__device__ __forceinline__ Num stretched(const Num& d, double s)
-{
-   const Scale f(s);
-   return Num{f(d.m), d.e + f.e};
-}
-
-// Products of one point for one outer direction, value m * 2^(e - 1078): la times the sum of
-// the differences s0, s1 with stretching factors f0, f1, and mu times m0 and m1.  c, ec:
-// limbs and exponents of mu and lambda.
-struct Triple {
-   Num la, m0, m1;
-};
-
-__device__ __forceinline__ Num times(const Num& d, int x, int y, int ec)
-{
-   return Num{mulc(d.m, make_int2(x, y)), d.e + ec - 1};
-}
-
-__device__ __forceinline__ Triple products(Num s0, Num s1, const Num& m0, const Num& m1, int4 c, int ec, double f0, double f1)
-{
-   if (!is_one(f0)) s0 = stretched(s0, f0);
-   if (!is_one(f1)) s1 = stretched(s1, f1);
-   const int es = max(s0.e, s1.e), emu = (int)(short)(ec & 0xffff);
-   Triple t;
-   t.la = Num{mulc(sar(s0.m, es - s0.e + 1) + sar(s1.m, es - s1.e + 1), make_int2(c.z, c.w)), es + (ec >> 16)};
-   t.m0 = times(m0, c.x, c.y, emu);
-   t.m1 = times(m1, c.x, c.y, emu);
-   return t;
-}
-
-// The outer difference of four products, e the largest of their exponents, value
-// m * 2^(e - 1074).  Equal products leave zero, which has no exponent: a component that they do
-// not reach keeps its own.
-__device__ __forceinline__ Num outer(i64 g0, i64 g1, i64 g2, i64 g3, int e0, int e1, int e2, int e3, int e)
-{
-   const i64 d = d1i(sar(g0, e - e0 + 4), sar(g1, e - e1 + 4), sar(g2, e - e2 + 4), sar(g3, e - e3 + 4));
-   return Num{d, d == 0 ? kNone : e};
-}
-
 __device__ __forceinline__ void copy16(void* dst, const void* src)
 {
    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
@@ -428,7 +386,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
 
       // Products of the own point
       const bool stz = !is_one(szk);
-      const Triple z = products(D[0][0], D[1][1], D[0][2], D[1][2], cc, ee, sxi, syj);
+      const int2 cm = make_int2(cc.x, cc.y), cl = make_int2(cc.z, cc.w);
+      const int emu = (int)(short)(ee & 0xffff), el = ee >> 16;
+      const Triple z = products(D[0][0], D[1][1], D[0][2], D[1][2], cm, emu, cl, el, sxi, syj);
       if (full) {
          auto to_x = [&](const Triple& t, int q) {
             sm.gx[0][q] = t.la.m;
@@ -446,8 +406,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
             sm.gye[1][q] = (short)t.la.e;
             sm.gye[2][q] = (short)t.m1.e;
          };
-         to_x(products(D[1][1], D[2][2], D[1][0], D[2][0], cc, ee, syj, szk), ty * PX + tx + HALO);
-         to_y(products(D[0][0], D[2][2], D[0][1], D[2][1], cc, ee, sxi, szk), (ty + HALO) * TX + tx);
+         to_x(products(D[1][1], D[2][2], D[1][0], D[2][0], cm, emu, cl, el, syj, szk), ty * PX + tx + HALO);
+         to_y(products(D[0][0], D[2][2], D[0][1], D[2][1], cm, emu, cl, el, sxi, szk), (ty + HALO) * TX + tx);
          if (halo) {
             // y outer: mu v_x, la (u_x + w_z), mu v_z;  x outer: la (v_y + w_z), mu u_y, mu u_z
             const int s = hrow * PX + hcl, o = yh ? 1 : PX, cs = yh ? 0 : 1, cm = 1 - cs;
@@ -457,7 +417,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
             }
             Num d0 = along(cs, s, o), d1 = down(2, s), d2 = along(cm, s, o), d3 = down(cm, s);
             if (small(d0) || small(d1) || small(d2) || small(d3)) rest(d0), rest(d1), rest(d2), rest(d3);
-            const Triple t = products(d0, d1, d2, d3, hc, he, hst, szk);
+            const Triple t = products(d0, d1, d2, d3, make_int2(hc.x, hc.y), (int)(short)(he & 0xffff), make_int2(hc.z, hc.w), he >> 16, hst, szk);
             if (yh) to_y(t, hrow * TX + tx);
             else to_x(t, (hrow - HALO) * PX + hcl);
          }

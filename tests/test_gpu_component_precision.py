@@ -7,7 +7,9 @@ sum, six on the way from L(u) to it, and in L(u) a weight of five roundings, or 
 coefficient of three, and a sum of 24 products: 2^-53 (3 (2|u| + |um|) + 16 dt^2/rho T) with
 T the magnitudes that tests/wide.py sums.  Of fields that depend on one coordinate only, in
 material that does not vary, the components are not coupled (the outer differences of equal
-products are zero in any arithmetic): T is then that of the component by itself.
+products are zero in any arithmetic): T is then that of the component by itself.  The
+kernel-level operator is held to 2^-53 16 T with the second differences' magnitudes taken of
+the differences of the values, which FP64 forms almost exactly.
 """
 import ctypes as C
 
@@ -114,6 +116,20 @@ def test_components_far_apart_coupled(sides, scale):
     _check(_material(rng), u, um, sides, coupled=True)
 
 
+def _largest(rng, shape):
+    return rng.choice([-1.0, 1.0], shape) * (2 - 2.0 ** -52)
+
+
+@pytest.mark.parametrize("sides", [1, 2])
+def test_largest_significands(sides):
+    """Values of one magnitude with all bits set and signs at random: the largest integers that
+    the sums meet."""
+    rng = np.random.default_rng(sides)
+    shape = (3,) + _grid_arrays()[0].shape
+    mat = [np.full(shape[1:], 1.0), np.full(shape[1:], 2 - 2.0 ** -52), np.full(shape[1:], 4 - 2.0 ** -51)]
+    _check(mat, _largest(rng, shape), _largest(rng, shape), sides, coupled=True)
+
+
 @pytest.mark.parametrize("axis", [0, 1, 2])
 @pytest.mark.parametrize("n", [15, 30, 45])
 def test_constant_displacement_with_a_small_part(axis, n):
@@ -138,3 +154,87 @@ def test_soft_and_stiff_coefficients(sides, ratio):
     _check(_material(rng, ratio, varying=False), u, 0.8 * u, sides, coupled=False)
     u = np.stack([np.sin(0.4 * x + 0.3 * y - 0.2 * z + c) for c in range(3)])
     _check(_material(rng, ratio), u, 0.8 * u, sides, coupled=True)
+
+
+def _check_operator(u, mu, la, st, coupled, soa):
+    val, terms = wide.operator(u, mu, la, st, H, differences=True)
+    if not coupled:
+        for c in range(3):
+            alone = np.zeros_like(u)
+            alone[c] = u[c]
+            terms[c] = wide.operator(alone, mu, la, st, H, differences=True)[1][c]
+    nx, ny, nz = SHAPE
+    b = (-1, nx + 2, -1, ny + 2, -1, nz + 2)
+    lay = np.moveaxis(u, 0, 3) if not soa else u
+    d = [dev(np.ascontiguousarray(a).ravel()) for a in (lay, mu, la, *st)]
+    lu = dev(np.zeros(u.size))
+    sg.check(sg.lib().sw4g_rhs4sg(soa, *b, nz, (C.c_int * 6)(), lu.data_ptr(), *[t.data_ptr() for t in d[:3]], H,
+                                  *[t.data_ptr() for t in d[3:]], None))
+    got = host(lu).reshape(u.shape) if soa else np.moveaxis(host(lu).reshape(*u.shape[1:], 3), 3, 0)
+    sel = (slice(None), slice(2, -2), slice(2, -2), slice(2, -2))
+    bar = 16 * wide.L(2) ** -53 * terms[sel]
+    err = abs(got[sel] - val[sel])
+    with np.errstate(all="ignore"):
+        assert np.all(err <= bar), float(np.nanmax(np.where(bar > 0, err / bar, np.inf * err)))
+
+
+def _profiles(kind, rng):
+    st = []
+    for n in SHAPE:
+        s = np.ones(n + 4)
+        if kind == "layers":
+            s = np.maximum(1e-4, 1 - np.abs(np.linspace(-1, 1, n + 4)) ** 3)
+        if kind == "any":
+            s = rng.choice([-1.0, 1.0], n + 4) * np.ldexp(1 + rng.random(n + 4), rng.integers(-30, 30, n + 4))
+            s[::9] = 0
+        st.append(s)
+    return st
+
+
+@pytest.mark.parametrize("soa", [1, 0])
+@pytest.mark.parametrize("profile", ["ones", "layers"])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("n", [10, 40, 300])
+def test_operator_components_far_apart_in_plane_waves(soa, profile, axis, n):
+    rng = np.random.default_rng(n + axis)
+    x = _grid_arrays()[axis]
+    u = np.stack([2.0 ** -(n * ((c - axis) % 3)) * np.sin(0.4 * x + rng.uniform(0, 6)) for c in range(3)])
+    st = _profiles(profile, rng)
+    if profile == "layers":  # equal products need equal factors along the other axes
+        st = [s if a == axis else np.ones_like(s) for a, s in enumerate(st)]
+    _, mu, la = _material(rng, varying=False)
+    _check_operator(u, mu, la, st, False, soa)
+
+
+@pytest.mark.parametrize("profile", ["ones", "layers", "any"])
+@pytest.mark.parametrize("scale", [(0, 0, 0), (0, 20, 40), (500, 700, 0)])
+@pytest.mark.parametrize("ratio", [2.0, 1e3, 1e-9])
+def test_operator_coupled(profile, scale, ratio):
+    rng = np.random.default_rng(sum(scale))
+    x, y, z = _grid_arrays()
+    u = np.stack([2.0 ** -scale[c] * np.sin(0.4 * x + rng.uniform(0, 6)) * np.cos(0.3 * y + rng.uniform(0, 6)) *
+                  np.cos(0.5 * z + rng.uniform(0, 6)) for c in range(3)])
+    _, mu, la = _material(rng, ratio)
+    _check_operator(u, mu, la, _profiles(profile, rng), True, 1)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("n", [15, 30, 45])
+def test_operator_constant_displacement_with_a_small_part(axis, n):
+    rng = np.random.default_rng(n)
+    x, y, z = _grid_arrays()
+    u = np.stack([2.0 ** -n * np.sin(0.4 * x + 0.3 * y + 0.2 * z + rng.uniform(0, 6)) for c in range(3)])
+    u[axis] += 1.0
+    _, mu, la = _material(rng)
+    _check_operator(u, mu, la, _profiles("ones", rng), True, 1)
+
+
+@pytest.mark.parametrize("profile", ["ones", "layers", "any"])
+def test_operator_largest_significands(profile):
+    rng = np.random.default_rng(8)
+    u = _largest(rng, (3,) + _grid_arrays()[0].shape)
+    mu, la = [f * np.ones(u.shape[1:]) for f in (2 - 2.0 ** -52, 4 - 2.0 ** -51)]
+    _check_operator(u, mu, la, _profiles(profile, rng), True, 1)
+    la *= -1  # coefficients of both signs
+    mu *= np.where(_grid_arrays()[0] % 2 == 0, 1.0, -1.0)
+    _check_operator(u, mu, la, _profiles(profile, rng), True, 1)

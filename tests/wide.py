@@ -20,10 +20,11 @@ def _interior(a):
     return out
 
 
-def operator(u, mu, la, st, h):
+def operator(u, mu, la, st, h, differences=False):
     """(L(u), terms): terms sums, per component, the magnitudes that one rounding of each
     product and sum is relative to: of a second difference every part of its weight times
-    both values, of a mixed term its coefficient times the inner differences."""
+    both values (times their difference, if differences), of a mixed term its coefficient
+    times the inner differences."""
     u, mu, la = [np.asarray(a, dtype=L) for a in (u, mu, la)]
     s = [_line(a, ax) for ax, a in enumerate(st)]
     out, terms = [], []
@@ -36,7 +37,8 @@ def operator(u, mu, la, st, h):
                  1: (a[-1] + a[2], 3 * (a[1] + a[0])), 2: (a[1], -0.75 * (a[0] + a[2]))}
             for m, (p, q) in w.items():
                 r = r + s[ax] * (p + q) * (_at(f, m, ax) - f) / 6
-                t = t + abs(s[ax]) * (abs(p) + abs(q)) * (abs(_at(f, m, ax)) + abs(f)) / 6
+                size = abs(_at(f, m, ax) - f) if differences else abs(_at(f, m, ax)) + abs(f)
+                t = t + abs(s[ax]) * (abs(p) + abs(q)) * size / 6
         for ax in range(3):
             if ax == c:
                 continue
