@@ -72,10 +72,10 @@ __device__ __forceinline__ Num add(const Num& a, const Num& b)
    return Num{to_odd(a.m, e - a.e + 1) + to_odd(b.m, e - b.e + 1), e + 1};
 }
 
-// The points of a column whose sums read a field or material value or a stretching factor
-// that is not finite, set to NaN after the march (see stage_fixed.cu: of the material a
-// component reads mu at every point of the three axes, lambda at its own point and along
-// its own axis).
+// The points of a column whose sums read a field value, a product c s or a product of two
+// stretching factors that is not finite, set to NaN after the march (see stage_fixed.cu: of the
+// coefficients along an axis the component of the axis reads (2 mu + lambda) s and lambda, the
+// others mu s and mu, and c s is not finite where c is not).
 __device__ void mark_not_finite(const OpFixed& a, int i, int j, int kbeg, int kend)
 {
    const Box& b = a.b;
@@ -84,15 +84,17 @@ __device__ void mark_not_finite(const OpFixed& a, int i, int j, int kbeg, int ke
    for (int k = kbeg; k <= kend; k++) {
       const long long p = pidx(b, i, j, k);
       auto bad = [&](int c, long long q) { return !isfinite(a.u[c * b.cs + b.ps * q]); };
-      bool nan[3] = {bad(0, p), bad(1, p), bad(2, p)}, all = !isfinite(a.mu[p]) || !isfinite(a.la[p]);
+      const double sx = str[0][0], sy = str[1][0], sz = str[2][k];
+      const bool xy = !isfinite(sx * sy), xz = !isfinite(sx * sz), yz = !isfinite(sy * sz);
+      bool nan[3] = {bad(0, p) || xy || xz, bad(1, p) || xy || yz, bad(2, p) || xz || yz};
       for (int ax = 0; ax < 3; ax++)
          for (int m = -2; m <= 2; m++) {
-            all = all || !isfinite(str[ax][(ax == 2 ? k : 0) + m]);
-            if (m == 0) continue;
             const long long q = p + m * st[ax];
-            all = all || !isfinite(a.mu[q]);
-            nan[ax] = nan[ax] || !isfinite(a.la[q]);
+            const double s = str[ax][(ax == 2 ? k : 0) + m], mu = a.mu[q];
+            const bool shear = !isfinite(mu * s), normal = !isfinite(fma(2.0, mu, a.la[q]) * s);
             for (int c = 0; c < 3; c++) {
+               nan[c] = nan[c] || (c == ax ? normal : shear);
+               if (m == 0) continue;
                nan[c] = nan[c] || bad(c, q);
                if (c == ax) continue;
                for (int n = -2; n <= 2; n++) {
@@ -103,7 +105,7 @@ __device__ void mark_not_finite(const OpFixed& a, int i, int j, int kbeg, int ke
             }
          }
       for (int c = 0; c < 3; c++)
-         if (all || nan[c]) a.lu[c * b.cs + b.ps * p] = __longlong_as_double(0x7ff8000000000000LL);
+         if (nan[c]) a.lu[c * b.cs + b.ps * p] = __longlong_as_double(0x7ff8000000000000LL);
    }
 }
 
@@ -212,6 +214,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
 
    if (tid == 0) sm.bad = 0;
    __syncthreads();
+   // a product of two factors may overflow where their biased exponents add to this
+   constexpr int kOver = 2 * 1023 + 1023;
+   auto exponent = [](double s) { return (__double2hiint(s) >> 20) & 0x7ff; };
+   const int exy = max(exponent(sxi), exponent(syj));
+   if (exponent(sxi) + exponent(syj) >= kOver) sm.bad = 1;
    // ring slots of planes k-2..k+2
    int qm2 = 3, qm1 = 4, q0 = 0, qp1 = 1, qp2 = 2;
    fetch(kbeg - 2);
@@ -266,6 +273,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
       __syncthreads();
       if (k < kend) fetch(k + 3);
       const double szk = __ldg(a.sz + (k - b.kb));
+      if (exy + exponent(szk) >= kOver) sm.bad = 1;
       const i64* v0 = &sm.v[q0][0][0];
       const unsigned* e0 = sm.ve[q0];
       const int qz[4] = {qm2, qm1, qp1, qp2};

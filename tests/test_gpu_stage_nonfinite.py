@@ -88,3 +88,34 @@ def test_operator_lambda_not_finite(soa, bad):
     ok = np.isfinite(want)
     scale = 64 * np.max((2 * mu + la)[np.isfinite(la)]) * np.max(np.abs(u)) / 0.3 ** 2
     assert np.max(np.abs(got - want)[ok]) <= 2.0 ** -46 * scale
+
+
+@pytest.mark.parametrize("case", ["mu s", "(2 mu + lambda) s", "sx sy", "sx sz"])
+def test_operator_products_that_overflow(case):
+    """Finite inputs whose products are not: mu or 2 mu + lambda times a factor, or two factors
+    of one point; the sums in FP64 are then infinite or NaN."""
+    nx, ny, nz = SHAPE
+    _, mu, la = smooth_material(nx, ny, nz, seed=4)
+    u, _ = smooth_fields(nx, ny, nz, seed=5)
+    st = [np.ones(n + 4) for n in SHAPE]
+    if case == "mu s":
+        mu *= 1e150
+        la *= 1e-150
+        st[1][9] = 1e200
+    elif case == "(2 mu + lambda) s":
+        la *= 1e150
+        st[1][9] = 1e200
+    else:
+        mu *= 1e-200
+        la *= 1e-200
+        st[0][20] = 1e160
+        st[1 if case == "sx sy" else 2][8] = -1e160
+    b = (-1, nx + 2, -1, ny + 2, -1, nz + 2)
+    want = np.zeros_like(u)
+    O.rhs4sg(1, b, nz, [0] * 6, want, u, mu, la, 0.3, *st)
+    lu = dev(np.zeros_like(u))
+    d = [dev(a) for a in (u, mu, la, *st)]
+    sg.check(sg.lib().sw4g_rhs4sg(1, *b, nz, (C.c_int * 6)(), lu.data_ptr(), *[t.data_ptr() for t in d[:3]], 0.3,
+                                  *[t.data_ptr() for t in d[3:]], None))
+    assert not np.all(np.isfinite(want))
+    assert np.array_equal(np.isfinite(host(lu)), np.isfinite(want))
