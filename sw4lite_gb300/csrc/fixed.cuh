@@ -141,18 +141,28 @@ __device__ __forceinline__ i64 mulc(i64 x, int2 c)
 }
 
 // x * f / 2^e for |x| < 2^62 and any finite factor f, with its full relative precision,
-// rounded to nearest; f / 2^e is below 1 in magnitude.
+// rounded to nearest; f / 2^e is below 1 in magnitude.  TINY: f may lie below the normal range
+// (asked for where the factors are a caller's; the time loop's profiles end at 1e-4, and the test
+// costs its stages 8 %).
+template <bool TINY>
 struct Scale {
    int hi, lo, e;
    bool neg;
    __device__ __forceinline__ explicit Scale(double f)
    {
       const int h = __double2hiint(f), eb = (h >> 20) & 0x7ff;
-      const int mh = eb == 0 ? 0 : (h & 0xfffff) | 0x100000;  // below the normal range: 0
-      const i64 c = (i64)(((unsigned long long)mh << 32) | (eb == 0 ? 0u : (unsigned)__double2loint(f))) << 4;
+      i64 c = (i64)(((unsigned long long)((h & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(f)) << 4;
+      e = eb - 1022;
+      if (!TINY) {
+         if (eb == 0) c = 0, e = -5000;
+      } else if (eb == 0) {  // zero and below the normal range
+         c = (__double_as_longlong(f) & 0xfffffffffffffLL) << 4;
+         const int n = c == 0 ? 0 : __clzll(c) - 7;
+         c <<= n;
+         e = c == 0 ? -5000 : -1021 - n;
+      }
       hi = (int)(c >> kSplit);
       lo = (int)(c & kMask) << 5;
-      e = eb == 0 ? -5000 : eb - 1022;
       neg = h < 0;
    }
    __device__ __forceinline__ i64 operator()(i64 x) const
@@ -167,9 +177,10 @@ struct Scale {
 __device__ __forceinline__ bool is_one(double x) { return __double_as_longlong(x) == 0x3ff0000000000000LL; }
 
 // times a stretching factor
+template <bool TINY>
 __device__ __forceinline__ Num stretched(const Num& d, double s)
 {
-   const Scale f(s);
+   const Scale<TINY> f(s);
    return Num{f(d.m), d.e + f.e};
 }
 
@@ -182,11 +193,12 @@ struct Triple {
 
 __device__ __forceinline__ Num times(const Num& d, int2 c, int e) { return Num{mulc(d.m, c), d.e + e - 1}; }
 
+template <bool TINY>
 __device__ __forceinline__ Triple products(Num s0, Num s1, const Num& m0, const Num& m1, int2 mu, int emu, int2 la, int ela,
                                            double f0, double f1)
 {
-   if (!is_one(f0)) s0 = stretched(s0, f0);
-   if (!is_one(f1)) s1 = stretched(s1, f1);
+   if (!is_one(f0)) s0 = stretched<TINY>(s0, f0);
+   if (!is_one(f1)) s1 = stretched<TINY>(s1, f1);
    const int es = max(s0.e, s1.e);
    Triple t;
    t.la = Num{mulc(sar(s0.m, es - s0.e + 1) + sar(s1.m, es - s1.e + 1), la), es + ela};
@@ -204,19 +216,32 @@ __device__ __forceinline__ Num outer(i64 g0, i64 g1, i64 g2, i64 g3, int e0, int
    return Num{d, d == 0 ? kNone : e};
 }
 
-// p * 2^e as FP64, rounded once; below the normal range 0, above it infinite.
-__device__ __forceinline__ double from_block(i64 p, int e)
+// p * 2^e as FP64, rounded once, above the range infinite.  Below the normal range it comes
+// times 2^kLow, with low set, so that it keeps its digits for the product that follows, whose
+// other factor brings 2^-kLow.
+constexpr int kLow = 200;
+__device__ __forceinline__ double from_block(i64 p, int e, bool& low)
 {
    const double r = __ll2double_rn(p);
    int hi = __double2hiint(r), lo = __double2loint(r);
-   const int eb = (hi >> 20) & 0x7ff, n = eb == 0 ? 0 : eb + e;
-   hi += e << 20;
+   const int eb = (hi >> 20) & 0x7ff;
+   low = eb + e <= 0;
+   e += low ? kLow : 0;
+   const int n = eb == 0 ? 0 : eb + e;
+   hi += (int)((unsigned)e << 20);
    if (n <= 0) hi = lo = 0;
    if (n >= 2047) {
       hi = p < 0 ? 0xfff00000 : 0x7ff00000;
       lo = 0;
    }
    return __hiloint2double(hi, lo);
+}
+
+// c * 2^-kLow for a factor c >= 0, by its exponent (0 below 2^(kLow - 1022))
+__device__ __forceinline__ double lowered(double c)
+{
+   const int hi = __double2hiint(c) - (kLow << 20);
+   return hi < (1 << 20) ? 0.0 : __hiloint2double(hi, __double2loint(c));
 }
 
 }  // namespace sw4g

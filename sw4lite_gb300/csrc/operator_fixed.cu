@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
                   const i64 s = (hh << up) + to_odd((xw >> 3) + wx, 27 - up);
                   // times the point's own factor
                   Num T = {s, s == 0 ? kNone : Ec + ep - up};
-                  if (!is_one(f)) T = stretched(T, f);
+                  if (!is_one(f)) T = stretched<true>(T, f);
                   S[c] = ax == 0 ? T : add(S[c], T);
                }
             }
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
       // products of the own point
       const int2 lm = limbs(cm[0]), ll = limbs(cm[1]);
       const int emu = ec[0] - 1022, ela = ec[1] - 1022;
-      const Triple z = products(D[0][0], D[1][1], D[0][2], D[1][2], lm, emu, ll, ela, sxi, syj);
+      const Triple z = products<true>(D[0][0], D[1][1], D[0][2], D[1][2], lm, emu, ll, ela, sxi, syj);
       if (full) {
          auto to_x = [&](const Triple& t, int q) {
             sm.gx[0][q] = t.la.m;
@@ -434,13 +434,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
             sm.gye[1][q] = (short)max(t.la.e, kNone);
             sm.gye[2][q] = (short)max(t.m1.e, kNone);
          };
-         to_x(products(D[1][1], D[2][2], D[1][0], D[2][0], lm, emu, ll, ela, syj, szk), ty * PX + tx + HALO);
-         to_y(products(D[0][0], D[2][2], D[0][1], D[2][1], lm, emu, ll, ela, sxi, szk), (ty + HALO) * TX + tx);
+         to_x(products<true>(D[1][1], D[2][2], D[1][0], D[2][0], lm, emu, ll, ela, syj, szk), ty * PX + tx + HALO);
+         to_y(products<true>(D[0][0], D[2][2], D[0][1], D[2][1], lm, emu, ll, ela, sxi, szk), (ty + HALO) * TX + tx);
          if (halo) {
             const int s = hrow * PX + hcl, o = yh ? 1 : PX, cs = yh ? 0 : 1, cc = 1 - cs;
             Num d0 = along(cs, s, o), d1 = down(2, s), d2 = along(cc, s, o), d3 = down(cc, s);
             if (small(d0) || small(d1) || small(d2) || small(d3)) rest(d0), rest(d1), rest(d2), rest(d3);
-            const Triple t = products(d0, d1, d2, d3, limbs(hm[0]), he[0] - 1022, limbs(hm[1]), he[1] - 1022, hin, szk);
+            const Triple t = products<true>(d0, d1, d2, d3, limbs(hm[0]), he[0] - 1022, limbs(hm[1]), he[1] - 1022, hin, szk);
             if (yh) to_y(t, hrow * TX + tx);
             else to_x(t, (hrow - HALO) * PX + hcl);
          }
@@ -460,8 +460,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
             Num cx = outer(x[0], x[1], x[3], x[4], hx[0], hx[1], hx[2], hx[3], max4(hx[0], hx[1], hx[2], hx[3]));
             Num cy = outer(y[0], y[TX], y[3 * TX], y[4 * TX], hy[0], hy[1], hy[2], hy[3], max4(hy[0], hy[1], hy[2], hy[3]));
             if (stx || sty || !is_one(szk)) {
-               cx = stretched(cx, c == 0 ? sxi : c == 1 ? sxi * syj : sxi * szk);
-               cy = stretched(cy, c == 0 ? syj * sxi : c == 1 ? syj : syj * szk);
+               cx = stretched<true>(cx, c == 0 ? sxi : c == 1 ? sxi * syj : sxi * szk);
+               cy = stretched<true>(cy, c == 0 ? syj * sxi : c == 1 ? syj : syj * szk);
             }
             P[c].e = max(S[c].e, max(cx.e, cy.e));
             const i64 s8 = to_odd(S[c].m, P[c].e - S[c].e + 3);  // second differences carry 1/6, mixed terms 1/144
@@ -480,9 +480,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
          for (int c = 0; c < 3; c++) {
             const int h0 = sm.gze[z0][c][tid], h1 = sm.gze[z1][c][tid], h3 = sm.gze[z3][c][tid], h4 = zn[c].e;
             Num g = outer(sm.gz[z0][c][tid], sm.gz[z1][c][tid], sm.gz[z3][c][tid], zn[c].m, h0, h1, h3, h4, max4(h0, h1, h3, h4));
-            if (stx || sty || !is_one(szp)) g = stretched(g, c == 0 ? szp * sxi : c == 1 ? szp * syj : szp);
+            if (stx || sty || !is_one(szp)) g = stretched<true>(g, c == 0 ? szp * sxi : c == 1 ? szp * syj : szp);
             const int eF = max(pq[0][c].e, g.e);
-            a.lu[c * b.cs + b.ps * pp] = a.cof * from_block(to_odd(pq[0][c].m, eF - pq[0][c].e) + to_odd(g.m, eF - g.e + 2), eF - 1072);
+            bool low;
+            const double lu = from_block(to_odd(pq[0][c].m, eF - pq[0][c].e) + to_odd(g.m, eF - g.e + 2), eF - 1072, low);
+            a.lu[c * b.cs + b.ps * pp] = (low ? lowered(a.cof) : a.cof) * lu;
          }
       }
       const Num zn[3] = {z.m0, z.m1, z.la};

@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
       const bool stz = !is_one(szk);
       const int2 cm = make_int2(cc.x, cc.y), cl = make_int2(cc.z, cc.w);
       const int emu = (int)(short)(ee & 0xffff), el = ee >> 16;
-      const Triple z = products(D[0][0], D[1][1], D[0][2], D[1][2], cm, emu, cl, el, sxi, syj);
+      const Triple z = products<false>(D[0][0], D[1][1], D[0][2], D[1][2], cm, emu, cl, el, sxi, syj);
       if (full) {
          auto to_x = [&](const Triple& t, int q) {
             sm.gx[0][q] = t.la.m;
@@ -406,8 +406,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
             sm.gye[1][q] = (short)t.la.e;
             sm.gye[2][q] = (short)t.m1.e;
          };
-         to_x(products(D[1][1], D[2][2], D[1][0], D[2][0], cm, emu, cl, el, syj, szk), ty * PX + tx + HALO);
-         to_y(products(D[0][0], D[2][2], D[0][1], D[2][1], cm, emu, cl, el, sxi, szk), (ty + HALO) * TX + tx);
+         to_x(products<false>(D[1][1], D[2][2], D[1][0], D[2][0], cm, emu, cl, el, syj, szk), ty * PX + tx + HALO);
+         to_y(products<false>(D[0][0], D[2][2], D[0][1], D[2][1], cm, emu, cl, el, sxi, szk), (ty + HALO) * TX + tx);
          if (halo) {
             // y outer: mu v_x, la (u_x + w_z), mu v_z;  x outer: la (v_y + w_z), mu u_y, mu u_z
             const int s = hrow * PX + hcl, o = yh ? 1 : PX, cs = yh ? 0 : 1, cm = 1 - cs;
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
             }
             Num d0 = along(cs, s, o), d1 = down(2, s), d2 = along(cm, s, o), d3 = down(cm, s);
             if (small(d0) || small(d1) || small(d2) || small(d3)) rest(d0), rest(d1), rest(d2), rest(d3);
-            const Triple t = products(d0, d1, d2, d3, make_int2(hc.x, hc.y), (int)(short)(he & 0xffff), make_int2(hc.z, hc.w), he >> 16, hst, szk);
+            const Triple t = products<false>(d0, d1, d2, d3, make_int2(hc.x, hc.y), (int)(short)(he & 0xffff), make_int2(hc.z, hc.w), he >> 16, hst, szk);
             if (yh) to_y(t, hrow * TX + tx);
             else to_x(t, (hrow - HALO) * PX + hcl);
          }
@@ -452,8 +452,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
             Num cx = outer(x[0], x[1], x[3], x[4], hx[0], hx[1], hx[2], hx[3], max4(hx[0], hx[1], hx[2], hx[3]));
             Num cy = outer(y[0], y[TX], y[3 * TX], y[4 * TX], hy[0], hy[1], hy[2], hy[3], max4(hy[0], hy[1], hy[2], hy[3]));
             if (stx || sty || stz) {
-               cx = stretched(cx, c == 0 ? sxi : c == 1 ? sxi * syj : sxi * szk);
-               cy = stretched(cy, c == 0 ? syj * sxi : c == 1 ? syj : syj * szk);
+               cx = stretched<false>(cx, c == 0 ? sxi : c == 1 ? sxi * syj : sxi * szk);
+               cy = stretched<false>(cy, c == 0 ? syj * sxi : c == 1 ? syj : syj * szk);
             }
             P[c].e = max(eS[c], max(cx.e, cy.e));
             P[c].m = to_odd(S[c], P[c].e - eS[c] + 1) + to_odd(cx.m, P[c].e - cx.e + 2) + to_odd(cy.m, P[c].e - cy.e + 2);
@@ -471,11 +471,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
          for (int c = 0; c < 3; c++) {
             const int h0 = sm.gze[z0][c][tid], h1 = sm.gze[z1][c][tid], h3 = sm.gze[z3][c][tid], h4 = zn[c].e;
             Num g = outer(sm.gz[z0][c][tid], sm.gz[z1][c][tid], sm.gz[z3][c][tid], zn[c].m, h0, h1, h3, h4, max4(h0, h1, h3, h4));
-            if (st) g = stretched(g, c == 0 ? szp * sxi : c == 1 ? szp * syj : szp);
+            if (st) g = stretched<false>(g, c == 0 ? szp * sxi : c == 1 ? szp * syj : szp);
             const int eF = max(pq[0][c].e, g.e);
             const i64 F = to_odd(pq[0][c].m, eF - pq[0][c].e) + to_odd(g.m, eF - g.e + 2);
-            const double lu = from_block(F, eF - 1072);
-            const double v = base[c] + cr * lu;
+            bool low;
+            const double lu = from_block(F, eF - 1072, low);
+            const double v = base[c] + (low ? lowered(cr) : cr) * lu;
             if (FORM != 0) em = max(em, (__double2hiint(v) >> 20) & 0x7ff);
             a.out[pp + c * npts] = v;
          }

@@ -67,7 +67,7 @@ def _predict(mat, u, um, dt, sides):
     return out, st
 
 
-def _check(mat, u, um, sides, coupled):
+def _check(mat, u, um, sides, coupled, least=0):
     rho, mu, la = mat
     dt = 0.3 * H / float(np.sqrt(np.max((4 * mu + la) / rho)))
     got, st = _predict(mat, u, um, dt, sides)
@@ -79,7 +79,7 @@ def _check(mat, u, um, sides, coupled):
             terms[c] = wide.operator(alone, mu, la, st, H)[1][c]
     d2 = wide.L(dt) ** 2 / wide.L(1) / rho
     want = 2 * wide.L(1) * u - um + d2 * val
-    bar = wide.L(2) ** -53 * (3 * (2 * abs(u) + abs(um)) + 16 * d2 * terms)
+    bar = wide.L(2) ** -53 * (3 * (2 * abs(u) + abs(um)) + 16 * d2 * terms) + least
     for where, x in got:
         sel = (slice(None), slice(2, -2), slice(2, -2), slice(2, -2))
         full = np.full(u.shape, np.nan)
@@ -156,7 +156,7 @@ def test_soft_and_stiff_coefficients(sides, ratio):
     _check(_material(rng, ratio), u, 0.8 * u, sides, coupled=True)
 
 
-def _check_operator(u, mu, la, st, coupled, soa):
+def _check_operator(u, mu, la, st, coupled, soa, least=0):
     val, terms = wide.operator(u, mu, la, st, H, differences=True)
     if not coupled:
         for c in range(3):
@@ -172,7 +172,7 @@ def _check_operator(u, mu, la, st, coupled, soa):
                                   *[t.data_ptr() for t in d[3:]], None))
     got = host(lu).reshape(u.shape) if soa else np.moveaxis(host(lu).reshape(*u.shape[1:], 3), 3, 0)
     sel = (slice(None), slice(2, -2), slice(2, -2), slice(2, -2))
-    bar = 16 * wide.L(2) ** -53 * terms[sel]
+    bar = 16 * wide.L(2) ** -53 * terms[sel] + least
     err = abs(got[sel] - val[sel])
     with np.errstate(all="ignore"):
         assert np.all(err <= bar), float(np.nanmax(np.where(bar > 0, err / bar, np.inf * err)))
@@ -238,3 +238,35 @@ def test_operator_largest_significands(profile):
     la *= -1  # coefficients of both signs
     mu *= np.where(_grid_arrays()[0] % 2 == 0, 1.0, -1.0)
     _check_operator(u, mu, la, _profiles(profile, rng), True, 1)
+
+
+LEAST = wide.L(2) ** -1074
+
+
+@pytest.mark.skipif(LEAST / 4 == 0, reason="needs an extended exponent range")
+def test_below_the_normal_range():
+    """Levels and results below 2^-1022 are rounded to multiples of 2^-1074, as FP64 does it: the
+    sum, the product dt^2/rho L and L itself, each once (half a unit), dt^2/rho being below 1.
+    The operator rounds its sum and the product with 1/(144 h^2) = 2.8, which multiplies the
+    first's half unit."""
+    rng = np.random.default_rng(3)
+    x, y, z = _grid_arrays()
+    wave = np.stack([np.sin(0.4 * x + 0.3 * y + 0.5 * z + rng.uniform(0, 6)) for c in range(3)])
+    u = np.round(wave * 2 ** 14) * 2.0 ** -1074
+    _check(_material(rng), u, 0.5 * np.round(u / 2.0 ** -1073) * 2.0 ** -1073, 2, True, least=2 * LEAST)
+    _, mu, la = _material(rng)
+    _check_operator(wave * 2.0 ** -440, mu * 2.0 ** -600, la * 2.0 ** -600, _profiles("layers", rng), True, 1, least=2 * LEAST)
+
+
+@pytest.mark.skipif(LEAST / 4 == 0, reason="needs an extended exponent range")
+def test_operator_factor_below_the_normal_range():
+    """A stretching factor of 3 x 2^-1040 along x and coefficients of 2^900: the x component of a
+    field in y has the mixed terms alone."""
+    rng = np.random.default_rng(4)
+    x, y, z = _grid_arrays()
+    u = np.zeros((3,) + x.shape)
+    u[1] = np.sin(0.4 * x + 0.3 * y + 0.5 * z)
+    _, mu, la = _material(rng)
+    st = _profiles("ones", rng)
+    st[0][:] = 3 * 2.0 ** -1040
+    _check_operator(u, mu * 2.0 ** 900, la * 2.0 ** 900, st, True, 1)
