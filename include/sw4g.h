@@ -299,6 +299,18 @@ int sw4g_ew_set_time_step(sw4g_ew* ew, double dt, double t0);
 /* dt from the CFL number, adjusted to end at tmax (EW::computeDT, src/EW.C:5041) */
 int sw4g_ew_compute_time_step(sw4g_ew* ew, double cfl, double tmax, double* dt, int* nsteps);
 double sw4g_ew_time(const sw4g_ew* ew);
+/* The arithmetic of an FP64 object's stages (no reference counterpart): block fixed-point on
+   the integer pipes, twice as fast, or FP64, whose weights take 80 bytes a grid point less.
+   An object is made with the first where its coefficients fit; it changes to the second where
+   a later allocation of its own finds no room.  Both have FP64's accuracy and differ in
+   rounding: runs that are to agree bit for bit, subdomains of one grid among them, need the
+   same form (sw4g_ew_step_group sees to it).  sw4g_ew_stage_form returns the form (-1 for the
+   FP32-mixed form); sw4g_ew_set_stage_form changes it between steps, prepares the coefficients
+   anew and gives the other form's memory back (SW4G_CUDA_ERROR, nothing changed, where the
+   fixed-point coefficients find no room). */
+enum { SW4G_STAGES_FP64 = 0, SW4G_STAGES_FIXED = 1 };
+int sw4g_ew_stage_form(const sw4g_ew* ew);
+int sw4g_ew_set_stage_form(sw4g_ew* ew, int form);
 /* CUDA graphs for the fused time loop and the gradient (on != 0): sw4g_ew_step and
    sw4g_ew_gradient then replay captured chunks of steps, bit-identical to direct
    launches; the forcing time and record row are kept in device memory.  Needs an

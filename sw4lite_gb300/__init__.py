@@ -92,6 +92,7 @@ def topo_desc(amp, xc, yc, lx, ly, zeta_break=0.95, order=4) -> TopoDesc:
 GAUSSIAN, C6SMOOTHBUMP, RICKER, VERYSMOOTHBUMP = 0, 1, 2, 3
 # boundary kinds (the reference's boundaryConditionType numbering)
 FREE, DIRICHLET, SUPERGRID, PERIODIC, INTERFACE = 0, 1, 2, 3, 4
+STAGES_FP64, STAGES_FIXED = 0, 1
 MODE_PHASES, MODE_FUSED = 0, 1
 # receiver record modes (the reference's TimeSeries::receiverMode numbering)
 REC_DISPLACEMENT, REC_DIV, REC_CURL, REC_STRAINS, REC_VELOCITY, REC_GRADIENT = 0, 1, 2, 3, 4, 5
@@ -147,6 +148,8 @@ _SIGS = {
     "sw4g_ew_compute_time_step": ([_VP, C.c_double, C.c_double, _D, _I], C.c_int),
     "sw4g_ew_time": ([_VP], C.c_double),
     "sw4g_ew_set_graphs": ([_VP, C.c_int], C.c_int),
+    "sw4g_ew_stage_form": ([_VP], C.c_int),
+    "sw4g_ew_set_stage_form": ([_VP, C.c_int], C.c_int),
     "sw4g_ew_set_gradient_memory": ([_VP, C.c_longlong], C.c_int),
     "sw4g_ew_set_source_discretization": ([_VP, C.c_int], C.c_int),
     "sw4g_ew_write_checkpoint": ([_VP, C.c_char_p, C.c_int], C.c_int),
@@ -402,6 +405,15 @@ class EW:
     def set_graphs(self, on=True):
         """Replay the fused time loop (and the gradient's loops) as CUDA graphs."""
         check(lib().sw4g_ew_set_graphs(self._h, int(bool(on))), "set_graphs")
+
+    def stage_form(self) -> int:
+        """The arithmetic of the FP64 stages: STAGES_FIXED or STAGES_FP64; -1 for the
+        FP32-mixed form."""
+        return lib().sw4g_ew_stage_form(self._h)
+
+    def set_stage_form(self, form):
+        """Change it between steps (sw4g_ew_set_stage_form)."""
+        check(lib().sw4g_ew_set_stage_form(self._h, form), "set_stage_form")
 
     def set_source_discretization(self, on_device=True):
         """Compute add_source's grid-point sources on the device (the whole batch,

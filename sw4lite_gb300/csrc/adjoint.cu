@@ -194,7 +194,7 @@ int EW::gradient(int nsteps, int ckpt, const double* obs, bool obs_on_device, do
          gc.mixed == (int)mixed_ && gc.host_grad == (int)!grad_on_device && gc.budget == grad_store_bytes_)) {
       drop_grad_cache();
       auto alloc = [&](double** p, size_t bytes) {
-         int s = cuda_ok(cudaMalloc(p, bytes));
+         int s = this->alloc(p, bytes);
          if (s == kOk) gc.mem.push_back(*p);
          return s;
       };

@@ -797,6 +797,16 @@ int sw4g_ew_status(sw4g_ew* ew)
    return ew ? ew->impl->status() : SW4G_BAD_ARGUMENT;
 }
 
+int sw4g_ew_stage_form(const sw4g_ew* ew)
+{
+   return ew ? ew->impl->stage_form() : -1;
+}
+
+int sw4g_ew_set_stage_form(sw4g_ew* ew, int form)
+{
+   return ew ? ew->impl->set_stage_form(form) : SW4G_BAD_ARGUMENT;
+}
+
 int sw4g_ew_enforce_bc(sw4g_ew* ew, double* u)
 {
    if (!ew || !u) return SW4G_BAD_ARGUMENT;

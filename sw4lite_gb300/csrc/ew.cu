@@ -156,31 +156,91 @@ int EW::init()
 }
 
 // The fixed-point stages' coefficients take 224 bytes a point, the FP64 stages' weights
-// 144.  The fixed-point stages run where their coefficients fit and leave room for the
-// phase order's work arrays (72 bytes a point, allocated when first used), so a grid that
-// fits with the FP64 stages alone runs on those: at 512^3 a step takes 95 ms on the FP64
-// stages, 40 ms on the fixed-point ones; an empty 288 GB device holds 7e8 points with
-// them and 8e8 without.
+// 144.  The fixed-point stages run where their coefficients fit and leave room for what the
+// object is known to allocate later: the phase order's work arrays and the staging buffer (96
+// bytes a point) and the curvilinear grid's coefficients.  Else, and where another allocation
+// of the object finds no room later (a gradient's levels), the FP64 stages run, so every grid and
+// gradient runs that fits with them: at 512^3 a step takes 95 ms on the FP64 stages, 50 ms on the
+// fixed-point ones.  The two round differently; stage_form tells which one runs.
 int EW::alloc_stage_coefficients()
 {
    const size_t n = (size_t)npts_;
    const Box b = make_box(1, b_.ib, b_.ie, b_.jb, b_.je, b_.kb, b_.ke);
-   const size_t wbytes = (size_t)fixed_weight_len(b) * sizeof(int2);
-   const size_t need = wbytes + n * (sizeof(int4) + 4 * sizeof(int) + 9 * sizeof(double));
+   size_t need = (size_t)fixed_weight_len(b) * sizeof(int2) + n * (sizeof(int4) + 4 * sizeof(int) + 12 * sizeof(double));
+   if (cv_)
+      need += curv_coef_doubles(cv_->npts, (long long)(cv_->b.ie - cv_->b.ib + 1) * (cv_->b.je - cv_->b.jb + 1)) * sizeof(double);
    size_t free = 0, total = 0;
    SW4G_TRY(cuda_ok(cudaMemGetInfo(&free, &total)));
-   if (free >= need + (size_t)(64 << 20)) {
-      if (cudaMalloc(&fc_.w, wbytes) == cudaSuccess && cudaMalloc(&fc_.c, n * sizeof(int4)) == cudaSuccess &&
-          cudaMalloc(&fc_.e, n * sizeof(int)) == cudaSuccess && cudaMalloc(&fc_.ew, 3 * n * sizeof(int)) == cudaSuccess &&
-          cudaMalloc(&fc_.bad, sizeof(int)) == cudaSuccess)
-         return kOk;
+   if (free >= need + (size_t)(64 << 20) && alloc_fixed_coefficients() == kOk) return kOk;
+   return alloc_fp64_weights();
+}
+
+int EW::alloc_fixed_coefficients()
+{
+   const size_t n = (size_t)npts_;
+   const Box b = make_box(1, b_.ib, b_.ie, b_.jb, b_.je, b_.kb, b_.ke);
+   if (cudaMalloc(&fc_.w, (size_t)fixed_weight_len(b) * sizeof(int2)) == cudaSuccess &&
+       cudaMalloc(&fc_.c, n * sizeof(int4)) == cudaSuccess && cudaMalloc(&fc_.e, n * sizeof(int)) == cudaSuccess &&
+       cudaMalloc(&fc_.ew, 3 * n * sizeof(int)) == cudaSuccess && cudaMalloc(&fc_.bad, sizeof(int)) == cudaSuccess)
+      return kOk;
+   cudaGetLastError();
+   free_fixed_coefficients();
+   return kCudaError;
+}
+
+int EW::alloc_fp64_weights()
+{
+   const size_t n = (size_t)npts_;
+   if (cudaMalloc(&wstore_, (kWeightArrays + kWeightSums) * n * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
-      free_fixed_coefficients();
+      wstore_ = nullptr;
+      return kCudaError;
    }
-   SW4G_TRY(cuda_ok(cudaMalloc(&wstore_, (kWeightArrays + kWeightSums) * n * sizeof(double))));
    for (int q = 0; q < kWeightArrays; q++) w_.p[q] = wstore_ + q * n;
    for (int q = 0; q < kWeightSums; q++) w_.s[q] = wstore_ + (kWeightArrays + q) * n;
    return kOk;
+}
+
+int EW::prepare_stages()
+{
+   const Box b = make_box(1, b_.ib, b_.ie, b_.jb, b_.je, b_.kb, b_.ke);
+   if (fc_.w) return launch_fixed_coef(b, mu_, la_, dprof_[3], dprof_[4], dprof_[5], g_.h, fc_, stream_);
+   return launch_weights(b, mu_, la_, dprof_[3], dprof_[4], dprof_[5], g_.h, w_, stream_);
+}
+
+int EW::set_stage_form(int form)
+{
+   if (mixed_) return kNotSupported;
+   if (!ready_ || part_ != 0 || (form != kStagesFp64 && form != kStagesFixed)) return kBadArgument;
+   if (form == stage_form()) return kOk;
+   SW4G_TRY(cuda_ok(cudaStreamSynchronize(stream_)));
+   drop_graphs();  // the graphs hold the old coefficients
+   if (form == kStagesFixed) {
+      SW4G_TRY(alloc_fixed_coefficients());  // beside the weights: without room these stay
+      cudaFree(wstore_);
+      wstore_ = nullptr;
+      w_ = WeightPtrs{};
+   } else if (alloc_fp64_weights() == kOk) {
+      free_fixed_coefficients();
+   } else {
+      free_fixed_coefficients();
+      SW4G_TRY(alloc_fp64_weights());
+   }
+   if (!material_) return kOk;
+   SW4G_TRY(prepare_stages());
+   return cuda_ok(cudaStreamSynchronize(stream_));
+}
+
+int EW::alloc_bytes(void** p, size_t bytes)
+{
+   *p = nullptr;
+   cudaError_t e = cudaMalloc(p, bytes);
+   if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();  // or the next launch would report it
+      if (stage_form() == kStagesFixed && set_stage_form(kStagesFp64) == kOk) e = cudaMalloc(p, bytes);
+      if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+   }
+   return cuda_ok(e);
 }
 
 void EW::free_fixed_coefficients()
@@ -211,10 +271,8 @@ int EW::set_material(const double* rho, const double* mu, const double* la, bool
    Box b = make_box(1, b_.ib, b_.ie, b_.jb, b_.je, b_.kb, b_.ke);
    for (int side = 0; side < 2; side++)
       if (zc_[side]) SW4G_TRY(launch_zcoef(b, g_.nz, side == 0, mu_, la_, zc_[side], stream_));
-   if (fc_.w) {
-      SW4G_TRY(launch_fixed_coef(b, mu_, la_, dprof_[3], dprof_[4], dprof_[5], g_.h, fc_, stream_));
-   } else if (!mixed_) {
-      SW4G_TRY(launch_weights(b, mu_, la_, dprof_[3], dprof_[4], dprof_[5], g_.h, w_, stream_));
+   if (!mixed_) {
+      SW4G_TRY(prepare_stages());
    } else {
       SW4G_TRY(launch_to_f32(npts_, rho_, rho32_, stream_));
       SW4G_TRY(launch_df2_from_f64(npts_, mu_, reinterpret_cast<float2*>(mu32_), stream_));
@@ -493,7 +551,7 @@ int EW::compute_time_step(double cfl, double tmax, double* dt, int* nsteps)
 int EW::ensure_staging()
 {
    if (staging_) return kOk;
-   return cuda_ok(cudaMalloc(&staging_, 3 * (size_t)npts_ * sizeof(double)));
+   return alloc(&staging_, 3 * (size_t)npts_ * sizeof(double));
 }
 
 int EW::set_fields(const double* u, const double* um, bool on_device)
@@ -562,11 +620,10 @@ int EW::enforce_bc(double* u)
 
 int EW::ensure_phase_arrays()
 {
-   if (lu_) return kOk;
+   if (lu_ && f_ && uacc_) return kOk;
    const size_t bytes = 3 * (size_t)npts_ * sizeof(double);
-   SW4G_TRY(cuda_ok(cudaMalloc(&lu_, bytes)));
-   SW4G_TRY(cuda_ok(cudaMalloc(&f_, bytes)));
-   SW4G_TRY(cuda_ok(cudaMalloc(&uacc_, bytes)));
+   for (double** p : {&lu_, &f_, &uacc_})
+      if (!*p) SW4G_TRY(alloc(p, bytes));
    SW4G_TRY(cuda_ok(cudaMemsetAsync(lu_, 0, bytes, stream_)));
    SW4G_TRY(cuda_ok(cudaMemsetAsync(uacc_, 0, bytes, stream_)));
    return kOk;
@@ -693,7 +750,7 @@ int EW::set_graphs(bool on)
 {
    if (!ready_) return kBadArgument;
    if (on && !stream_) return kNotSupported;  // no stream capture on the legacy default stream
-   if (on && !dclock_) SW4G_TRY(cuda_ok(cudaMalloc(&dclock_, 4 * sizeof(double))));
+   if (on && !dclock_) SW4G_TRY(alloc(&dclock_, 4 * sizeof(double)));
    if (!on) drop_graphs();
    graphs_ = on;
    return kOk;
@@ -819,10 +876,10 @@ int EW::set_receivers(int n, const int* ijk, const int* mode, int capacity, cons
    rec_initial_ = false;
    rec_curv_ = false;
    if (n == 0) return kOk;
-   SW4G_TRY(cuda_ok(cudaMalloc(&drec_mem_, host.size() * sizeof(int))));
+   SW4G_TRY(alloc(&drec_mem_, host.size() * sizeof(int)));
    SW4G_TRY(cuda_ok(cudaMemcpy(drec_mem_, host.data(), host.size() * sizeof(int),
                                cudaMemcpyHostToDevice)));
-   SW4G_TRY(cuda_ok(cudaMalloc(&records_, (size_t)capacity * nvals * sizeof(double))));
+   SW4G_TRY(alloc(&records_, (size_t)capacity * nvals * sizeof(double)));
    SW4G_TRY(cuda_ok(cudaMemsetAsync(records_, 0, (size_t)capacity * nvals * sizeof(double), stream_)));
    const int* d = static_cast<const int*>(drec_mem_);
    drec_.n = n;

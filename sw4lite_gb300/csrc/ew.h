@@ -59,6 +59,12 @@ enum StepMode : int {
    kModeFused = 1,   // fused predictor and corrector stage kernels
 };
 
+// The arithmetic of an FP64 object's stages (stage_form)
+enum StageForm : int {
+   kStagesFp64 = 0,   // stage_fused.cu
+   kStagesFixed = 1,  // stage_fixed.cu
+};
+
 class EW {
  public:
    // topo != nullptr: a curvilinear grid over that topography on top of this grid,
@@ -141,6 +147,11 @@ class EW {
    // Synchronises the object's stream and returns kTimeout if a kernel's bounded wait
    // gave up since the last call (clearing the flag), else kOk.
    int status();
+   // The form its stages run in: chosen when the object is made (alloc_stage_coefficients),
+   // kStagesFp64 from then on if a later allocation of its own finds no room, or what
+   // set_stage_form asks for; -1 in the FP32-mixed form.  Between steps only.
+   int stage_form() const { return mixed_ ? -1 : fc_.w ? kStagesFixed : kStagesFp64; }
+   int set_stage_form(int form);
    // CUDA graphs for the fused time loop: when on, step() replays captured chunks of
    // kGraphSteps steps (a multiple of the level rotation's period 3) and gradient()
    // replays its forward chunks, recompute segments and adjoint segments; the forcing
@@ -274,7 +285,18 @@ class EW {
    WeightPtrs w_{};  // ... or, without room for them, of the FP64 stages
    double* wstore_ = nullptr;
    int alloc_stage_coefficients();
+   int alloc_fixed_coefficients();
+   int alloc_fp64_weights();
    void free_fixed_coefficients();
+   int prepare_stages();  // the stages' coefficients from the material
+   // Device memory of a made object.  Where there is no room the fixed-point coefficients,
+   // 80 bytes a point more than the FP64 stages' weights, make some.
+   int alloc_bytes(void** p, size_t bytes);
+   template <class T>
+   int alloc(T** p, size_t bytes)
+   {
+      return alloc_bytes(reinterpret_cast<void**>(p), bytes);
+   }
    double* lev_[4] = {};
    int iu_ = 0, ium_ = 1;
    double* lu_ = nullptr;   // phase mode work arrays

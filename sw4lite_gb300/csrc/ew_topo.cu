@@ -214,16 +214,16 @@ int EW::set_material_grid(int grid, const double* rho, const double* mu, const d
    SW4G_TRY(cuda_ok(cudaMemcpyAsync(cv_->mu, mu, bytes, kind, stream_)));
    SW4G_TRY(cuda_ok(cudaMemcpyAsync(cv_->la, la, bytes, kind, stream_)));
    if (!cv_->coef)
-      SW4G_TRY(cuda_ok(cudaMalloc(&cv_->coef, curv_coef_doubles(cv_->npts, (long long)(cv_->b.ie - cv_->b.ib + 1) *
-                                                                           (cv_->b.je - cv_->b.jb + 1)) *
-                                                 sizeof(double))));
+      SW4G_TRY(alloc(&cv_->coef, curv_coef_doubles(cv_->npts, (long long)(cv_->b.ie - cv_->b.ib + 1) *
+                                                                  (cv_->b.je - cv_->b.jb + 1)) *
+                                     sizeof(double)));
    const Bounds& cb = cv_->b;
    SW4G_TRY(curv_coef_setup(make_box(1, cb.ib, cb.ie, cb.jb, cb.je, cb.kb, cb.ke), cv_->mu, cv_->la,
                             cv_->rho, cv_->met, cv_->jac, dprof_[3], dprof_[4], cv_->coef, &cv_->cc,
                             stream_));
    if (mixed_) {
       if (!cv_->coefdf)
-         SW4G_TRY(cuda_ok(cudaMalloc(&cv_->coefdf, curv_coef_df_floats(cv_->npts) * sizeof(float))));
+         SW4G_TRY(alloc(&cv_->coefdf, curv_coef_df_floats(cv_->npts) * sizeof(float)));
       SW4G_TRY(curv_coef_df_setup(cv_->npts, cv_->cc, cv_->coefdf, &cv_->cd, stream_));
    }
    SW4G_TRY(cuda_ok(cudaStreamSynchronize(stream_)));

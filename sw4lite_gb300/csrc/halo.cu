@@ -177,6 +177,13 @@ int step_group(EW* const* subs, int n, const int* nb, int nsteps)
       }
       return kOk;
    };
+   // one arithmetic for all, or the subdomains would not reproduce the undivided run
+   bool fp64 = false;
+   for (int s = 0; s < n; s++) fp64 = fp64 || subs[s]->stage_form() == kStagesFp64;
+   for (int s = 0; s < n && st == kOk && fp64; s++) {
+      on(s);
+      if (subs[s]->stage_form() == kStagesFixed) st = subs[s]->set_stage_form(kStagesFp64);
+   }
    for (int step = 0; step < nsteps && st == kOk; step++) {
       for (int part = 0; part < 3 && st == kOk; part++) {
          for (int s = 0; s < n && st == kOk; s++) {

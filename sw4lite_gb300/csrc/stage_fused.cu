@@ -881,6 +881,7 @@ int launch_fused_stage(const FusedStage& st, cudaStream_t stream)
    const Box& b = st.b;
    if (b.cs != b.npts) return kNotSupported;  // SoA only
    if (st.fc.w) return launch_fixed_stage(st, stream);
+   if (!st.w.p[0]) return kCudaError;  // a change of the form found no room for the weights
    FusedArgs a;
    a.ib = b.ib; a.ie = b.ie; a.jb = b.jb; a.je = b.je; a.kb = b.kb; a.ke = b.ke;
    a.ni = b.ni; a.nij = b.nij; a.npts = b.npts;

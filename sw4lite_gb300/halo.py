@@ -90,12 +90,26 @@ def torch_transfer(group=None):
     return run
 
 
+def agree_on_stages(ew, group=None, device=None):
+    """The same arithmetic on every rank: the FP64 stages where one rank's object runs on
+    them (EW.stage_form).  Collective."""
+    import torch
+    import torch.distributed as dist
+
+    form = torch.tensor([ew.stage_form()], dtype=torch.int32, device=device)
+    dist.all_reduce(form, op=dist.ReduceOp.MIN, group=group)
+    if 0 <= int(form) < ew.stage_form():
+        ew.set_stage_form(int(form))
+
+
 def step_distributed(ew, neighbors, nsteps, group=None):
     """nsteps steps of this rank's subdomain object with torch.distributed halo
-    exchanges (NCCL for device buffers)."""
+    exchanges (NCCL for device buffers), all ranks on one form of the stages."""
     import torch
 
     dev = torch.device("cuda", torch.cuda.current_device())
+    if any(n >= 0 for n in neighbors):
+        agree_on_stages(ew, group, dev)
     bufs = {(a, s): torch.empty(ew.halo_bytes(a), dtype=torch.uint8, device=dev)
             for a in (0, 1) for s in (0, 1)}
 

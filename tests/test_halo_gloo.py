@@ -103,3 +103,36 @@ def test_blocks_tile_the_grid_and_neighbours_agree(gnx, gny, px, py):
                 else:
                     assert (ti0, ti1) == (i0, i1) and (tj1 + 1 == j0 if q == 2 else tj0 == j1 + 1)
     assert np.all(cover[1:, 1:] == 1)
+
+
+class _Stages:
+    """An object's form of the stages, without a GPU."""
+
+    def __init__(self, form):
+        self.form = form
+
+    def stage_form(self):
+        return self.form
+
+    def set_stage_form(self, form):
+        self.form = form
+
+
+def _agree_main(rank, world, port, forms, out_dir):
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))
+    sys.path.insert(0, ROOT)
+    import torch.distributed as dist
+    from sw4lite_gb300 import halo
+    dist.init_process_group("gloo", rank=rank, world_size=world)
+    ew = _Stages(forms[rank])
+    halo.agree_on_stages(ew)
+    with open(os.path.join(out_dir, f"rank{rank}.txt"), "w") as fh:
+        fh.write(str(ew.form))
+    dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("forms,want", [((1, 0), 0), ((1, 1), 1), ((0, 0), 0), ((-1, -1), -1)])
+def test_ranks_agree_on_the_stages(tmp_path, forms, want):
+    """Block fixed-point (1) only where every rank runs it; the FP32-mixed form (-1) as it is."""
+    mp.spawn(_agree_main, args=(2, _free_port(), forms, str(tmp_path)), nprocs=2, join=True)
+    assert [int(open(tmp_path / f"rank{r}.txt").read()) for r in range(2)] == [want] * 2
