@@ -300,19 +300,11 @@ int launch_curv_operator(const CurvSpec& s, int k1, int k2, double* lu, cudaStre
    a.sy = s.stry;
    a.lu = lu;
    static_assert(sizeof(Smem) <= 113 * 1024, "two CTAs per SM");
-   // the opt-in shared-memory size is a per-device function attribute
-   int dev = 0;
-   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kCudaError;
-   static int slots[64] = {};  // CTAs resident at once
-   if (!slots[dev]) {
-      int sms = 0;
-      if (cudaFuncSetAttribute(curv_operator_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)) != cudaSuccess ||
-          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-         return kCudaError;
-      slots[dev] = std::max(1, sms) * CTAS;
-   }
+   static std::atomic<int> resident[64];
+   const int slots = resident_slots(resident, (const void*)curv_operator_kernel, NTHREADS, sizeof(Smem));
+   if (slots < 1) return kCudaError;
    const int gx = blocks_for(s.ie - s.ib - 3, TX), gy = blocks_for(s.je - s.jb - 3, TY), nk = k2 - k1 + 1;
-   a.kchunk = planes_per_cta((long long)gx * gy, nk, slots[dev]);
+   a.kchunk = planes_per_cta((long long)gx * gy, nk, slots);
    const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY);
    curv_operator_kernel<<<grid, block, sizeof(Smem), st>>>(a);
    return launch_status();

@@ -321,17 +321,10 @@ int launch_damping_layers(int order, const Box& b, int k1, int k2, const double*
    }
    a.beta = order == 4 ? beta : -0.5 * beta;
    a.emax = emax;
-   // the opt-in shared-memory size is a per-device function attribute
    const size_t smem = order == 4 ? sizeof(Shape<4>) : sizeof(Shape<6>);
    const void* kern = order == 4 ? (const void*)damping_layers_kernel<4> : (const void*)damping_layers_kernel<6>;
-   int dev = 0;
-   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kCudaError;
-   static bool attr_set[2][64] = {};
-   bool& set = attr_set[order == 4 ? 0 : 1][dev];
-   if (!set) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return kCudaError;
-      set = true;
-   }
+   static std::atomic<int> resident[2][64];
+   if (resident_slots(resident[order == 4 ? 0 : 1], kern, kThreads, smem) < 1) return kCudaError;
    const int gx = blocks_for(a.i1 - a.i0 + 1, TX), gy = blocks_for(a.j1 - a.j0 + 1, TY), nk = a.k1 - a.k0 + 1;
    a.kchunk = layer_chunk(gx, gy, nk);
    const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY);

@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "common.cuh"
 
 namespace sw4g {
@@ -420,6 +422,10 @@ int launch_uacc_slab(const Box& b, int k0, int k1, const double* up, const doubl
                      const double* um, double* out, cudaStream_t s);
 int launch_fused_stage(const FusedStage& st, cudaStream_t stream);
 int launch_fixed_stage(const FusedStage& st, cudaStream_t stream);
+int multiprocessors();
+// CTAs of a kernel that the current device holds at once (0: an error), with the kernel's
+// shared memory opted in.  Both are per device and kept in slots.
+int resident_slots(std::atomic<int> (&slots)[64], const void* kern, int threads, size_t smem);
 // planes per CTA of a fixed-point march of cols CTA columns over nk planes
 int planes_per_cta(long long cols, int nk, int slots);
 // lu = L(u) on the centred rows k1..k2 (operator_fixed.cu)

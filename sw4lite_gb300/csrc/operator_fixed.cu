@@ -526,19 +526,11 @@ int launch_operator_fixed(const Box& b, int k1, int k2, double* lu, const double
    a.lu = lu;
    a.cof = 1.0 / (144 * h * h);
    static_assert(sizeof(Smem) <= 113 * 1024, "two CTAs per SM");
-   // the opt-in shared-memory size is a per-device function attribute
-   int dev = 0;
-   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kCudaError;
-   static int slots[64] = {};  // CTAs resident at once
-   if (!slots[dev]) {
-      int sms = 0;
-      if (cudaFuncSetAttribute(operator_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)) != cudaSuccess ||
-          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-         return kCudaError;
-      slots[dev] = std::max(1, sms) * resident_ctas((const void*)operator_fixed_kernel, NTHREADS, sizeof(Smem));
-   }
+   static std::atomic<int> resident[64];
+   const int slots = resident_slots(resident, (const void*)operator_fixed_kernel, NTHREADS, sizeof(Smem));
+   if (slots < 1) return kCudaError;
    const int gx = blocks_for(b.ie - b.ib - 3, TX), gy = blocks_for(b.je - b.jb - 3, TY), nk = k2 - k1 + 1;
-   a.kchunk = planes_per_cta((long long)gx * gy, nk, slots[dev]);
+   a.kchunk = planes_per_cta((long long)gx * gy, nk, slots);
    const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY);
    operator_fixed_kernel<<<grid, block, sizeof(Smem), s>>>(a);
    return launch_status();

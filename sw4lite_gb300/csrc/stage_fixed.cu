@@ -667,20 +667,10 @@ int launch_fixed_stage(const FusedStage& st, cudaStream_t stream)
    const void* kern = form == 0 ? (const void*)fixed_stage_kernel<0>
                       : form == 1 ? (const void*)fixed_stage_kernel<1>
                                   : (const void*)fixed_stage_kernel<2>;
-   // the opt-in shared-memory size is a per-device function attribute
-   int dev = 0;
-   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kCudaError;
-   static bool attr_set[3][64] = {};
-   static int slots[3][64] = {};  // CTAs resident at once
-   if (!attr_set[form][dev]) {
-      int sms = 0;
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-         return kCudaError;
-      slots[form][dev] = std::max(1, sms) * resident_ctas(kern, NTHREADS, smem);
-      attr_set[form][dev] = true;
-   }
-   a.kchunk = st.kchunk > 0 ? st.kchunk : planes_per_cta((long long)gx * gy, nk, slots[form][dev]);
+   static std::atomic<int> resident[3][64];
+   const int slots = resident_slots(resident[form], kern, NTHREADS, smem);
+   if (slots < 1) return kCudaError;
+   a.kchunk = st.kchunk > 0 ? st.kchunk : planes_per_cta((long long)gx * gy, nk, slots);
    const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY, 1);
    if (form == 0)
       fixed_stage_kernel<0><<<grid, block, smem, stream>>>(a);

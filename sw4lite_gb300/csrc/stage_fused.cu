@@ -841,16 +841,33 @@ int resident_ctas(const void* kernel, int threads, size_t smem)
    return n > 0 ? n : 1;
 }
 
+// SMs of the current device; a GB300's where no device answers (host arithmetic alone).
+int multiprocessors()
+{
+   int sms = 0, dev = 0;
+   if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+       sms > 0)
+      return sms;
+   cudaGetLastError();
+   return 152;
+}
+
+int resident_slots(std::atomic<int> (&slots)[64], const void* kern, int threads, size_t smem)
+{
+   int dev = 0;
+   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+   int n = slots[dev].load(std::memory_order_acquire);
+   if (n > 0) return n;
+   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+   n = multiprocessors() * resident_ctas(kern, threads, smem);
+   slots[dev].store(n, std::memory_order_release);
+   return n;
+}
+
 int stage_kchunk(long long cols, int nk, int resident, int min_planes)
 {
    if (nk < 1) return 1;
-   int sms = 0, dev = 0;
-   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-       sms < 1) {
-      cudaGetLastError();
-      sms = 152;
-   }
-   const long long slots = (long long)sms * std::max(1, resident);
+   const long long slots = (long long)multiprocessors() * std::max(1, resident);
    const int forced = stage_chunks_override();
    int chunks = 1;
    if (forced > 0) {

@@ -653,7 +653,7 @@ int launch_mixed_stage(const MixedStage& st, cudaStream_t stream)
    // SM, and beside a second sweep of the gradient, many short ones (a topography grid's two
    // steps 2.02 ms a call; 2.43 with planes_per_cta's few long ones).
    const long long cols = (long long)gx * gy;
-   a.kchunk = st.alone ? planes_per_cta(cols, nk, 152 * resident[st.corrector][dev])
+   a.kchunk = st.alone ? planes_per_cta(cols, nk, multiprocessors() * resident[st.corrector][dev])
                        : stage_kchunk(cols, nk, resident[st.corrector][dev], 12);
    const dim3 grid(gx, gy, (nk + a.kchunk - 1) / a.kchunk), block(TX, TY, 1);
    if (st.corrector == 1)
