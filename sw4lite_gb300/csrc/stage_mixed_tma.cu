@@ -302,7 +302,17 @@ __global__ void __maxnreg__(128)
          issue_F(kbeg - 2);
       }
       for (int k = kbeg - 4; k <= kend; k++) {
-         if (__syncthreads_or(0)) return;  // (A)
+         if (__syncthreads_or(0)) {  // (A)
+            // not before the copies in flight, up to F(k + 2) and M(k), have landed (or their
+            // own waits give up): they would write to the next CTA's shared memory
+            if (tx == 0) {
+               const int m = max(k, kbeg);
+               mbar_wait(barF, (min(k + 2, kfin) - (kbeg - 2)) & 1);
+               for (int q = max(m - 1, kbeg); q <= m; q++) mbar_wait(barM0 + 8 * (q & 1), ((q - kbeg) >> 1) & 1);
+            }
+            __syncwarp();
+            return;
+         }
          if (tx == 0) {
             fence_async_shared();
             if (k + 3 <= kfin) issue_F(k + 3);
