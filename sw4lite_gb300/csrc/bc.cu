@@ -3,10 +3,10 @@
 //
 // Sides are processed in order 0..5 on the caller's stream, because windows of later sides
 // overlap earlier ones at edges and the free-surface solve reads ghost values written by
-// the lateral sides.  Without boundary data and periodic sides every window is zero, their
-// order does not matter and none meets what a free surface reads or writes in z: one launch
-// for all of them (a step at 48 x 40 x 36 spent 25 us on ten launches of 2.5 us), then the
-// free surfaces.
+// the lateral sides.  Without boundary data and periodic sides every window is zero and their
+// order does not matter: one launch for all of them (a step at 48 x 40 x 36 spent 25 us on
+// ten launches of 2.5 us), then the free surfaces, unless the window of side 5 meets the planes
+// that a free surface on side 4 reads (1..4) or writes (0).
 //   bccnd 1 (Dirichlet) / 2 (supergrid): copy the boundary data into the 2 ghost
 //     planes of the side's window (zero when no data array is given);
 //   bccnd 3 (periodic): copy from the point one period inside;
@@ -149,7 +149,8 @@ int bc_sides(int soa, int ib, int ie, int jb, int je, int kb, int ke, const int 
       if ((bccnd[side] != 1 && bccnd[side] != 2) || w.i1 < w.i0 || w.j1 < w.j0 || w.k1 < w.k0) continue;
       if (w.i0 < ib || w.i1 > ie || w.j0 < jb || w.j1 > je || w.k0 < kb || w.k1 > ke) return kBadArgument;
       points += (long long)(w.i1 - w.i0 + 1) * (w.j1 - w.j0 + 1) * (w.k1 - w.k0 + 1);
-      if (points > 0x7fffffffLL) {  // beyond the kernel's 32-bit count
+      const bool meets = side == 5 && bccnd[4] == 0 && w.k0 <= 4 && w.k1 >= 0;
+      if (meets || points > 0x7fffffffLL) {  // or beyond the kernel's 32-bit count
          zeros = false;
          break;
       }

@@ -190,3 +190,37 @@ def test_operator_non_finite_inputs(where):
     ref = np.zeros_like(u)
     O.rhs4sg(1, g.bounds, g.nz, [0] * 6, ref, u, mu, la, g.h, *st)
     assert np.array_equal(np.isfinite(_operator(g, 1, u, mu, la, st)), np.isfinite(ref))
+
+
+@pytest.mark.parametrize("soa", [1, 0])
+@pytest.mark.parametrize("nz,planes", [(3, None), (12, (3, 6)), (12, (-1, 0))])
+def test_bcfortsg_zero_window_among_the_free_surface_planes(soa, nz, planes):
+    """The window of side 5 meets the planes that the free surface on side 4 reads or writes: a
+    grid of three planes, and a caller's own window.  The sides act in their order."""
+    bccnd = (2, 2, 2, 2, 0, 2)
+    g = Grid(15, 13, nz, h=0.5)
+    rng = np.random.default_rng(7 + soa)
+    u0 = g.field3(rng)
+    _, mu, la = g.material(rng)
+    sx, sy, _ = g.stretching(rng)
+    wind, _ = O.boundary_windows(g.bounds, (g.nx, g.ny, g.nz), bccnd)
+    wind = [int(x) for x in wind]
+    if planes:
+        wind[34:36] = planes
+    _, _, _, sbop = O.stencil_coefficients()
+    ref = u0.copy()
+    O.bcfortsg(soa, g.bounds, wind, (g.nx, g.ny, g.nz), ref, g.h, bccnd, sbop, mu, la, [None] * 6, sx, sy)
+    du, dmu, dla, dsx, dsy = dev(u0), dev(mu), dev(la), dev(sx), dev(sy)
+
+    def sides(field, active):
+        sg.check(sg.lib().sw4g_bcfortsg(soa, *g.bounds, (C.c_int * 36)(*wind), g.nx, g.ny, g.nz, field.data_ptr(), g.h,
+                                        (C.c_int * 6)(*[b if s in active else 4 for s, b in enumerate(bccnd)]),
+                                        C.cast((C.c_double * 6)(*sbop), sg._D), dmu.data_ptr(), dla.data_ptr(),
+                                        (C.c_void_p * 6)(), dsx.data_ptr(), dsy.data_ptr(), stream()))
+
+    one_by_one = dev(u0)
+    for s in range(6):
+        sides(one_by_one, (s,))
+    sides(du, range(6))
+    assert np.array_equal(host(du), host(one_by_one))
+    assert rel_err(host(du), ref) <= 1e-14
