@@ -584,7 +584,9 @@ __global__ void fixed_coef_kernel(Box b, const double* __restrict__ mu, const do
             ew[p + ax * b.npts] = (int)((unsigned)et[1] << 16 | ((unsigned)et[0] & 0xffffu));
          }
       }
-      if (any) *bad = 1;
+      // ghost points off two axes' interiors are in no stencil
+      const int off = (i < b.ib + 2 || i > b.ie - 2) + (j < b.jb + 2 || j > b.je - 2) + (k < b.kb + 2 || k > b.ke - 2);
+      if (any && off < 2) *bad = 1;
    }
 }
 

@@ -119,3 +119,20 @@ def test_operator_products_that_overflow(case):
                                   *[t.data_ptr() for t in d[3:]], None))
     assert not np.all(np.isfinite(want))
     assert np.array_equal(np.isfinite(host(lu)), np.isfinite(want))
+
+
+def test_ghost_edges_of_the_material_are_in_no_stencil():
+    """Material that is NaN on the ghost points off two axes' interiors: the same bits as with
+    finite values there."""
+    nx, ny, nz = SHAPE
+    mat = smooth_material(nx, ny, nz, seed=2)
+    dt = 0.3 * 0.05 / float(np.sqrt(np.max((4 * mat[1] + mat[2]) / mat[0])))
+    u, um = smooth_fields(nx, ny, nz, seed=7)
+    want, _ = _predicted(mat, u, um, dt, 0.05)
+    k, j, i = np.meshgrid(*[(np.arange(n + 4) < 2) | (np.arange(n + 4) >= n + 2) for n in (nz, ny, nx)], indexing="ij")
+    edges = (i.astype(int) + j + k >= 2).ravel()
+    for a in mat[1:]:
+        a[edges] = np.nan
+    got, _ = _predicted(mat, u, um, dt, 0.05)
+    m = (slice(None), slice(2, -2), slice(2, -2))
+    assert np.array_equal(got[m], want[m])
