@@ -84,11 +84,11 @@ def measured_peaks():
 # words) and mu, lambda, rho (3), writes the new level (3): 15 FP64 words
 CORR_STAGE_WORDS = 15
 # DRAM bytes and warp instructions per interior point of the fixed-point FP64 stage kernels
-# (ncu captures at 256^3, profiles/fixed_stage_c2_256.md: corrector 5.590e9 B and
-# 1,187,100,000 warp instructions, predictor 1,143,807,280, over 256^3 points); both grow
+# (ncu captures at 256^3, profiles/fixed_stage_c2_256.md: corrector 5.805e9 B and
+# 1,546,625,220 warp instructions, predictor 1,494,646,876, over 256^3 points); both grow
 # with the point count.  An SM issues at most 4 warp instructions a clock.
-CORR_STAGE_DRAM_BYTES_PER_PT = 333.2
-WARP_INST_PER_PT = {"corr": 1187100000 / 256 ** 3, "pred": 1143807280 / 256 ** 3}
+CORR_STAGE_DRAM_BYTES_PER_PT = 346.0
+WARP_INST_PER_PT = {"corr": 1546625220 / 256 ** 3, "pred": 1494646876 / 256 ** 3}
 WARP_INST_PER_CLK_PER_SM = 4
 # FP64-pipe warp instructions per interior point of the same stages in FP64 arithmetic
 # (profiles/fp64_pipe_c2_512.md): what the fixed-point form avoids.  The pipe issues 2 FP64

@@ -240,7 +240,8 @@ __global__ void grad_profiles_kernel(int n, const double* __restrict__ st, const
 // that other kernels leave: beside the damping, the closures and the last CTAs of a stage
 // (the fixed-point stages themselves leave none while they fill the SMs), or beside the
 // predictor form of the FP64 stages (16K of an SM's: three of grad_df_kernel's CTAs at 72
-// registers, but one of 128 threads).  Issue slots bound them: 62 and 67 % busy alone.
+// registers, but one of 128 threads).  Issue slots bound them: 75 % (edge) and
+// 65 % (the sums) busy alone at 128^3.
 constexpr int kGradThreads = 64;
 
 // w1 = up - 2u + um; the pairs of b1, mt (adjoint shift) and w1, u, um (forward
