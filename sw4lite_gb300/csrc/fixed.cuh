@@ -104,18 +104,21 @@ __device__ __forceinline__ int headroom(i64 m)
 }
 
 // m * 2^e with the leading bit of m brought to bit 60 (left at bit 61 if it is there): what is
-// formed from a difference keeps its accuracy, however small it is against its terms.  A
-// difference below 2^32 is left for `rest`.
-__device__ __forceinline__ Num normal(i64 m, int e)
+// formed from a difference keeps its accuracy, however small it is against its terms.  Below
+// 2^32 the exponent is lowered by kBelow on top, right for zero, and tiny tells of a difference
+// that is not zero, for which `rest` finishes.
+constexpr int kBelow = 16384;
+__device__ __forceinline__ Num normal(i64 m, int e, bool& tiny)
 {
    const int n = headroom<60>(m);
-   return Num{m << n, e - n};
+   const bool below = n == 29;  // the upper word is sign alone
+   tiny = tiny || (below && m != 0);
+   return Num{m << n, e - n - (below ? kBelow : 0)};
 }
-__device__ __forceinline__ bool small(const Num& d) { return __clz((int)(d.m >> 32) ^ (int)(d.m >> 63)) > 3; }
 __device__ __forceinline__ void rest(Num& d)
 {
-   const int n = max(__clzll(d.m ^ (d.m >> 63)) - 3, 0);
-   d = Num{d.m << n, d.m == 0 ? kNone : d.e - n};
+   const int n = max(__clzll(d.m ^ (d.m >> 63)) - 3, 0), e = d.e < -kBelow / 2 ? d.e + kBelow : d.e;
+   d = Num{d.m << n, d.m == 0 ? kNone : e - n};
 }
 
 // 8 (fp1 - fm1) + (fm2 - fp2)
@@ -125,9 +128,9 @@ __device__ __forceinline__ i64 d1i(i64 fm2, i64 fm1, i64 fp1, i64 fp2)
 }
 
 // The difference d1i(x) of values |x| < 2^57 aligned to the exponent e of the largest
-__device__ __forceinline__ Num difference(i64 x0, i64 x1, i64 x2, i64 x3, int e0, int e1, int e2, int e3, int e)
+__device__ __forceinline__ Num difference(i64 x0, i64 x1, i64 x2, i64 x3, int e0, int e1, int e2, int e3, int e, bool& tiny)
 {
-   return normal(d1i(sar(x0, e - e0), sar(x1, e - e1), sar(x2, e - e2), sar(x3, e - e3)), e);
+   return normal(d1i(sar(x0, e - e0), sar(x1, e - e1), sar(x2, e - e2), sar(x3, e - e3)), e, tiny);
 }
 
 // x * C / 2^57 for |x| < 2^62 and a coefficient |C| < 2^57 held as c.x = C >> 26,

@@ -279,24 +279,25 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
       const int qz[4] = {qm2, qm1, qp1, qp2};
       // differences of component c at the point s along an axis of the plane (stride o) or
       // across the planes
-      auto along = [&](int c, int s, int o) {
+      auto along = [&](int c, int s, int o, bool& tiny) {
          const i64* v = v0 + c * PLANE + s;
          const int x0 = unpack(c, e0[s - 2 * o]), x1 = unpack(c, e0[s - o]), x2 = unpack(c, e0[s + o]), x3 = unpack(c, e0[s + 2 * o]);
-         return difference(v[-2 * o], v[-o], v[o], v[2 * o], x0, x1, x2, x3, max4(x0, x1, x2, x3));
+         return difference(v[-2 * o], v[-o], v[o], v[2 * o], x0, x1, x2, x3, max4(x0, x1, x2, x3), tiny);
       };
-      auto down = [&](int c, int s) {
+      auto down = [&](int c, int s, bool& tiny) {
          const int x0 = unpack(c, sm.ve[qm2][s]), x1 = unpack(c, sm.ve[qm1][s]), x2 = unpack(c, sm.ve[qp1][s]), x3 = unpack(c, sm.ve[qp2][s]);
-         return difference(sm.v[qm2][c][s], sm.v[qm1][c][s], sm.v[qp1][c][s], sm.v[qp2][c][s], x0, x1, x2, x3, max4(x0, x1, x2, x3));
+         return difference(sm.v[qm2][c][s], sm.v[qm1][c][s], sm.v[qp1][c][s], sm.v[qp2][c][s], x0, x1, x2, x3, max4(x0, x1, x2, x3), tiny);
       };
 
       Num D[3][3];  // differences along x, y, z of the components
+      bool few = false;  // one of them has lost nearly all its bits
       Num S[3] = {{0, kNone}, {0, kNone}, {0, kNone}};
       if (!full) {
-         D[0][0] = along(0, own, 1);
-         D[0][2] = along(2, own, 1);
-         D[1][1] = along(1, own, PX);
-         D[1][2] = along(2, own, PX);
-         rest(D[0][0]), rest(D[0][2]), rest(D[1][1]), rest(D[1][2]);
+         D[0][0] = along(0, own, 1, few);
+         D[0][2] = along(2, own, 1, few);
+         D[1][1] = along(1, own, PX, few);
+         D[1][2] = along(2, own, PX, few);
+         if (few) rest(D[0][0]), rest(D[0][2]), rest(D[1][1]), rest(D[1][2]);
       } else {
          const int qx = ty * PX + tx, qy = ty * TX + tx;
 #pragma unroll
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
                      const int s = m < 2 ? m - 2 : m - 1;
                      x[m] = sar(ax == 0 ? v0[c * PLANE + own + s] : ax == 1 ? v0[c * PLANE + own + s * PX] : sm.v[qz[m]][c][own], E - e[m]);
                   }
-                  D[ax][c] = normal(d1i(x[0], x[1], x[2], x[3]), E);
+                  D[ax][c] = normal(d1i(x[0], x[1], x[2], x[3]), E, few);
                   // differences to the own value, aligned by the size of their products with the weights,
                   // the largest brought to bit 57
                   const i64 x0 = sar(v0[c * PLANE + own], Ec - eo);
@@ -372,8 +373,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
                   if (tiny)
 #pragma unroll
                      for (int m = 0; m < 4; m++) {
-                        const int n = max(__clzll(x[m] ^ (x[m] >> 63)) - 6, 0);
-                        pe[m] = x[m] == 0 ? kNone : pe[m] - n;
+                        const int n = max(__clzll(x[m] ^ (x[m] >> 63)) - 6, 0), e = pe[m];
+                        pe[m] = x[m] == 0 ? kNone : e - n;
                         x[m] <<= n;
                      }
                   const int ep = max4(pe[0], pe[1], pe[2], pe[3]);
@@ -401,18 +402,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
          for (int c = 0; c < 3; c++) S[c].e = max(S[c].e - 1020, kNone);
       }
 
-      if (full) {
-         bool any = false;
+      if (full && few)
 #pragma unroll
          for (int ax = 0; ax < 3; ax++)
 #pragma unroll
-            for (int c = 0; c < 3; c++) any = any || small(D[ax][c]);
-         if (any)
-#pragma unroll
-            for (int ax = 0; ax < 3; ax++)
-#pragma unroll
-               for (int c = 0; c < 3; c++) rest(D[ax][c]);
-      }
+            for (int c = 0; c < 3; c++) rest(D[ax][c]);
       // products of the own point
       const int2 lm = limbs(cm[0]), ll = limbs(cm[1]);
       const int emu = ec[0] - 1022, ela = ec[1] - 1022;
@@ -438,8 +432,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) operator_fixed_kernel(OpFixed a)
          to_y(products<true>(D[0][0], D[2][2], D[0][1], D[2][1], lm, emu, ll, ela, sxi, szk), (ty + HALO) * TX + tx);
          if (halo) {
             const int s = hrow * PX + hcl, o = yh ? 1 : PX, cs = yh ? 0 : 1, cc = 1 - cs;
-            Num d0 = along(cs, s, o), d1 = down(2, s), d2 = along(cc, s, o), d3 = down(cc, s);
-            if (small(d0) || small(d1) || small(d2) || small(d3)) rest(d0), rest(d1), rest(d2), rest(d3);
+            bool some = false;
+            Num d0 = along(cs, s, o, some), d1 = down(2, s, some), d2 = along(cc, s, o, some), d3 = down(cc, s, some);
+            if (some) rest(d0), rest(d1), rest(d2), rest(d3);
             const Triple t = products<true>(d0, d1, d2, d3, limbs(hm[0]), he[0] - 1022, limbs(hm[1]), he[1] - 1022, hin, szk);
             if (yh) to_y(t, hrow * TX + tx);
             else to_x(t, (hrow - HALO) * PX + hcl);

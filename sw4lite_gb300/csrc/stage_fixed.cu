@@ -32,7 +32,7 @@
 //  * FP64 remains in forming up - 2u + um and in the update.
 // What bounds them: the latency of twelve warps an SM and the integer pipes (about 2900
 // instructions a warp of 32 points, half of them at half rate), the corrector also the FP64
-// operations of its stage field.  At 512^3 the predictor takes 17.9 ms and the corrector 25.5 ms
+// operations of its stage field.  At 512^3 the predictor takes 17.9 ms and the corrector 25.8 ms
 // with the damping, against 40.6 and 53.8 ms with the sums in FP64 (stage_fused.cu), whose 160
 // and 198 FP64 operations a point saturate the 1.7 that an SM completes per clock.  (One
 // exponent for a point's three components, and one for all its weights, took 15.2 and 22.5 ms,
@@ -285,32 +285,37 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
 #pragma unroll
             for (int ax = 0; ax < 3; ax++) ew[ax] = __ldg(a.ew + plane + col + ax * npts);
       }
+      if (hcol >= 0) {
+         hc = __ldg(a.c + plane + hcol);
+         he = __ldg(a.e + plane + hcol);
+      }
       const double szk = __ldg(a.sz + (k - a.kb));
       const i64* v0 = &sm.v[q0][0][0];
       const short* e0 = &sm.ve[q0][0][0];
       const int qz[4] = {qm2, qm1, qp1, qp2};
       // value and exponent of component c at the point s, m points along an axis of the plane
       // (stride o) or, as down, planes
-      auto along = [&](int c, int s, int o) {
+      auto along = [&](int c, int s, int o, bool& tiny) {
          const i64* v = v0 + c * PLANE + s;
          const short* e = e0 + c * PLANE + s;
          const int x0 = e[-2 * o], x1 = e[-o], x2 = e[o], x3 = e[2 * o];
-         return difference(v[-2 * o], v[-o], v[o], v[2 * o], x0, x1, x2, x3, max4(x0, x1, x2, x3));
+         return difference(v[-2 * o], v[-o], v[o], v[2 * o], x0, x1, x2, x3, max4(x0, x1, x2, x3), tiny);
       };
-      auto down = [&](int c, int s) {
+      auto down = [&](int c, int s, bool& tiny) {
          const int x0 = sm.ve[qm2][c][s], x1 = sm.ve[qm1][c][s], x2 = sm.ve[qp1][c][s], x3 = sm.ve[qp2][c][s];
-         return difference(sm.v[qm2][c][s], sm.v[qm1][c][s], sm.v[qp1][c][s], sm.v[qp2][c][s], x0, x1, x2, x3, max4(x0, x1, x2, x3));
+         return difference(sm.v[qm2][c][s], sm.v[qm1][c][s], sm.v[qp1][c][s], sm.v[qp2][c][s], x0, x1, x2, x3, max4(x0, x1, x2, x3), tiny);
       };
 
       Num D[3][3];  // differences along x, y, z of the components
+      bool tiny = false;
       i64 S[3] = {0, 0, 0};
       int eS[3] = {kNone, kNone, kNone};
 
       if (!full) {
-         D[0][0] = along(0, own, 1);
-         D[0][2] = along(2, own, 1);
-         D[1][1] = along(1, own, PX);
-         D[1][2] = along(2, own, PX);
+         D[0][0] = along(0, own, 1, tiny);
+         D[0][2] = along(2, own, 1, tiny);
+         D[1][1] = along(1, own, PX, tiny);
+         D[1][2] = along(2, own, PX, tiny);
       } else {
          // the largest exponent along each axis, and of a component's w x
          int E[3][3], eo[3];
@@ -348,7 +353,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
                   const int e = ax == 0 ? e0[c * PLANE + own + s] : ax == 1 ? e0[c * PLANE + own + s * PX] : sm.ve[qz[m]][c][own];
                   x[m] = sar(ax == 0 ? v0[c * PLANE + own + s] : ax == 1 ? v0[c * PLANE + own + s * PX] : sm.v[qz[m]][c][own], E_ - e);
                }
-               D[ax][c] = normal(d1i(x[0], x[1], x[2], x[3]), E_);
+               D[ax][c] = normal(d1i(x[0], x[1], x[2], x[3]), E_, tiny);
                const i64 x0 = sar(v0[c * PLANE + own], A - eo[c]);
 #pragma unroll
                for (int m = 0; m < 4; m++) {
@@ -368,20 +373,16 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
          }
       }
 
-      // differences that cancelled almost or fully
-      if (!full) {
-         rest(D[0][0]), rest(D[0][2]), rest(D[1][1]), rest(D[1][2]);
-      } else {
-         bool any = false;
-#pragma unroll
-         for (int ax = 0; ax < 3; ax++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) any = any || small(D[ax][c]);
-         if (any)
+      // differences that cancelled almost
+      if (tiny) {
+         if (!full) {
+            rest(D[0][0]), rest(D[0][2]), rest(D[1][1]), rest(D[1][2]);
+         } else {
 #pragma unroll
             for (int ax = 0; ax < 3; ax++)
 #pragma unroll
                for (int c = 0; c < 3; c++) rest(D[ax][c]);
+         }
       }
 
       // Products of the own point
@@ -411,12 +412,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) fixed_stage_kernel(FixedArgs a)
          if (halo) {
             // y outer: mu v_x, la (u_x + w_z), mu v_z;  x outer: la (v_y + w_z), mu u_y, mu u_z
             const int s = hrow * PX + hcl, o = yh ? 1 : PX, cs = yh ? 0 : 1, cm = 1 - cs;
-            if (hcol >= 0) {
-               hc = __ldg(a.c + plane + hcol);
-               he = __ldg(a.e + plane + hcol);
-            }
-            Num d0 = along(cs, s, o), d1 = down(2, s), d2 = along(cm, s, o), d3 = down(cm, s);
-            if (small(d0) || small(d1) || small(d2) || small(d3)) rest(d0), rest(d1), rest(d2), rest(d3);
+            bool some = false;
+            Num d0 = along(cs, s, o, some), d1 = down(2, s, some), d2 = along(cm, s, o, some), d3 = down(cm, s, some);
+            if (some) rest(d0), rest(d1), rest(d2), rest(d3);
             const Triple t = products<false>(d0, d1, d2, d3, make_int2(hc.x, hc.y), (int)(short)(he & 0xffff), make_int2(hc.z, hc.w), he >> 16, hst, szk);
             if (yh) to_y(t, hrow * TX + tx);
             else to_x(t, (hrow - HALO) * PX + hcl);
