@@ -11,7 +11,7 @@ import pytest
 
 import sw4lite_gb300 as sg
 from oracle import oracle as O
-from tests import (test_gpu_adjoint, test_gpu_graphs, test_gpu_halo, test_gpu_nancheck, test_gpu_stage_fixed,
+from tests import (wide, test_gpu_adjoint, test_gpu_graphs, test_gpu_halo, test_gpu_nancheck, test_gpu_stage_fixed,
                    test_gpu_step, test_gpu_topo)
 from tests.adjoint_util import AdjointCase, oracle_forward
 from tests.gpu_util import dev, host, smooth_fields, smooth_material
@@ -233,3 +233,39 @@ def test_topography_takes_the_room_of_the_coefficients():
     b, form = run(True)
     assert form == sg.STAGES_FP64
     assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(a))
+
+
+def test_the_fixed_form_is_no_further_off_than_fp64_sums():
+    """Eight steps of both forms against extended precision (predictor, corrector, no damping):
+    the error of the fixed-point form, over all components, is no larger."""
+    nx, ny, nz = shape = (21, 20, 19)
+    h, steps = 0.05, 8
+    rho, mu, la = mat = smooth_material(nx, ny, nz, seed=6)
+    dt = 0.3 * h / float(np.sqrt(np.max((4 * mu + la) / rho)))
+    fields = smooth_fields(nx, ny, nz, seed=4, scale=1.0)
+    cut = (slice(None),) + (slice(2, -2),) * 3
+    for a in fields:  # ghost planes as a Dirichlet side leaves them
+        b = a.reshape(3, nz + 4, ny + 4, nx + 4)
+        inner = b[cut].copy()
+        b[:] = 0
+        b[cut] = inner
+    u, um = [a.reshape(3, nz + 4, ny + 4, nx + 4).astype(wide.L) for a in fields]
+    r, m, l = [a.reshape(nz + 4, ny + 4, nx + 4) for a in mat]
+    one = [np.ones(n + 4) for n in shape]
+    d2 = wide.L(dt) ** 2
+    for _ in range(steps):
+        up = 2 * u - um + d2 / r * wide.operator(u, m, l, one, h)[0]
+        up[~np.broadcast_to(wide._interior(np.ones_like(r)) > 0, up.shape)] = 0
+        new = up + d2 / 12 / r * wide.operator(up - 2 * u + um, m, l, one, h)[0]
+        u, um = new, u
+    error = {}
+    for form in (sg.STAGES_FIXED, sg.STAGES_FP64):
+        ew = sg.EW(sg.grid_desc(nx, ny, nz, h, bc=(1,) * 6, sg_gp=4))
+        ew.set_stage_form(form)
+        ew.set_material(*[dev(a) for a in mat])
+        ew.set_time_step(dt, 0.0)
+        got = _steps(ew, *fields, steps).reshape(u.shape)
+        ew.close()
+        e = got[cut] - u[cut]
+        error[form] = float(np.sqrt(np.sum(e * e) / np.sum(u[cut] ** 2)))
+    assert error[sg.STAGES_FIXED] <= error[sg.STAGES_FP64] < 1e-14, error
