@@ -13,7 +13,7 @@
 //
 // What bounds it: the latency of twelve warps an SM and the integer pipes, about 5000
 // instructions a warp of 32 points, and 20 FP64 operations a point, against 410 for one thread
-// per point that forms every weight and inner difference anew: 256 x 200 x 150 points 2.18 ms
+// per point that forms every weight and inner difference anew: 256 x 200 x 150 points 2.15 ms
 // against 5.97 ms.  (One exponent for a point's components and coefficients: 1.74 ms, and the
 // smaller ones lost digits.)
 #include <algorithm>
